@@ -195,6 +195,29 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
+int sm_count(int* n) {
+  static int nsm[64] = {};
+  int dev = 0;
+  JFG_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
+  if (!nsm[dev]) JFG_CUDA_TRY(cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev));
+  *n = nsm[dev];
+  return JFG_OK;
+}
+
+// largest tile (16 R) that still gives two CTAs per SM (the list-restricted
+// launches count their full batch: the active count is not known here)
+int tile_r(const jfg_contract_desc& d, bool f32, int sms) {
+  const long long gz = (long long)d.batch * d.nseg;
+  auto ctas = [&](int t) {
+    return (long long)((d.P + t - 1) / t) * ((d.M + t - 1) / t) * gz;
+  };
+  // FP32 launches big enough for 128 x 128 tiles take them (8 x 8 outputs per
+  // thread: half the shared-memory loads per FMA of the 64 x 64 tile)
+  if (f32 && ctas(128) >= 2 * sms) return 8;
+  return ctas(64) >= 2 * sms ? 4 : ctas(32) >= 2 * sms ? 2 : 1;
+}
+
 // 128 x 128 tiles for FP32 only (64 FP64 accumulators would not fit)
 template <typename T, int E>
 void launch_r8(dim3 grid, const jfg_contract_desc& d, const T* op, const T* in, T* out,
@@ -214,20 +237,9 @@ int launch_simt(const jfg_contract_desc& d, const T* op, const T* in, T* out,
   if (d.epilogue != JFG_EPI_NONE && d.epilogue != JFG_EPI_MUL_FIELD &&
       d.epilogue != JFG_EPI_DIV_EIG)
     return JFG_ERR_ARG;
-  // largest tile that still gives two CTAs per SM (the list-restricted
-  // launches count their full batch: the active count is not known here)
-  static int nsm[64] = {};
-  int dev = 0;
-  JFG_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
-  if (!nsm[dev]) JFG_CUDA_TRY(cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev));
-  auto ctas = [&](int t) {
-    return (long long)((d.P + t - 1) / t) * ((d.M + t - 1) / t) * gz;
-  };
-  // FP32 launches big enough for 128 x 128 tiles take them (8 x 8 outputs per
-  // thread: half the shared-memory loads per FMA of the 64 x 64 tile)
-  const bool r8 = std::is_same<T, float>::value && ctas(128) >= 2 * nsm[dev];
-  const int R = r8 ? 8 : ctas(64) >= 2 * nsm[dev] ? 4 : ctas(32) >= 2 * nsm[dev] ? 2 : 1;
+  int sms = 0;
+  JFG_TRY(sm_count(&sms));
+  const int R = tile_r(d, std::is_same<T, float>::value, sms);
   const int tile = 16 * R;
   dim3 grid((d.P + tile - 1) / tile, (d.M + tile - 1) / tile, (unsigned)gz);
   if (grid.y > 65535) return JFG_ERR_ARG;
@@ -300,6 +312,11 @@ int validate_desc(const jfg_contract_desc& d) {
   if (d.epilogue < 0 || d.epilogue > 2) return JFG_ERR_ARG;
   if ((d.batch_list == nullptr) != (d.batch_count == nullptr)) return JFG_ERR_ARG;
   return JFG_OK;
+}
+
+int contract_f64_tile(const jfg_contract_desc& d) {
+  int sms = 0;
+  return 16 * (sm_count(&sms) == JFG_OK ? tile_r(d, false, sms) : 4);
 }
 
 int contract_f64(const jfg_contract_desc& d, const double* op, const double* in, double* out,

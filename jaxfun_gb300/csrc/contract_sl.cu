@@ -1,0 +1,962 @@
+// FP64 per-axis contraction on the tensor cores by error-free slicing:
+//
+//   out[b][s][m][p] = alpha * epi(sum_k op[s][m][k] * in[b][s][p][k]) + beta * out
+//
+// with FP64 operands and FP64 results.  GB300 issues about 2 FP64 FMAs per
+// clock per SM, so the CUDA-core contraction (contract_simt.cu) is bound by
+// that pipe at ~1.24 TFLOP/s.  Here every operand row becomes a 62-bit
+// fixed-point number per element (one power-of-two scale per row), cut into
+// eight signed base-256 digits that FP16 holds exactly; products of digits are
+// accumulated exactly by the tensor cores (kind::f16, FP32 accumulators that
+// stay below 2^24 in magnitude), and the accumulators of equal weight are put
+// together in integer arithmetic and rounded to FP64 once.  This is the
+// error-free transformation of matrix products of Ozaki, Ogita, Oishi and
+// Rump (Numerical Algorithms 59, 2012) in the form that Mukunoki, Ozaki,
+// Ogita and Imamura (ISC 2020) gave it for tensor cores.
+//
+// Accuracy.  The operator's columns are first scaled by powers of two to a
+// largest entry in [1, 2) and the input's columns by the inverse, so that a
+// column of large entries against small coefficients (derivatives of spectral
+// bases) does not cost digits.  An element then keeps 61 bits below its
+// scaled row's largest one, and the digit products left out (weights 2^-64
+// and below) are as small.  Level d sums at most d + 1 digit pairs, each
+// below 2^14 K: levels 0..3 cannot pass 2^24 for K <= 256 (0 and 1 for
+// K <= 512), and a level that did could only lose its last bits, which weigh
+// 2^-8d.  Rows with an infinity or a NaN (in the operator or the input) are
+// summed by plain FP64 FMAs in the epilogue.
+//
+// Tile.  A CTA takes PT input rows (p) of one problem and segment, cuts them
+// into digits and keeps all K of all eight digits in shared memory as the
+// MMA's N operand: a block of PT zero rows, then PT rows per digit (K-major,
+// 128-byte swizzle).  The operator's digits, cut once per call into a
+// workspace, stream through TMA as the M operand (128 rows by 64 K of one
+// digit, 16 KB).  Levels are accumulated in pairs (2h, 2h + 1), 2 PT columns
+// of TMEM each: operator digit i meets input digits 2h - i and 2h + 1 - i,
+// which are neighbouring blocks of the N operand (the zero block stands for
+// digit -1), 20 MMAs of N = 2 PT per 16 K for 36 digit products.  Pairs are
+// kept apart because only MMAs of one shape on one accumulator are ordered
+// among themselves.  The MMAs of one operator digit share its tile through the
+// collector buffer: 37 clocks per MMA of N = 64 against 48 when each reads the
+// tile from shared memory (measured; 32 would be the tensor pipe's own).  Two
+// accumulator sets of 8 PT columns (all 512 columns of TMEM for PT = 32) let
+// the epilogue of one set run during the MMAs of the next, and with K <= 128
+// two input tiles fit, so that cutting overlaps them too.  PT = 16 serves K in
+// (256, 512] and launches too small to fill the chip with PT = 32.  When all
+// operator digits fit in the stages (M <= 128, K <= 64) they are loaded once
+// per CTA.
+//
+// The epilogue uses integers throughout: on the FP64 pipe (a warp instruction
+// holds its scheduler's share for 64 clocks) even the two additions that would
+// round a result cost more than the 35 integer instructions.
+//
+// Warps: 0 TMA producer, 1 TMEM allocator and MMA issuer, 2-9 cut the input,
+// 10-17 epilogue (two per TMEM lane quarter).  Every wait is bounded
+// (tc_common.cuh); after a timeout the issued MMAs and loads are waited for
+// before TMEM is freed, and jfg_device_status() reports it.
+#include <cooperative_groups.h>
+#include <cuda_fp16.h>
+
+#include "jfg_internal.cuh"
+#include "tc_common.cuh"
+
+namespace jfg {
+
+__device__ int g_sl_status = 0;
+
+namespace {
+
+constexpr int NS = 8;             // digits
+constexpr int NWS = 8;            // warps that cut the input
+constexpr int NWE = 8;            // epilogue warps
+constexpr int SL_NT = 64 + 32 * (NWS + NWE);
+constexpr uint32_t ABYTES = 128 * 128;  // one operator stage: 128 rows x 64 FP16
+constexpr int A_MAX = 8;          // operator stages
+constexpr int STG_LD = 9;         // epilogue staging: 32 rows x 8 columns, padded
+constexpr int RING = 4;           // input tiles whose row exponents are kept
+constexpr int COL_MAX = 3 * 512;  // column exponents (segments x K padded to 64)
+constexpr int SPECIAL = 1 << 20;  // row exponent of a row with inf or NaN
+// Sum of two row exponents from which a running FP64 sum of up to 512 products
+// (each below 2^(sum - 2044)) could overflow; rows with specials are above it.
+constexpr int BIG = 3068 - 10;
+constexpr int NO_COLUMN = -3000;  // column exponent of an all-zero column
+constexpr size_t SMEM_LIMIT = 227 * 1024;
+
+struct SlLaunch {
+  CUtensorMap amap;  // operator digits {K, M, segment x digit}
+  jfg_contract_desc d;
+  const double* op;
+  const double* in;
+  double* out;
+  const int* row_e;      // [segments][M]
+  const int16_t* col_e;  // [segments][kpad]
+  int op_segs;           // segments of the operator (1: shared by all)
+  int row_ld;            // row exponents per segment
+  int kpad;              // K padded to 64
+  int nkb;               // 64-element K blocks
+  int bbuf;              // input tiles in shared memory
+  int astages;
+  int a_res;             // 1: every operator tile has its own stage, loaded once
+  int vec2;              // input rows are 16-byte aligned
+  int scaled;            // alpha != 1
+  int nptiles, mtiles;
+};
+
+// exponent field of x, at least 1 (subnormals), plus the column's exponent
+__device__ __forceinline__ int elem_e(double x, int ce) {
+  const int ex = (__double2hiint(x) >> 20) & 0x7FF;
+  return (ex ? ex : 1) + ce;
+}
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((__double2hiint(x) & 0x7FFFFFFF) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool not_finite(double x) {
+  return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000;
+}
+
+// 16-bit integer e of eight packed in v
+__device__ __forceinline__ int short_of(const uint4& v, int e) {
+  const uint32_t w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
+  return (e & 1) ? (int)w >> 16 : (int)(w << 16) >> 16;
+}
+
+// x 2^(61 - E) truncated to an integer (|.| < 2^62; e = elem_e(x) <= E, E its
+// row's maximum), plus 0x80 in every byte: byte 7 - j is then digit j + 128.
+__device__ __forceinline__ unsigned long long biased_fixed(double x, int e, int E) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t mh = (hi & 0xFFFFFu) | ((hi & 0x7FF00000u) ? 0x100000u : 0u);
+  const unsigned long long m = ((unsigned long long)mh << 32 | lo) << 9;
+  const unsigned s = min((unsigned)(E - e), 63u);  // a zero with e > E wraps to 63
+  const unsigned long long v = m >> s;
+  const unsigned long long sg = (unsigned long long)((long long)((unsigned long long)hi << 32) >> 63);
+  return (v ^ sg) - sg + 0x8080808080808080ull;
+}
+
+// digit j of eight consecutive elements as packed FP16: byte b - 128, formed
+// as the FP16 number 1024 + b minus 1152 (both exact)
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int j) {
+  const uint32_t x = j < 4 ? (uint32_t)(a >> 32) : (uint32_t)a;
+  const uint32_t y = j < 4 ? (uint32_t)(b >> 32) : (uint32_t)b;
+  const uint32_t t = 3 - (j & 3);
+  const uint32_t u = (__byte_perm(x, y, t | ((4 + t) << 8)) & 0x00FF00FFu) | 0x64006400u;
+  const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&u), __floats2half2_rn(1152.f, 1152.f));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// ---------------------------------------------------------------------------
+// operator digits
+// ---------------------------------------------------------------------------
+
+constexpr int SPLIT_T = 256;
+constexpr int SPLIT_CL = 8;
+
+struct SlSeg {
+  const double* src;
+  long long ld;
+  int M, K, Kp, kpad;
+  uint16_t* dig;  // [NS][M][Kp]
+  int* row_e;
+  int16_t* col_e;
+};
+struct SlSplitArgs {
+  SlSeg s[SL_MAX_SEGS];
+};
+
+// One cluster of 8 CTAs per operator segment: column maxima over each CTA's
+// rows, combined through distributed shared memory; then one warp per row
+// finds the row's exponent and writes its digits.  A few microseconds, bound
+// by the latency of two reads of the rows (256 x 256: 4 rows per warp).
+__global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
+    k_sl_split(const __grid_constant__ SlSplitArgs A) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ int cmax[512];
+  __shared__ int16_t ce[512];
+  const SlSeg& q = A.s[blockIdx.x / SPLIT_CL];
+  const int rank = (int)cl.block_rank();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k = threadIdx.x; k < q.K; k += SPLIT_T) {
+    int mx = -1;
+    for (int m = rank; m < q.M; m += SPLIT_CL) {
+      const double x = q.src[(long long)m * q.ld + k];
+      if (!is_zero(x) && !not_finite(x)) mx = max(mx, elem_e(x, 0));
+    }
+    cmax[k] = mx;
+  }
+  cl.sync();
+  for (int k = threadIdx.x; k < q.kpad; k += SPLIT_T) {
+    int c = 0;
+    if (k < q.K) {
+      int mx = -1;
+      for (int r = 0; r < SPLIT_CL; ++r) mx = max(mx, cl.map_shared_rank(cmax, r)[k]);
+      c = mx < 0 ? NO_COLUMN : mx - 1023;
+    }
+    if (k < 512) ce[k] = (int16_t)c;
+    if (rank == 0) q.col_e[k] = (int16_t)c;
+  }
+  cl.sync();  // also keeps cmax alive until every peer has read it
+  for (int m = rank + SPLIT_CL * warp; m < q.M; m += SPLIT_CL * (SPLIT_T / 32)) {
+    const double* row = q.src + (long long)m * q.ld;
+    int E = -(1 << 19);
+    bool bad = false;
+    double x[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int k = 8 * (lane + 32 * i) + e;
+        x[i][e] = k < q.K ? row[k] : 0.0;
+        if (not_finite(x[i][e])) bad = true;
+        // the column's exponent moves to the input: subtract it here
+        else if (!is_zero(x[i][e])) E = max(E, elem_e(x[i][e], -(int)ce[k]));
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+    bad = __any_sync(0xffffffffu, bad);
+    if (bad) E = SPECIAL;
+    if (lane == 0) q.row_e[m] = E < -(1 << 18) ? 0 : E;
+    if (E < -(1 << 18)) E = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int k0 = 8 * (lane + 32 * i);
+      if (k0 >= q.Kp) continue;
+      unsigned long long f[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        f[e] = biased_fixed(x[i][e], elem_e(x[i][e], k0 + e < q.K ? -(int)ce[k0 + e] : 0), E);
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        uint4 v;
+        v.x = digit_pair(f[0], f[1], j);
+        v.y = digit_pair(f[2], f[3], j);
+        v.z = digit_pair(f[4], f[5], j);
+        v.w = digit_pair(f[6], f[7], j);
+        *reinterpret_cast<uint4*>(q.dig + ((long long)j * q.M + m) * q.Kp + k0) = v;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// the contraction
+// ---------------------------------------------------------------------------
+
+// MMAs that keep operand A in the collector buffer, or take it from there
+#define JFG_MMA_COLLECT(NAME, USAGE)                                                          \
+  __device__ __forceinline__ void NAME(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,    \
+                                       uint32_t accum) {                                      \
+    asm volatile(                                                                             \
+        "{\n\t.reg .pred p;\n\t"                                                             \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                          \
+        "tcgen05.mma.cta_group::1.kind::f16.collector::a::" USAGE " [%0], %1, %2, %3, p;\n\t}" \
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accum));                                    \
+  }
+JFG_MMA_COLLECT(mma_fill, "fill")
+JFG_MMA_COLLECT(mma_use, "use")
+JFG_MMA_COLLECT(mma_lastuse, "lastuse")
+#undef JFG_MMA_COLLECT
+
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(addr));
+}
+// wait for the loads into r[0..31] (the operands order the uses after it)
+__device__ __forceinline__ void tmem_wait32(uint32_t* r) {
+  asm volatile(
+      "tcgen05.wait::ld.sync.aligned;"
+      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+        "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
+        "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]),
+        "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]),
+        "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
+}
+
+__device__ __forceinline__ int level_int(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+// four levels as one integer: ((a 2^8 + b) 2^8 + c) 2^8 + d
+__device__ __forceinline__ long long level_join(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  return mad_wide(level_int(a), 1 << 24,
+                  mad_wide(level_int(b), 1 << 16, mad_wide(level_int(c), 1 << 8, level_int(d))));
+}
+
+// A rare element of the epilogue, summed as it stands and in the CUDA-core
+// path's order, so that it overflows, underflows and spreads specials the same
+// way: one whose rows hold an infinity or a NaN, whose terms are large enough
+// for a running sum to overflow, or whose exponent leaves the normal range.
+__device__ __noinline__ double plain_sum(const double* a, const double* y, int K) {
+  double v = 0.0;
+  for (int k = 0; k < K; ++k) v = fma(a[k], y[k], v);
+  return v;
+}
+
+// H + lo 2^-32 (both below 2^51 in magnitude) rounded to nearest even as a
+// double times 2^sh; rare is set when its exponent leaves the normal range.
+// No branches: the eight columns of a step run interleaved.
+__device__ __forceinline__ double level_value(long long H, long long lo, int sh, bool& rare) {
+  H += lo >> 32;
+  uint32_t w2 = (uint32_t)(H >> 32), w1 = (uint32_t)H, w0 = (uint32_t)lo;
+  const uint32_t s = (uint32_t)((int)w2 >> 31);
+  // magnitude of the 96-bit number: ones' complement and 1 if negative
+  asm("{\n\t"
+      "xor.b32 %0, %0, %3;\n\txor.b32 %1, %1, %3;\n\txor.b32 %2, %2, %3;\n\t"
+      "add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;\n\t}"
+      : "+r"(w0), "+r"(w1), "+r"(w2)
+      : "r"(s), "r"(s & 1u));
+  int e = sh + 1086;  // biased exponent of a number whose top bit is bit 95
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {  // whole words of leading zeros
+    const bool z = w2 == 0;
+    w2 = z ? w1 : w2;
+    w1 = z ? w0 : w1;
+    w0 = z ? 0u : w0;
+    e = z ? e - 32 : e;
+  }
+  const int z = __clz((int)w2);
+  w2 = __funnelshift_l(w1, w2, z);
+  w1 = __funnelshift_l(w0, w1, z);
+  w1 |= __funnelshift_l(0u, w0, z) != 0 ? 1u : 0u;  // what is cut off stays visible
+  e -= z;
+  // to 53 bits, ties to even; a carry out of the top leaves 2^64
+  uint32_t c;
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, 0, 0;"
+      : "+r"(w1), "+r"(w2), "=r"(c)
+      : "r"(0x3FFu + ((w1 >> 11) & 1u)));
+  w2 |= c << 31;
+  e += (int)c;
+  const bool nz = w2 != 0;
+  rare = nz && (unsigned)(e - 1) >= 2046u;
+  // the leading bit adds the 1 that the exponent field is short of
+  const uint32_t hi = ((w2 >> 11) + ((uint32_t)(e - 1) << 20)) | (s & 0x80000000u);
+  return __hiloint2double(nz ? (int)hi : 0, (int)__funnelshift_r(w1, w2, 11));
+}
+
+template <int EPI, bool BETA, int PT>
+__global__ void __launch_bounds__(SL_NT, 1)
+    k_contract_sl(const __grid_constant__ SlLaunch L) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int s_nb;
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const jfg_contract_desc& d = L.d;
+  constexpr uint32_t DBLK = (uint32_t)PT * 128;        // one digit of one K block
+  constexpr uint32_t KBLK = (NS + 1) * DBLK;           // zero block and digits
+  const uint32_t bbytes = (uint32_t)L.nkb * KBLK;
+  uint8_t* bs = smem;                                   // [bbuf][nkb][1 + NS][PT][64]
+  uint8_t* as = smem + (uint32_t)L.bbuf * bbytes;       // [astages]
+  double* stg = (double*)(as + (uint32_t)L.astages * ABYTES);
+  int* row_e = (int*)(stg + NWE * 32 * STG_LD);         // [RING][PT]
+  int16_t* col_e = (int16_t*)(row_e + RING * PT);       // [op_segs][kpad]
+  uint64_t* bars = (uint64_t*)(col_e + COL_MAX);
+  uint64_t* afull = bars;
+  uint64_t* aempty = bars + A_MAX;
+  uint64_t* bfull = bars + 2 * A_MAX;
+  uint64_t* bempty = bfull + 2;
+  uint64_t* dfull = bfull + 4;
+  uint64_t* dempty = bfull + 6;
+  uint64_t* done = bfull + 8;
+  uint32_t* tmem_slot = (uint32_t*)(bfull + 9);
+
+  // warp-uniform to the compiler, so that the MMA issuer's addresses stay in
+  // uniform registers
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    s_nb = active_count(d.batch_list, d.batch_count, d.batch);
+    for (int i = 0; i < A_MAX; ++i) {
+      tc::mbar_init(&afull[i], 1);
+      tc::mbar_init(&aempty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bfull[i], NWS);
+      tc::mbar_init(&bempty[i], 1);
+      tc::mbar_init(&dfull[i], 1);
+      tc::mbar_init(&dempty[i], NWE);
+    }
+    tc::mbar_init(done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < L.op_segs * L.kpad; i += SL_NT) col_e[i] = L.col_e[i];
+  for (int i = threadIdx.x; i < L.bbuf * L.nkb * (int)(DBLK / 16); i += SL_NT)
+    *reinterpret_cast<uint4*>(bs + (i / (DBLK / 16)) * KBLK + (i % (DBLK / 16)) * 16) =
+        make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc::smem_u32(tmem_slot)),
+                 "r"(2 * NS * PT)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  // items: (problem slot, segment, p tile), all operator tiles of each; with
+  // fewer of these than CTAs, every operator tile is an item of its own
+  const int nb = s_nb;
+  const unsigned base_items = (unsigned)nb * d.nseg * L.nptiles;
+  const int msplit = (base_items < gridDim.x) ? L.mtiles : 1;
+  const unsigned items = base_items * msplit;
+  const int mt_n = msplit > 1 ? 1 : L.mtiles;
+  auto decode = [&](unsigned t, int& mt0, int& pt, int& slot, int& s) {
+    mt0 = 0;
+    if (msplit > 1) {
+      mt0 = (int)(t % (unsigned)msplit);
+      t /= (unsigned)msplit;
+    }
+    pt = (int)(t % (unsigned)L.nptiles);
+    t /= (unsigned)L.nptiles;
+    slot = (int)(t / (unsigned)d.nseg);
+    s = (int)t - slot * d.nseg;
+  };
+
+  if (warp == 0) {
+    // ---------------- operator producer ----------------
+    if (lane == 0) {
+      if (L.a_res) {
+        for (int t = 0; t < L.mtiles * L.nkb * NS; ++t) {
+          const int i = t % NS, kb = (t / NS) % L.nkb, mt = t / NS / L.nkb;
+          tc::mbar_expect_tx(&afull[t], ABYTES);
+          tc::tma_load_3d(as + t * ABYTES, &L.amap, &afull[t], kb * 64, mt * 128, i);
+        }
+        for (int t = 0; t < L.mtiles * L.nkb * NS; ++t) tc::mbar_wait(&afull[t], 0, &g_sl_status);
+      } else {
+        int st = 0;
+        uint32_t ph = 0;
+        long long issued = 0;
+        bool ok = true;
+        for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
+          int mt0, pt, slot, s;
+          decode(t, mt0, pt, slot, s);
+          const int os = L.op_segs > 1 ? s : 0;
+          for (int mt = mt0; ok && mt < mt0 + mt_n; ++mt)
+            for (int kb = 0; ok && kb < L.nkb; ++kb)
+              for (int i = 0; i < NS; ++i) {
+                if (issued >= L.astages && !tc::mbar_wait(&aempty[st], ph ^ 1u, &g_sl_status)) {
+                  ok = false;
+                  break;
+                }
+                tc::mbar_expect_tx(&afull[st], ABYTES);
+                tc::tma_load_3d(as + st * ABYTES, &L.amap, &afull[st], kb * 64, mt * 128,
+                                os * NS + i);
+                ++issued;
+                if (++st == L.astages) {
+                  st = 0;
+                  ph ^= 1u;
+                }
+              }
+        }
+        // the last use of every stage must have landed before exit
+        for (long long q = issued > L.astages ? issued - L.astages : 0; q < issued; ++q)
+          tc::mbar_wait(&afull[q % L.astages], (uint32_t)(q / L.astages) & 1u, &g_sl_status);
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    // the whole warp walks the loop, one elected lane issues
+    const uint64_t ad0 = tc::sdesc_sw128(tc::smem_u32(as));
+    const uint64_t bd0 = tc::sdesc_sw128(tc::smem_u32(bs));
+    constexpr uint32_t idesc =  // FP16 x FP16 -> FP32, M = 128, N = 2 PT
+        (1u << 4) | ((uint32_t)(2 * PT) >> 3 << 17) | ((128u >> 4) << 24);
+    int st = 0, bslot = 0;
+    uint32_t aph = 0, bph = 0, unit = 0;
+    bool ok = true, any = false;
+    for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
+      if (!tc::mbar_wait(&bfull[bslot], bph, &g_sl_status)) {
+        ok = false;
+        break;
+      }
+      const uint64_t bdt = bd0 + (((uint32_t)bslot * bbytes) >> 4);
+      for (int mi = 0; ok && mi < mt_n; ++mi, ++unit) {
+        const uint32_t db = unit & 1u;
+        if (unit >= 2 && !tc::mbar_wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u, &g_sl_status)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + db * (NS * PT);
+        if (L.a_res) st = mi * L.nkb * NS;
+        for (int kb = 0; ok && kb < L.nkb; ++kb) {
+          const int rest = d.K - kb * 64;
+          const int n16 = rest >= 64 ? 4 : (rest + 15) / 16;
+          const uint64_t bdk = bdt + (((uint32_t)kb * KBLK) >> 4);
+#pragma unroll
+          for (int i = 0; i < NS; ++i) {
+            if (!tc::mbar_wait(&afull[st], aph, &g_sl_status)) {
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            any = true;
+            const uint64_t ad = ad0 + (((uint32_t)st * ABYTES) >> 4);
+            if (elect_one()) {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                if (kk >= n16) break;
+                const uint32_t more = (kb | kk | i) ? 1u : 0u;
+                // pairs h = (i + 1) / 2 .. 3 share the operator tile: it stays
+                // in the collector buffer from the first to the last
+#pragma unroll
+                for (int h = 3; h >= i / 2; --h) {
+                  const uint64_t bd = bdk + (((uint32_t)(2 * h - i + 1) * DBLK + 32 * kk) >> 4);
+                  const uint32_t D = acc + 2 * PT * h;
+                  if (h == 3 && h == i / 2)
+                    tc::mma_bf16(D, ad + 2 * kk, bd, idesc, more);
+                  else if (h == 3)
+                    mma_fill(D, ad + 2 * kk, bd, idesc, more);
+                  else if (h == i / 2)
+                    mma_lastuse(D, ad + 2 * kk, bd, idesc, more);
+                  else
+                    mma_use(D, ad + 2 * kk, bd, idesc, more);
+                }
+              }
+              if (!L.a_res) tc::mma_commit(&aempty[st]);
+            }
+            __syncwarp();
+            if (++st == L.astages) {
+              st = 0;
+              if (!L.a_res) aph ^= 1u;
+            }
+          }
+        }
+        if (ok && elect_one()) tc::mma_commit(&dfull[db]);
+        __syncwarp();
+      }
+      if (ok && elect_one()) tc::mma_commit(&bempty[bslot]);
+      __syncwarp();
+      if (++bslot == L.bbuf) {
+        bslot = 0;
+        bph ^= 1u;
+      }
+    }
+    if (any) {  // every MMA has finished before TMEM is freed
+      if (elect_one()) tc::mma_commit(done);
+      __syncwarp();
+      tc::mbar_wait(done, 0, &g_sl_status);
+    }
+  } else if (warp < 2 + NWS) {
+    // ---------------- cut the input rows into digits ----------------
+    constexpr int RW = PT / NWS;  // rows per warp
+    constexpr int UPR = 32 / RW;  // lanes per row, one chunk of 8 elements each per step
+    constexpr int STEPS = 4;      // chunks per lane: 8 UPR STEPS elements = 256 (PT 32) or 512
+    const int row = (warp - 2) * RW + lane % RW;
+    const int u = lane / RW;
+    // chunk of this lane within a step, so that the eight lanes of a
+    // quarter-warp store to different 16-byte columns of the swizzled rows
+    const int cu = PT == 32 ? ((u >> 1) | ((u & 1) << 2))
+                            : (((u & 3) << 1) | ((u >> 2) & 1) | (u & 8));
+    double x[STEPS][8];
+    auto load = [&](unsigned t) {
+      int mt0, pt, slot, s;
+      decode(t, mt0, pt, slot, s);
+      const int b = active_problem(d.batch_list, nb, d.batch, slot);
+      const int p = pt * PT + row;
+      const double* src = L.in + (long long)(b < 0 ? 0 : b) * d.in_batch +
+                          (long long)s * d.in_seg + (long long)p * d.in_ld;
+      const bool live = b >= 0 && p < d.P;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k0 = 8 * (cu + UPR * i);
+        if (live && k0 + 8 <= d.K) {
+          if (L.vec2) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              const double2 v = __ldg((const double2*)(src + k0 + e));
+              x[i][e] = v.x;
+              x[i][e + 1] = v.y;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[i][e] = __ldg(src + k0 + e);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            x[i][e] = live && k0 + e < d.K ? __ldg(src + k0 + e) : 0.0;
+        }
+      }
+      return s;
+    };
+    int bslot = 0, ring = 0;
+    uint32_t bph = 0;
+    unsigned n = 0;
+    int s = 0;
+    if (blockIdx.x < items) s = load(blockIdx.x);
+    for (unsigned t = blockIdx.x; t < items; t += gridDim.x, ++n) {
+      const int16_t* ce = col_e + (L.op_segs > 1 ? s : 0) * L.kpad;
+      int E = -(1 << 19);
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k0 = 8 * (cu + UPR * i);
+        if (k0 < L.kpad) {
+          const uint4 c = *reinterpret_cast<const uint4*>(ce + k0);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            bad = bad || not_finite(x[i][e]);
+            if (!is_zero(x[i][e])) E = max(E, elem_e(x[i][e], short_of(c, e)));
+          }
+        }
+      }
+#pragma unroll
+      for (int o = RW; o < 32; o <<= 1) {
+        E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+        bad = __shfl_xor_sync(0xffffffffu, (int)bad, o) || bad;
+      }
+      if (E < -(1 << 18)) E = 0;
+      if (bad) E = SPECIAL;
+      if (n >= (unsigned)L.bbuf && !tc::mbar_wait(&bempty[bslot], bph ^ 1u, &g_sl_status)) break;
+      if (u == 0) row_e[ring * PT + row] = E;
+      uint8_t* dst = bs + (uint32_t)bslot * bbytes + DBLK + row * 128;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int q = cu + UPR * i, k0 = 8 * q;
+        if (k0 < L.kpad) {
+          const uint4 c = *reinterpret_cast<const uint4*>(ce + k0);
+          unsigned long long f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = biased_fixed(x[i][e], elem_e(x[i][e], short_of(c, e)), E);
+          uint8_t* o = dst + (uint32_t)(q >> 3) * KBLK + (((q & 7) ^ (row & 7)) << 4);
+#pragma unroll
+          for (int j = 0; j < NS; ++j) {
+            uint4 v;
+            v.x = digit_pair(f[0], f[1], j);
+            v.y = digit_pair(f[2], f[3], j);
+            v.z = digit_pair(f[4], f[5], j);
+            v.w = digit_pair(f[6], f[7], j);
+            *reinterpret_cast<uint4*>(o + j * DBLK) = v;
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bfull[bslot]);
+      if (t + gridDim.x < items) s = load(t + gridDim.x);
+      ring = (ring + 1) & (RING - 1);
+      if (++bslot == L.bbuf) {
+        bslot = 0;
+        bph ^= 1u;
+      }
+    }
+  } else {
+    // ---------------- epilogue ----------------
+    const int ew = warp - 2 - NWS;
+    const int quarter = warp & 3, half = ew >> 2;
+    double* st8 = stg + ew * 32 * STG_LD;
+    const int sr = lane >> 3, sc = lane & 7;
+    int ring = 0;
+    uint32_t unit = 0;
+    bool ok = true;
+    for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
+      int mt0, pt, slot, s;
+      decode(t, mt0, pt, slot, s);
+      const int b = active_problem(d.batch_list, nb, d.batch, slot);
+      const int os = L.op_segs > 1 ? s : 0;
+      const long long ib = (long long)(b < 0 ? 0 : b) * d.in_batch + (long long)s * d.in_seg;
+      double* outS = L.out + (long long)(b < 0 ? 0 : b) * d.out_batch + (long long)s * d.out_seg;
+      double c0 = 0.0, c1 = 1.0;
+      if (EPI == JFG_EPI_DIV_EIG && b >= 0) {
+        if (d.c0) c0 = ((const double*)d.c0)[b];
+        if (d.c1) c1 = ((const double*)d.c1)[b];
+      }
+      for (int mt = mt0; mt < mt0 + mt_n; ++mt, ++unit) {
+        const int m0 = mt * 128 + 32 * quarter;
+        const int m = m0 + lane;
+        const int Ea = m < d.M ? __ldg(L.row_e + (long long)os * L.row_ld + m) : 0;
+        const uint32_t db = unit & 1u;
+        if (!tc::mbar_wait(&dfull[db], (unit >> 1) & 1u, &g_sl_status)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + db * (NS * PT) + ((uint32_t)(32 * quarter) << 16);
+#pragma unroll 1
+        for (int cb = 0; cb < PT / 16; ++cb) {
+          const int col0 = half * (PT / 2) + cb * 8;
+          long long H[8];
+          uint32_t r[32];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tmem_ld8(acc + j * PT + col0, r + 8 * j);
+          tmem_wait32(r);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) H[c] = level_join(r[c], r[8 + c], r[16 + c], r[24 + c]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tmem_ld8(acc + (4 + j) * PT + col0, r + 8 * j);
+          tmem_wait32(r);
+          if (cb == PT / 16 - 1) {  // the accumulators are read: the next tile may have them
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&dempty[db]);
+          }
+          int Ep[8];
+#pragma unroll
+          for (int c = 0; c < 8; c += 4)
+            *reinterpret_cast<int4*>(Ep + c) =
+                *reinterpret_cast<const int4*>(row_e + ring * PT + col0 + c);
+          unsigned rare = 0;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            bool x;
+            st8[lane * STG_LD + c] =
+                level_value(H[c], level_join(r[c], r[8 + c], r[16 + c], r[24 + c]),
+                            Ea + Ep[c] - 2080, x);
+            rare |= (x || Ea + Ep[c] >= BIG) ? 1u << c : 0u;
+          }
+          if (rare && m < d.M && b >= 0) {
+            const double* a = L.op + (long long)os * d.op_seg + (long long)m * d.op_ld;
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) {
+              const int p = pt * PT + col0 + c;
+              if ((rare >> c & 1u) && p < d.P)
+                st8[lane * STG_LD + c] = plain_sum(a, L.in + ib + (long long)p * d.in_ld, d.K);
+            }
+          }
+          __syncwarp();
+          const int p = pt * PT + col0 + sc;
+          if (p < d.P && b >= 0) {
+            const double lp = EPI == JFG_EPI_DIV_EIG ? __ldg((const double*)d.lam_p + p) : 0.0;
+            double* o = outS + (long long)(m0 + sr) * d.out_ld + p;
+            const double* f = (const double*)d.field + (long long)b * d.field_batch +
+                              (long long)s * d.field_seg + (long long)(m0 + sr) * d.field_ld + p;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int mm = m0 + 4 * i + sr;
+              if (mm < d.M) {
+                double v = st8[(4 * i + sr) * STG_LD + sc];
+                if (EPI == JFG_EPI_MUL_FIELD)
+                  v *= __ldg(f);
+                else if (EPI == JFG_EPI_DIV_EIG)
+                  v = v / (c0 + c1 * (__ldg((const double*)d.lam_m + mm) + lp));
+                if (L.scaled) v *= d.alpha;
+                if (BETA) v += d.beta * *o;
+                *o = v;
+              }
+              o += 4 * d.out_ld;
+              if (EPI == JFG_EPI_MUL_FIELD) f += 4 * d.field_ld;
+            }
+          }
+          __syncwarp();
+        }
+      }
+      ring = (ring + 1) & (RING - 1);
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(2 * NS * PT));
+  }
+}
+
+template <int EPI, bool BETA>
+int set_attr() {
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, BETA, 32>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SMEM_LIMIT - 1024));
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, BETA, 16>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SMEM_LIMIT - 1024));
+  return JFG_OK;
+}
+
+// once per device: shared-memory opt-in (call before a capture)
+int device_setup(int* sms) {
+  static int nsm[64] = {};
+  int dev = 0;
+  JFG_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
+  if (!nsm[dev]) {
+    JFG_TRY((set_attr<JFG_EPI_NONE, false>()));
+    JFG_TRY((set_attr<JFG_EPI_NONE, true>()));
+    JFG_TRY((set_attr<JFG_EPI_MUL_FIELD, false>()));
+    JFG_TRY((set_attr<JFG_EPI_MUL_FIELD, true>()));
+    JFG_TRY((set_attr<JFG_EPI_DIV_EIG, false>()));
+    JFG_TRY((set_attr<JFG_EPI_DIV_EIG, true>()));
+    int n = 0;
+    JFG_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    nsm[dev] = n;
+  }
+  *sms = nsm[dev];
+  return JFG_OK;
+}
+
+inline int kp8(int K) { return (K + 7) / 8 * 8; }
+inline int kp64(int K) { return (K + 63) / 64 * 64; }
+
+template <int PT>
+int launch(const SlLaunch& L, dim3 grid, size_t smem, cudaStream_t st) {
+  const bool beta = L.d.beta != 0.0;
+#define JFG_SL(E)                                                        \
+  if (beta)                                                              \
+    k_contract_sl<E, true, PT><<<grid, SL_NT, smem, st>>>(L);            \
+  else                                                                   \
+    k_contract_sl<E, false, PT><<<grid, SL_NT, smem, st>>>(L)
+  switch (L.d.epilogue) {
+    case JFG_EPI_NONE:
+      JFG_SL(JFG_EPI_NONE);
+      break;
+    case JFG_EPI_MUL_FIELD:
+      JFG_SL(JFG_EPI_MUL_FIELD);
+      break;
+    default:
+      JFG_SL(JFG_EPI_DIV_EIG);
+      break;
+  }
+#undef JFG_SL
+  JFG_LAUNCHED();
+  return JFG_OK;
+}
+
+}  // namespace
+
+size_t sl_op_bytes(int nseg, int M, int K) {
+  if (K < 1 || K > SL_KMAX || M < 1 || nseg < 1) return 0;
+  return align_up((size_t)nseg * NS * M * kp8(K) * 2, 256) + align_up((size_t)nseg * M * 4, 256) +
+         align_up((size_t)nseg * kp64(K) * 2, 256);
+}
+
+SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, void* work) {
+  SlOp o;
+  o.src = src;
+  o.ld = ld;
+  o.seg = seg;
+  o.nseg = nseg;
+  o.M = M;
+  o.K = K;
+  if (!work || K > SL_KMAX) return o;
+  char* w = (char*)work;
+  o.dig = (uint16_t*)w;
+  w += align_up((size_t)nseg * NS * M * kp8(K) * 2, 256);
+  o.row_e = (int*)w;
+  w += align_up((size_t)nseg * M * 4, 256);
+  o.col_e = (int16_t*)w;
+  return o;
+}
+
+int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st) {
+  SlSplitArgs A;
+  int n = 0;
+  for (int i = 0; i < nops; ++i) {
+    const SlOp& o = ops[i];
+    if (!o.dig) continue;
+    if (!o.src || o.K > SL_KMAX) return JFG_ERR_ARG;
+    const int Kp = kp8(o.K), kpad = kp64(o.K);
+    for (int s = 0; s < o.nseg; ++s) {
+      if (n == SL_MAX_SEGS) return JFG_ERR_ARG;
+      A.s[n++] = SlSeg{o.src + s * o.seg,
+                       o.ld,
+                       o.M,
+                       o.K,
+                       Kp,
+                       kpad,
+                       o.dig + (size_t)s * NS * o.M * Kp,
+                       o.row_e + (size_t)s * o.M,
+                       o.col_e + (size_t)s * kpad};
+    }
+  }
+  if (n == 0) return JFG_OK;
+  k_sl_split<<<n * SPLIT_CL, SPLIT_T, 0, st>>>(A);
+  JFG_LAUNCHED();
+  return JFG_OK;
+}
+
+bool sl_pays(const jfg_contract_desc& d, double min_work) {
+  if (d.K > SL_KMAX || d.M < 1 || d.M > 65536 || d.P < 1 || d.batch < 1 || d.nseg > 3 ||
+      (long long)d.batch * d.nseg > 65535 ||
+      (long long)d.batch * d.nseg * ((d.P + 15) / 16) * ((d.M + 127) / 128) > 0x3FFFFFFF)
+    return false;
+  const int t = contract_f64_tile(d);
+  const double tiles = (double)d.batch * d.nseg * ((d.M + t - 1) / t) * ((d.P + t - 1) / t);
+  return tiles * t * t * ((d.K + 15) / 16 * 16) >= min_work;
+}
+
+int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, double* out,
+                cudaStream_t st) {
+  JFG_TRY(validate_desc(d));
+  if (!in || !out || !op.dig || d.K != op.K || d.M > op.M || d.K > SL_KMAX) return JFG_ERR_ARG;
+  if (op.nseg != 1 && op.nseg < d.nseg) return JFG_ERR_ARG;
+  if (d.batch == 0 || d.M == 0 || d.P == 0) return JFG_OK;
+  if ((long long)d.batch * d.nseg > 65535) return JFG_ERR_ARG;
+  int sms = 0;
+  JFG_TRY(device_setup(&sms));
+  EncodeTiledFn enc = tensor_map_encoder();
+  if (!enc) return JFG_ERR_UNSUPPORTED;
+  SlLaunch L = {};
+  L.d = d;
+  L.d.op_ld = op.ld;
+  L.d.op_seg = op.seg;
+  L.op = op.src;
+  L.in = in;
+  L.out = out;
+  L.row_e = op.row_e;
+  L.col_e = op.col_e;
+  L.op_segs = d.nseg > 1 && op.nseg > 1 ? d.nseg : 1;
+  L.row_ld = op.M;
+  L.kpad = kp64(d.K);
+  L.nkb = L.kpad / 64;
+  L.mtiles = (d.M + 127) / 128;
+  if (L.op_segs * L.kpad > COL_MAX) return JFG_ERR_UNSUPPORTED;
+  // PT 32 streams each operator digit past twice the rows that 16 does; 16
+  // where K > 256 would not fit, or 32 would leave half the SMs without work
+  const long long t32 = (long long)d.batch * d.nseg * ((d.P + 31) / 32) * L.mtiles;
+  const int PT = (d.K > 256 || (2 * t32 <= sms && d.P > 16)) ? 16 : 32;
+  L.nptiles = (d.P + PT - 1) / PT;
+  const long long items = (long long)d.batch * d.nseg * L.nptiles * L.mtiles;
+  if (items > 0x3FFFFFFF) return JFG_ERR_UNSUPPORTED;
+  const size_t bbytes = (size_t)L.nkb * PT * (NS + 1) * 128;
+  L.bbuf = 2 * bbytes <= 144 * 1024 ? 2 : 1;
+  const size_t fixed = 1024 + L.bbuf * bbytes + NWE * 32 * STG_LD * 8 + RING * PT * 4 +
+                       COL_MAX * 2 + (2 * A_MAX + 10) * 8;
+  const size_t room = (SMEM_LIMIT - 1024 - fixed) / ABYTES;
+  L.astages = room > A_MAX ? A_MAX : (int)room;
+  if (L.astages < 2) return JFG_ERR_UNSUPPORTED;
+  L.a_res = L.op_segs == 1 && L.mtiles * L.nkb * NS <= L.astages ? 1 : 0;
+  L.vec2 = ((uintptr_t)in & 15) == 0 && !(d.in_ld & 1) && !(d.in_seg & 1) && !(d.in_batch & 1);
+  L.scaled = d.alpha != 1.0;
+  const int Kp = kp8(d.K);
+  const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)op.M, (cuuint64_t)(op.nseg * NS)};
+  const cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * op.M};
+  const cuuint32_t box[3] = {64, 128, 1}, estr[3] = {1, 1, 1};
+  if (enc(&L.amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)op.dig, dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return JFG_ERR_ARG;
+  const dim3 grid((unsigned)(items < sms ? items : sms));
+  const size_t smem = fixed + (size_t)L.astages * ABYTES;
+  return PT == 32 ? launch<32>(L, grid, smem, st) : launch<16>(L, grid, smem, st);
+}
+
+int sl_setup() {
+  int sms = 0;
+  JFG_TRY(device_setup(&sms));
+  return tensor_map_encoder() ? JFG_OK : JFG_ERR_UNSUPPORTED;
+}
+
+int sl_status_take(int* status) {
+  int zero = 0;
+  JFG_CUDA_TRY(cudaMemcpyFromSymbol(status, g_sl_status, sizeof(int)));
+  JFG_CUDA_TRY(cudaMemcpyToSymbol(g_sl_status, &zero, sizeof(int)));
+  return JFG_OK;
+}
+
+}  // namespace jfg

@@ -1846,12 +1846,14 @@ extern "C" int jfg_tc_autotune(int ngroups, const jfg_contract_desc* descs,
 }
 
 extern "C" int jfg_device_status(void) {
-  int s = 0, g = 0;
+  int s = 0, g = 0, sl = 0;
   int r = jfg::tc_status_take(&s);
   if (r != JFG_OK) return r;
   r = jfg::gemm_status_take(&g);
   if (r != JFG_OK) return r;
-  return s != JFG_OK ? s : g;
+  r = jfg::sl_status_take(&sl);
+  if (r != JFG_OK) return r;
+  return s != JFG_OK ? s : g != JFG_OK ? g : sl;
 }
 
 extern "C" void jfg_split_tf32_host(size_t n, const double* src, float* hi, float* lo) {

@@ -88,6 +88,8 @@ struct DotOut {
   int* nb = nullptr;
 };
 
+// tile of the FP64 CUDA-core launch (64, 32 or 16)
+int contract_f64_tile(const jfg_contract_desc& d);
 int contract_f64(const jfg_contract_desc& d, const double* op, const double* in, double* out,
                  cudaStream_t st);
 int contract_f32(const jfg_contract_desc& d, const float* op, const float* in, float* out,
@@ -121,6 +123,47 @@ int single_autotune();
 // One-time per-device setup of the tensor-core kernels (shared-memory opt-in,
 // tensor-map encoder); call before capturing their first launch into a graph.
 int tc_setup();
+
+// An FP64 operator cut into FP16 digits for the tensor-core FP64 contraction
+// (contract_sl.cu): where the operator itself lies and, in a workspace of
+// sl_op_bytes, its digits, row exponents and column exponents.
+constexpr int SL_KMAX = 512;      // largest contracted extent
+constexpr int SL_MAX_SEGS = 8;    // operator segments cut in one launch
+// CUDA-core multiply-adds of a pass (its tiles' padding included) from which
+// the tensor-core contraction is faster: when the operator is cut in the same
+// call, and when it has been cut before.  Two passes of 32 x 64^2 (8.4e6
+// each): 31.5 us cut in the call against 41.9 us; of 16 x 64^2: 31.7 against
+// 25.4 us, of which the cut is ~9 us.
+constexpr double SL_MIN_WORK = 8e6;
+constexpr double SL_MIN_WORK_CUT = 4e6;
+struct SlOp {
+  const double* src = nullptr;
+  long long ld = 0, seg = 0;
+  int nseg = 0, M = 0, K = 0;
+  uint16_t* dig = nullptr;  // null: not cut, the CUDA-core contraction serves it
+  int* row_e = nullptr;
+  int16_t* col_e = nullptr;
+  // segment s alone
+  SlOp segment(int s) const {
+    SlOp o = *this;
+    o.src += s * seg;
+    o.nseg = 1;
+    if (dig) {
+      o.dig += (size_t)s * 8 * M * ((K + 7) / 8 * 8);
+      o.row_e += (size_t)s * M;
+      o.col_e += (size_t)s * ((K + 63) / 64 * 64);
+    }
+    return o;
+  }
+};
+size_t sl_op_bytes(int nseg, int M, int K);  // 0 when K > SL_KMAX
+SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, void* work);
+int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st);  // operators without dig are skipped
+bool sl_pays(const jfg_contract_desc& d, double min_work = SL_MIN_WORK);
+int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, double* out,
+                cudaStream_t st);
+int sl_setup();
+int sl_status_take(int* status);
 
 inline int contract(Engine e, const jfg_contract_desc& d, OpRef<double> op, const double* in,
                     double* out, cudaStream_t st) {
@@ -195,15 +238,28 @@ template <typename T>
 int tp_apply(Engine e, int ndim, const int* rows, const int* cols, int batch,
              const OpRef<T>* mats, const T* in, T* out, void* work, size_t work_bytes,
              cudaStream_t st, const T* shift = nullptr);
+// sl (FP64): E and W cut by the caller (fd_sl_ops); null: cut in the call
+// when the workspace has room for them and a pass is large enough
 template <typename T>
 int fd_solve(Engine e, int ndim, int n, int batch, OpRef<T> E, OpRef<T> W, const T* lam,
              const T* c0, const T* c1, const T* rhs, T* out, void* work, size_t work_bytes,
-             cudaStream_t st, Active act = Active(), const DotOut* dot = nullptr);
+             cudaStream_t st, Active act = Active(), const DotOut* dot = nullptr,
+             const SlOp* sl = nullptr);
+// sl (FP64): the packed operators cut by the caller (varcoef_sl_ops)
 template <typename T>
 int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, const T* kw,
                   const T* u, T* v, void* work, size_t work_bytes, cudaStream_t st,
                   Active act = Active(), const H16Ops* h16 = nullptr,
-                  const DotOut* dot = nullptr);
+                  const DotOut* dot = nullptr, const SlOp* sl = nullptr);
+// Workspace and layout of the cut operators of fd_solve (2: E, W) and
+// varcoef_apply (SL_VARCOEF); sl_split_ops cuts them.
+constexpr int SL_VARCOEF = 4;
+size_t fd_sl_bytes(int n);
+void fd_sl_ops(int n, const double* E, const double* W, void* work, SlOp* out);
+// whether a varcoef_apply is large enough to cut its operators for it
+bool varcoef_pays(int ndim, int n, int nq, int batch, double min_work);
+size_t varcoef_sl_bytes(int ndim, int n, int nq);
+void varcoef_sl_ops(int ndim, int n, int nq, const double* ops, void* work, SlOp* out);
 // number of inverse row scales of the 2-D packed operators (TH engine)
 inline long long varcoef_h16_rows(int n, int nq) { return 4LL * nq + 3LL * n; }
 inline long long varcoef_h16_rows_nd(int ndim, int n, int nq) {
@@ -213,7 +269,10 @@ inline long long varcoef_h16_rows_nd(int ndim, int n, int nq) {
 // Read and clear the device status word of the BF16 GEMM kernel.
 int gemm_status_take(int* status);
 
+// Scratch of the pass sequences (with room for cut FP64 operators: *_ws_sl;
+// the sequences accept either and cut in the call when there is room).
 size_t tp_apply_ws(int ndim, const int* rows, const int* cols, int batch, int eb);
+size_t tp_apply_ws_sl(int ndim, const int* rows, const int* cols, int batch, int eb);
 size_t fd_ws(int ndim, int n, int batch, int eb);
 size_t varcoef_ws(int ndim, int n, int nq, int batch, int eb);
 

@@ -296,9 +296,10 @@ MixedLayout layout(int ndim, int n, int nq, int batch) {
   L.vec32 = align_up((size_t)L.Npad * batch * 4, 256);
   L.ws64 = align_up(varcoef_ws(ndim, n, nq, batch, 8), 256);
   L.wsin = pcg_ws<float>(ndim, nq, nq, batch);
-  // the FP64 operator split once per solve into (hi, lo) pairs for the
-  // double-FP32 residual passes
+  // the FP64 operator split once per solve: into (hi, lo) pairs for the
+  // double-FP32 residual passes, or cut into digits for the tensor cores
   L.opdf = align_up((size_t)8 * n * nq * sizeof(float2), 256);
+  if (varcoef_sl_bytes(ndim, n, nq) > L.opdf) L.opdf = varcoef_sl_bytes(ndim, n, nq);
   // per-problem outer state: ||rhs||, outer count, state, residual kind, four
   // lists and a control block
   L.outer = align_up((size_t)batch * 8, 256) + 7 * align_up((size_t)batch * 4, 256) + 256;
@@ -562,7 +563,29 @@ extern "C" int jfg_pcg_varcoef_mixed_guess(const jfg_mixed_plan* plan, const dou
   void* wsin = w;
   w += Lo.wsin;
   float2* opdf = (float2*)w;
-  if (P.residual == 1) JFG_TRY(split_pairs_f64(P.ops64, opdf, 8LL * n * nq, st));
+  // The recomputed residuals r = b - A x, in 2-D: FP64 on the tensor cores
+  // (both values of P.residual) from the size on where that is the faster way
+  // (128 problems, N = 256: the solve 55.8 -> 49.9 ms), else double-FP32 or
+  // FP64 on the CUDA cores.  3-D keeps the latter: at 128^3 its stopping rule
+  // leaves ~1e-9 of the answer to the rounding of the whole path, and another
+  // residual arithmetic moved answers by up to 1.2e-9 (as far from the tight
+  // solution as before).
+  SlOp cut[SL_VARCOEF];
+  const bool sl = ndim == 2 && varcoef_pays(ndim, n, nq, batch, SL_MIN_WORK_CUT);
+  if (sl) {
+    varcoef_sl_ops(ndim, n, nq, P.ops64, opdf, cut);
+    JFG_TRY(sl_setup());
+    JFG_TRY(sl_split_ops(cut, SL_VARCOEF, st));
+  } else if (P.residual == 1) {
+    JFG_TRY(split_pairs_f64(P.ops64, opdf, 8LL * n * nq, st));
+  }
+  const bool df = !sl && P.residual == 1;
+  const OpRef<double> ops64{P.ops64, df ? (const double*)opdf : nullptr};
+  auto apply64 = [&](const double* u, double* v, void* ws, size_t ws_bytes, Active act) -> int {
+    return varcoef_apply<double>(df ? Engine::DF : Engine::F64, ndim, n, nq, batch, ops64, P.kw64,
+                                 u, v, ws, ws_bytes, st, act, nullptr, nullptr,
+                                 sl ? cut : nullptr);
+  };
 
   PcgProblem<float> pb;
   pb.engine = P.apply_f16 ? Engine::TH : Engine::TC;
@@ -592,10 +615,7 @@ extern "C" int jfg_pcg_varcoef_mixed_guess(const jfg_mixed_plan* plan, const dou
   const dim3 ugrid(blocks_for(Lo.Nun, 256), batch);
   const dim3 sgrid(NBS, batch);
   auto residual = [&]() -> int {
-    JFG_TRY(varcoef_apply<double>(
-        P.residual == 1 ? Engine::DF : Engine::F64, ndim, n, nq, batch,
-        OpRef<double>{P.ops64, P.residual == 1 ? (const double*)opdf : nullptr}, P.kw64, x, r64,
-        ws64, Lo.ws64, st));
+    JFG_TRY(apply64(x, r64, ws64, Lo.ws64, Active()));
     k_sub_from64<<<blocks_for(tot64, 4096), 256, 0, st>>>(rhs, r64, tot64);
     JFG_LAUNCHED();
     return JFG_OK;
@@ -682,10 +702,7 @@ extern "C" int jfg_pcg_varcoef_mixed_guess(const jfg_mixed_plan* plan, const dou
                                         ctrl, batch);
     JFG_LAUNCHED();
     // recomputed residuals r = rhs - A x
-    JFG_TRY(varcoef_apply<double>(
-        P.residual == 1 ? Engine::DF : Engine::F64, ndim, n, nq, batch,
-        OpRef<double>{P.ops64, P.residual == 1 ? (const double*)opdf : nullptr}, P.kw64, x, r64,
-        ws64, Lo.ws64, st, Active{rdf, ctrl + 1}));
+    JFG_TRY(apply64(x, r64, ws64, Lo.ws64, Active{rdf, ctrl + 1}));
     k_sub_from64_list<<<ugrid, 256, 0, st>>>(rhs, r64, Lo.Nun, rdf, ctrl + 1, batch);
     JFG_LAUNCHED();
     // updated residuals r -= ||r|| A32 d (the apply's scratch is the inner

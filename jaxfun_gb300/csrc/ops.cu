@@ -47,6 +47,36 @@ size_t tp_apply_ws(int ndim, const int* rows, const int* cols, int batch, int eb
   return 2 * tp_inter_bytes(ndim, rows, cols, batch, eb) + align_up(ops * sizeof(float2), 256);
 }
 
+// the axes whose pass is large enough for the tensor-core FP64 contraction
+static void tp_sl_axes(int ndim, const int* rows, const int* cols, int batch, bool* on) {
+  double rest = 1;  // the field at axis i: later axes are already rows
+  for (int i = 0; i < ndim; ++i) rest *= cols[i];
+  for (int i = ndim - 1; i >= 0; --i) {
+    const double P = rest / cols[i];
+    rest = P * rows[i];
+    on[i] = P <= 2147483647.0 && sl_pays(make_desc(batch, rows[i], (int)P, cols[i]));
+  }
+}
+
+// with room for the operators of those axes cut into digits behind it (FP64)
+size_t tp_apply_ws_sl(int ndim, const int* rows, const int* cols, int batch, int eb) {
+  size_t b = tp_apply_ws(ndim, rows, cols, batch, eb);
+  if (eb != 8 || ndim < 1 || ndim > 3) return b;
+  bool on[3];
+  tp_sl_axes(ndim, rows, cols, batch, on);
+  for (int i = 0; i < ndim; ++i)
+    if (on[i]) b += sl_op_bytes(1, rows[i], cols[i]);
+  return b;
+}
+
+// One FP64 pass: on the tensor cores when its operator has been cut and the
+// pass is large enough, else on the CUDA cores.
+static int contract_f64_or_sl(const jfg_contract_desc& d, const SlOp* sl, const double* op,
+                              const double* in, double* out, cudaStream_t st) {
+  if (sl && sl->dig && sl_pays(d, SL_MIN_WORK_CUT)) return contract_sl(d, *sl, in, out, st);
+  return contract_f64(d, op, in, out, st);
+}
+
 // out[i] = shift[i % per] for i < total: the constant field of an affine
 // transform, written before the last pass accumulates into it (beta = 1)
 template <typename T>
@@ -71,10 +101,36 @@ int tp_apply(Engine e, int ndim, const int* rows, const int* cols, int batch,
   if (ndim > 1 && (!work || work_bytes < need)) return JFG_ERR_WORKSPACE;
   const size_t inter = tp_inter_bytes(ndim, rows, cols, batch, (int)sizeof(T));
   T* buf[2] = {(T*)work, (T*)((char*)work + inter)};
+  // FP64 data: with room for them, the operators of passes large enough for the
+  // tensor-core contraction are cut into digits, equal ones once
+  SlOp sl[3];
+  if constexpr (std::is_same<T, double>::value) {
+    if ((e == Engine::F64 || e == Engine::DF) && batch > 0 && work &&
+        work_bytes >= tp_apply_ws_sl(ndim, rows, cols, batch, 8)) {
+      char* w = (char*)work + need;
+      SlOp todo[3];
+      int n = 0;
+      bool on[3];
+      tp_sl_axes(ndim, rows, cols, batch, on);
+      for (int i = ndim - 1; i >= 0; --i) {
+        if (!on[i]) continue;
+        for (int j = i + 1; j < ndim && !sl[i].dig; ++j)
+          if (sl[j].dig && mats[j].hi == mats[i].hi && rows[j] == rows[i] && cols[j] == cols[i])
+            sl[i] = sl[j];
+        if (sl[i].dig) continue;
+        sl[i] = todo[n++] = sl_op((const double*)mats[i].hi, cols[i], 0, 1, rows[i], cols[i], w);
+        w += sl_op_bytes(1, rows[i], cols[i]);
+      }
+      JFG_TRY(sl_split_ops(todo, n, st));
+    }
+  }
+
   // Double-FP32: split every operator once into (hi, lo) pairs and keep the
   // intermediates split between the passes (no FP64 work in the tile loads)
-  const bool dfp = std::is_same<T, double>::value && e == Engine::DF && work &&
-                   work_bytes >= need && batch > 0;
+  const bool df = std::is_same<T, double>::value && e == Engine::DF && work &&
+                  work_bytes >= need && batch > 0;
+  // (only when no pass runs on the tensor cores, whose fields are FP64)
+  const bool dfp = df && !sl[0].dig && !sl[1].dig && !sl[2].dig;
   OpRef<T> opr[3];
   for (int i = 0; i < ndim; ++i) opr[i] = mats[i];
   if (dfp) {
@@ -114,6 +170,9 @@ int tp_apply(Engine e, int ndim, const int* rows, const int* cols, int batch,
     if (dfp)
       JFG_TRY(contract_df64(d, (const double*)opr[ax].hi, (const float2*)opr[ax].lo,
                             (const double*)src, (double*)dst, st, t > 0, t < ndim - 1));
+    else if (sl[ax].dig)
+      JFG_TRY(contract_f64_or_sl(d, &sl[ax], (const double*)mats[ax].hi, (const double*)src,
+                                 (double*)dst, st));
     else
       JFG_TRY(contract(e, d, mats[ax], src, dst, st));
     for (int i = ndim - 1; i > 0; --i) shape[i] = shape[i - 1], order[i] = order[i - 1];
@@ -140,10 +199,22 @@ size_t fd_ws(int ndim, int n, int batch, int eb) {
   return 2 * align_up(field * eb, 256) + align_up((size_t)n * n * eb, 256);
 }
 
+// the pass that decides whether the operators are cut
+static bool fd_pays(int ndim, int n, int batch, double min_work) {
+  const double P = ndim == 3 ? (double)n * n : n;
+  return P <= 2147483647.0 && sl_pays(make_desc(batch, n, (int)P, n), min_work);
+}
+
+size_t fd_sl_bytes(int n) { return 2 * sl_op_bytes(1, n, n); }
+void fd_sl_ops(int n, const double* E, const double* W, void* work, SlOp* out) {
+  out[0] = sl_op(E, n, 0, 1, n, n, work);
+  out[1] = sl_op(W, n, 0, 1, n, n, (char*)work + sl_op_bytes(1, n, n));
+}
+
 template <typename T>
 int fd_solve(Engine e, int ndim, int n, int batch, OpRef<T> E, OpRef<T> W, const T* lam,
              const T* c0, const T* c1, const T* rhs, T* out, void* work, size_t work_bytes,
-             cudaStream_t st, Active act, const DotOut* dot) {
+             cudaStream_t st, Active act, const DotOut* dot, const SlOp* sl) {
   if (dot && dot->nb) *dot->nb = 0;
   if ((ndim != 2 && ndim != 3) || n < 1 || batch < 0 || !E.hi || !W.hi || !lam || !rhs ||
       !out)
@@ -162,6 +233,15 @@ int fd_solve(Engine e, int ndim, int n, int batch, OpRef<T> E, OpRef<T> W, const
     count_launches(1);
   }
   long long P = (long long)n * (ndim == 3 ? n : 1);
+  SlOp own[2];
+  if constexpr (std::is_same<T, double>::value) {
+    if (!sl && e == Engine::F64 && n <= SL_KMAX && work_bytes >= need + fd_sl_bytes(n) &&
+        fd_pays(ndim, n, batch, SL_MIN_WORK)) {
+      fd_sl_ops(n, (const double*)E.hi, (const double*)W.hi, (char*)work + need, own);
+      JFG_TRY(sl_split_ops(own, 2, st));
+      sl = own;
+    }
+  }
   const T* src = rhs;
   int b = 0;
   for (int t = 0; t < 2 * ndim; ++t) {
@@ -177,6 +257,8 @@ int fd_solve(Engine e, int ndim, int n, int batch, OpRef<T> E, OpRef<T> W, const
     if constexpr (std::is_same<T, float>::value) {
       // the divide pass can fuse r.M^-1 r (sum of acc * out)
       JFG_TRY(contract(e, d, t < ndim ? E : W, src, dst, st, t == ndim - 1 ? dot : nullptr));
+    } else if (sl) {
+      JFG_TRY(contract_f64_or_sl(d, sl + (t < ndim ? 0 : 1), t < ndim ? E.hi : W.hi, src, dst, st));
     } else {
       JFG_TRY(contract(e, d, t < ndim ? E : W, src, dst, st));
     }
@@ -206,10 +288,35 @@ size_t varcoef_ws(int ndim, int n, int nq, int batch, int eb) {
   return align_up(a * batch * eb, 256) + align_up(b * batch * eb, 256);
 }
 
+bool varcoef_pays(int ndim, int n, int nq, int batch, double min_work) {
+  const double P = ndim == 2 ? nq : (double)nq * nq;
+  return P <= 2147483647.0 && sl_pays(make_desc(batch, nq, (int)P, n), min_work);
+}
+
+// the operators of the passes below, in their order
+size_t varcoef_sl_bytes(int ndim, int n, int nq) {
+  if (ndim == 2)
+    return sl_op_bytes(1, 2 * nq, n) + sl_op_bytes(2, nq, n) + sl_op_bytes(2, n, nq) +
+           sl_op_bytes(1, n, 2 * nq);
+  return sl_op_bytes(1, 2 * nq, n) + sl_op_bytes(3, nq, n) + sl_op_bytes(3, n, nq);
+}
+void varcoef_sl_ops(int ndim, int n, int nq, const double* ops, void* work, SlOp* out) {
+  const long long nn = (long long)n * nq;
+  const int S = ndim == 2 ? 2 : 3;
+  char* w = (char*)work;
+  out[0] = sl_op(ops, n, 0, 1, 2 * nq, n, w);
+  w += sl_op_bytes(1, 2 * nq, n);
+  out[1] = sl_op(ops + 2 * nn, n, nn, S, nq, n, w);
+  w += sl_op_bytes(S, nq, n);
+  out[2] = sl_op(ops + (2 + S) * nn, nq, nn, S, n, nq, w);
+  w += sl_op_bytes(S, n, nq);
+  out[3] = ndim == 2 ? sl_op(ops + 6 * nn, 2 * nq, 0, 1, n, 2 * nq, w) : SlOp();
+}
+
 template <typename T>
 int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, const T* kw,
                   const T* u, T* v, void* work, size_t work_bytes, cudaStream_t st,
-                  Active act, const H16Ops* h16, const DotOut* dot) {
+                  Active act, const H16Ops* h16, const DotOut* dot, const SlOp* sl) {
   if (dot && dot->nb) *dot->nb = 0;
   if ((ndim != 2 && ndim != 3) || n < 1 || nq < 1 || batch < 0 || !ops.hi || !kw || !u || !v)
     return JFG_ERR_ARG;
@@ -225,8 +332,24 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
   // pairs (in bufB, free until the second pass) and the intermediates stay
   // split between the passes, so no tile load does FP64 work.
   const bool dfp = std::is_same<T, double>::value && e == Engine::DF && ops.lo != nullptr;
+  SlOp own[SL_VARCOEF];
+  if constexpr (std::is_same<T, double>::value) {
+    if (!sl && e == Engine::F64 && work_bytes >= need + varcoef_sl_bytes(ndim, n, nq) &&
+        varcoef_pays(ndim, n, nq, batch, SL_MIN_WORK)) {
+      varcoef_sl_ops(ndim, n, nq, (const double*)ops.hi, (char*)work + need, own);
+      JFG_TRY(sl_split_ops(own, SL_VARCOEF, st));
+      sl = own;
+    }
+  }
+  // k: the operator's place in sl, seg >= 0: that segment of it alone
   auto pass = [&](const jfg_contract_desc& d, OpRef<T> op, const T* in, T* out, bool pin,
-                  bool pout) -> int {
+                  bool pout, int k, int seg = -1) -> int {
+    if constexpr (std::is_same<T, double>::value) {
+      if (sl) {
+        const SlOp o = seg >= 0 ? sl[k].segment(seg) : sl[k];
+        return contract_f64_or_sl(d, &o, op.hi, in, out, st);
+      }
+    }
     if (dfp)
       return contract_df64(d, (const double*)op.hi, (const float2*)op.lo, (const double*)in,
                            (double*)out, st, pin, pout);
@@ -286,7 +409,7 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
         return JFG_OK;
       }
     }
-    JFG_TRY(pass(d1, ops, u1, bufA, dfp, dfp));
+    JFG_TRY(pass(d1, ops, u1, bufA, dfp, dfp, 0));
     // 2: G[b][s][p][q] = kw[b][p][q] * sum_j {D,B}[p][j] T[b][s][q][j]
     jfg_contract_desc d2 = make_desc(batch, nq, nq, n, act);
     d2.nseg = 2;
@@ -300,7 +423,7 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
     d2.field_ld = nq;
     d2.field_seg = 0;
     d2.field_batch = (long long)nq * nq;
-    JFG_TRY(pass(d2, ops.offset(2 * nn), bufA, bufB, dfp, dfp));
+    JFG_TRY(pass(d2, ops.offset(2 * nn), bufA, bufB, dfp, dfp, 1));
     // 3: H[b][k][s][p] = sum_q {B^T,D^T}[k][q] G[b][s][p][q]   (M=n, P=nq, K=nq)
     jfg_contract_desc d3 = make_desc(batch, n, nq, nq, act);
     d3.nseg = 2;
@@ -310,10 +433,10 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
     d3.out_ld = 2LL * nq;
     d3.out_seg = nq;
     d3.out_batch = 2 * nn;
-    JFG_TRY(pass(d3, ops.offset(4 * nn), bufB, bufA, dfp, dfp));
+    JFG_TRY(pass(d3, ops.offset(4 * nn), bufB, bufA, dfp, dfp, 2));
     // 4: V[b][i][k] = sum_{s,p} [D^T|B^T][i][(s,p)] H[b][k][(s,p)]   (M=n, P=n, K=2nq)
     jfg_contract_desc d4 = make_desc(batch, n, n, 2 * nq, act);
-    JFG_TRY(pass(d4, ops.offset(6 * nn), bufA, v, dfp, false));
+    JFG_TRY(pass(d4, ops.offset(6 * nn), bufA, v, dfp, false, 3));
     return JFG_OK;
   }
 
@@ -387,16 +510,16 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
   }
   // 1: T1[b][(s2,q2)][(i0,i1)] = sum_i2 [B;D] U                 (M=2nq, P=n^2, K=n)
   jfg_contract_desc d1 = make_desc(batch, 2 * nq, (int)n2, n, act);
-  JFG_TRY(pass(d1, BD, u1, bufA, dfp, dfp));
+  JFG_TRY(pass(d1, BD, u1, bufA, dfp, dfp, 0));
   // 2a: s2=0 rows with [B;D]: T2[b][(c,q1)][(q2,i0)], c in {0,1}  (M=2nq, P=nq*n, K=n)
   jfg_contract_desc d2 = make_desc(batch, 2 * nq, (int)nn, n, act);
   d2.in_batch = 2 * nq * n2;
   d2.out_batch = 3 * q2 * n;
-  JFG_TRY(pass(d2, BD, bufA, bufB, dfp, dfp));
+  JFG_TRY(pass(d2, BD, bufA, bufB, dfp, dfp, 0));
   // 2b: s2=1 rows with B -> c = 2
   jfg_contract_desc d2b = d2;
   d2b.M = nq;
-  JFG_TRY(pass(d2b, BD, bufA + nq * n2, bufB + 2 * q2 * n, dfp, dfp));
+  JFG_TRY(pass(d2b, BD, bufA + nq * n2, bufB + 2 * q2 * n, dfp, dfp, 0));
   // 3: G[b][c][p0][(q1,q2)] = kw * sum_i0 {D,B,B}[p0][i0] T2[b][c][(q1,q2)][i0]
   jfg_contract_desc d3 = make_desc(batch, nq, (int)q2, n, act);
   d3.nseg = 3;
@@ -410,7 +533,7 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
   d3.field_ld = q2;
   d3.field_seg = 0;
   d3.field_batch = q2 * nq;
-  JFG_TRY(pass(d3, Q3, bufB, bufA, dfp, dfp));
+  JFG_TRY(pass(d3, Q3, bufB, bufA, dfp, dfp, 1));
   // 4: H1[b][c][k2][(p0,q1)] = sum_q2 {B^T,B^T,D^T}[k2][q2] G     (M=n, P=nq^2, K=nq)
   jfg_contract_desc d4 = make_desc(batch, n, (int)q2, nq, act);
   d4.nseg = 3;
@@ -419,21 +542,21 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
   d4.in_batch = 3 * q2 * nq;
   d4.out_seg = q2 * n;
   d4.out_batch = 3 * q2 * n;
-  JFG_TRY(pass(d4, Q4, bufA, bufB, dfp, dfp));
+  JFG_TRY(pass(d4, Q4, bufA, bufB, dfp, dfp, 2));
   // 5: H2a = B^T (c=0), H2b = D^T (c=1) + B^T (c=2)      (M=n, P=n*nq, K=nq)
   T* H2a = bufA;
   T* H2b = bufA + (size_t)batch * n2 * nq;
   jfg_contract_desc d5 = make_desc(batch, n, (int)nn, nq, act);
   d5.in_batch = 3 * q2 * n;
-  JFG_TRY(pass(d5, Q4, bufB, H2a, dfp, dfp));
-  JFG_TRY(pass(d5, Q4.offset(2 * nn), bufB + q2 * n, H2b, dfp, dfp));
+  JFG_TRY(pass(d5, Q4, bufB, H2a, dfp, dfp, 2, 0));
+  JFG_TRY(pass(d5, Q4.offset(2 * nn), bufB + q2 * n, H2b, dfp, dfp, 2, 2));
   d5.beta = 1.0;
-  JFG_TRY(pass(d5, Q4, bufB + 2 * q2 * n, H2b, dfp, dfp));
+  JFG_TRY(pass(d5, Q4, bufB + 2 * q2 * n, H2b, dfp, dfp, 2, 0));
   // 6: V = D^T (x) on H2a + B^T (x) on H2b                 (M=n, P=n^2, K=nq)
   jfg_contract_desc d6 = make_desc(batch, n, (int)n2, nq, act);
-  JFG_TRY(pass(d6, Q4.offset(2 * nn), H2a, v, dfp, false));
+  JFG_TRY(pass(d6, Q4.offset(2 * nn), H2a, v, dfp, false, 2, 2));
   d6.beta = 1.0;
-  JFG_TRY(pass(d6, Q4, H2b, v, dfp, false));
+  JFG_TRY(pass(d6, Q4, H2b, v, dfp, false, 2, 0));
   return JFG_OK;
 }
 
@@ -560,16 +683,17 @@ template int tp_apply<float>(Engine, int, const int*, const int*, int, const OpR
                              const float*, float*, void*, size_t, cudaStream_t, const float*);
 template int fd_solve<double>(Engine, int, int, int, OpRef<double>, OpRef<double>,
                               const double*, const double*, const double*, const double*,
-                              double*, void*, size_t, cudaStream_t, Active, const DotOut*);
+                              double*, void*, size_t, cudaStream_t, Active, const DotOut*,
+                              const SlOp*);
 template int fd_solve<float>(Engine, int, int, int, OpRef<float>, OpRef<float>, const float*,
                              const float*, const float*, const float*, float*, void*, size_t,
-                             cudaStream_t, Active, const DotOut*);
+                             cudaStream_t, Active, const DotOut*, const SlOp*);
 template int varcoef_apply<double>(Engine, int, int, int, int, OpRef<double>, const double*,
                                    const double*, double*, void*, size_t, cudaStream_t, Active,
-                                   const H16Ops*, const DotOut*);
+                                   const H16Ops*, const DotOut*, const SlOp*);
 template int varcoef_apply<float>(Engine, int, int, int, int, OpRef<float>, const float*,
                                   const float*, float*, void*, size_t, cudaStream_t, Active,
-                                  const H16Ops*, const DotOut*);
+                                  const H16Ops*, const DotOut*, const SlOp*);
 
 }  // namespace jfg
 
@@ -720,7 +844,7 @@ extern "C" int jfg_exp_weighted_backward_f64(int ndim, int n, int nq, int batch,
 extern "C" size_t jfg_tp_apply_workspace_size(int ndim, const int* rows, const int* cols,
                                               int batch, int elem_bytes) {
   if (!rows || !cols) return 0;
-  return jfg::tp_apply_ws(ndim, rows, cols, batch, elem_bytes);
+  return jfg::tp_apply_ws_sl(ndim, rows, cols, batch, elem_bytes);
 }
 
 extern "C" int jfg_tp_apply_f64(int ndim, const int* rows, const int* cols, int batch,
@@ -794,7 +918,10 @@ extern "C" int jfg_tp_apply_affine_f64(int ndim, const int* rows, const int* col
 }
 
 extern "C" size_t jfg_fd_solve_workspace_size(int ndim, int n, int batch, int elem_bytes) {
-  return jfg::fd_ws(ndim, n, batch, elem_bytes);
+  return jfg::fd_ws(ndim, n, batch, elem_bytes) + (elem_bytes == 8 && (ndim == 2 || ndim == 3) && n > 0 && batch > 0 &&
+                  jfg::fd_pays(ndim, n, batch, jfg::SL_MIN_WORK)
+              ? jfg::fd_sl_bytes(n)
+              : 0);
 }
 
 extern "C" int jfg_fd_solve_f64(int ndim, int n, int batch, const double* E, const double* W,
@@ -968,7 +1095,11 @@ extern "C" void jfg_split_f16_rows_nd_host(int ndim, int n, int nq, const double
 
 extern "C" size_t jfg_varcoef_workspace_size(int ndim, int n, int nq, int batch,
                                              int elem_bytes) {
-  return jfg::varcoef_ws(ndim, n, nq, batch, elem_bytes);
+  return jfg::varcoef_ws(ndim, n, nq, batch, elem_bytes) +
+         (elem_bytes == 8 && (ndim == 2 || ndim == 3) && n > 0 && batch > 0 &&
+                  jfg::varcoef_pays(ndim, n, nq, batch, jfg::SL_MIN_WORK)
+              ? jfg::varcoef_sl_bytes(ndim, n, nq)
+              : 0);
 }
 
 extern "C" int jfg_varcoef_apply_f64(int ndim, int n, int nq, int batch, const double* ops,

@@ -559,6 +559,14 @@ size_t pcg_ws(int ndim, int n, int nq, int batch) {
   return 4 * vec + 3 * scal + small + inner;
 }
 
+// the FP64 solver's operators cut into digits, behind the scratch
+static size_t pcg_sl_bytes(int ndim, int n, int nq, int batch) {
+  return (ndim == 2 || ndim == 3) && n > 0 && nq > 0 && batch > 0 &&
+                 varcoef_pays(ndim, n, nq, batch, SL_MIN_WORK_CUT)
+             ? varcoef_sl_bytes(ndim, n, nq) + fd_sl_bytes(n)
+             : 0;
+}
+
 template size_t pcg_ws<double>(int, int, int, int);
 template size_t pcg_ws<float>(int, int, int, int);
 
@@ -576,7 +584,7 @@ int PcgCtx<T>::init(const PcgProblem<T>& problem, T* x_, void* work, size_t work
   batch = pb.batch;
   if ((ndim != 2 && ndim != 3) || n < 1 || nq < n || batch < 1 || !pb.rhs || !x)
     return JFG_ERR_ARG;
-  const size_t need = pcg_ws<T>(ndim, n, nq, batch);
+  const size_t need = pcg_ws<T>(ndim, n, nq, batch);  // a multiple of 256
   if (!work || work_bytes < need) return JFG_ERR_WORKSPACE;
   N = 1;
   for (int i = 0; i < ndim; ++i) N *= n;
@@ -613,6 +621,19 @@ int PcgCtx<T>::init(const PcgProblem<T>& problem, T* x_, void* work, size_t work
   sm += align_up((size_t)H16_SLOTS * batch * sizeof(unsigned), 256);
   inner = sm;
   inner_bytes = work_bytes - (size_t)(sm - w);
+  sl = false;
+  if constexpr (std::is_same<T, double>::value) {
+    const size_t cut = pcg_sl_bytes(ndim, n, nq, batch);
+    if (pb.engine == Engine::F64 && pb.m_engine == Engine::F64 && cut > 0 &&
+        work_bytes >= need + cut) {
+      inner_bytes -= cut;
+      char* c = (char*)work + need;
+      varcoef_sl_ops(ndim, n, nq, pb.ops.hi, c, sl_a);
+      fd_sl_ops(n, pb.E.hi, pb.W.hi, c + varcoef_sl_bytes(ndim, n, nq), sl_m);
+      sl = true;
+      JFG_TRY(sl_setup());  // before the iterations are captured
+    }
+  }
   work_ptr = work;
   work_size = work_bytes;
   th = pb.engine == Engine::TH;
@@ -634,15 +655,22 @@ int PcgCtx<T>::init(const PcgProblem<T>& problem, T* x_, void* work, size_t work
 }
 
 template <typename T>
+int PcgCtx<T>::cut_operators() {
+  if (!sl) return JFG_OK;
+  JFG_TRY(sl_split_ops(sl_a, SL_VARCOEF, st));
+  return sl_split_ops(sl_m, 2, st);
+}
+
+template <typename T>
 int PcgCtx<T>::applyA(const T* in, T* out, Active a, DotOut* dot) {
   return varcoef_apply<T>(pb.engine, ndim, n, nq, batch, pb.ops, pb.kw, in, out, inner,
-                          inner_bytes, st, a, th ? &h16 : nullptr, dot);
+                          inner_bytes, st, a, th ? &h16 : nullptr, dot, sl ? sl_a : nullptr);
 }
 
 template <typename T>
 int PcgCtx<T>::applyM(const T* in, T* out, Active a, DotOut* dot) {
   return fd_solve<T>(pb.m_engine, ndim, n, batch, pb.E, pb.W, pb.lam, nullptr, pb.fd_scale, in,
-                     out, inner, inner_bytes, st, a, dot);
+                     out, inner, inner_bytes, st, a, dot, sl ? sl_m : nullptr);
 }
 
 // out . M^-1 in into part: fused into the preconditioner when possible
@@ -825,6 +853,7 @@ int pcg_run(const PcgProblem<T>& pb, T* x, int use_x0, double tol, int maxiter, 
   if (!(tol > 0.0) || maxiter < 0) return JFG_ERR_ARG;
   PcgCtx<T> c;
   JFG_TRY(c.init(pb, x, work, work_bytes, st));
+  JFG_TRY(c.cut_operators());
   k_set_tol<<<(pb.batch + 127) / 128, 128, 0, st>>>(c.tolv, tol, pb.batch);
   JFG_LAUNCHED();
   JFG_TRY(c.start(nullptr, nullptr, use_x0, pb.judge_x0));
@@ -875,7 +904,9 @@ template int pcg_run<float>(const PcgProblem<float>&, float*, int, double, int, 
 }  // namespace jfg
 
 extern "C" size_t jfg_pcg_workspace_size(int ndim, int n, int nq, int batch, int elem_bytes) {
-  if (elem_bytes == 8) return jfg::pcg_ws<double>(ndim, n, nq, batch);
+  if (elem_bytes == 8)
+    return jfg::align_up(jfg::pcg_ws<double>(ndim, n, nq, batch), 256) +
+           jfg::pcg_sl_bytes(ndim, n, nq, batch);
   return jfg::pcg_ws<float>(ndim, n, nq, batch);
 }
 

@@ -83,6 +83,10 @@ struct PcgCtx {
   bool th = false, fuse_pq = false, fuse_rz = false;
   int nb_pq = 16, nb_rz = 16;
   H16Ops h16;
+  // FP64: the operators cut into digits once per solve (cut_operators), when
+  // the workspace has room behind the scratch of the passes
+  SlOp sl_a[SL_VARCOEF], sl_m[2];
+  bool sl = false;
   int maxit = 0;             // per-problem iteration cap since its start (0: none)
   bool track_ready = false;  // problems leaving the active list go to the ready list
 
@@ -92,6 +96,7 @@ struct PcgCtx {
   // (re)start the listed problems (list NULL: all) from x = 0, or from x with
   // use_x0 (judged against the zero start with judge); tolv must be set
   int start(const int* list, const int* count, int use_x0, bool judge);
+  int cut_operators();
   int iteration(int it);
   int chunk();  // CH iterations through the cached graph (launched directly on the
                 // legacy default stream, which cannot be captured)
