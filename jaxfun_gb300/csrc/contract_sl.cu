@@ -255,17 +255,6 @@ JFG_MMA_COLLECT(mma_use, "use")
 JFG_MMA_COLLECT(mma_lastuse, "lastuse")
 #undef JFG_MMA_COLLECT
 
-// one lane of the (converged) warp
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t.reg .pred P1;\n\t"
-      "elect.sync _|P1, 0xffffffff;\n\t"
-      "selp.b32 %0, 1, 0, P1;\n\t}"
-      : "=r"(p));
-  return p != 0;
-}
-
 __device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

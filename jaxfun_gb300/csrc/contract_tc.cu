@@ -470,7 +470,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint64_t* fbar = bars + 3 * S + 7;      // [16] field box landed (two per epilogue warp)
   uint32_t* tmem_slot = (uint32_t*)(bars + 3 * S + 23);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // warp-uniform to the compiler, like the TMEM base below: the MMA issuer's
+  // descriptors then stay in uniform registers
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   auto Xh = [&](int st) { return sbase + (size_t)st * stage_bytes; };
   auto Xl = [&](int st) { return sbase + (size_t)st * stage_bytes + XBYTES; };
@@ -513,7 +516,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // sequence, paid by every role at every tile.
   auto decode = [&](long long t, int& gi, int& pt, int& mc, int& b, int& s, bool need_b) {
     gi = 0;
-    while (gi + 1 < L.ngroups && t >= tb[gi + 1]) ++gi;
+    if (G > 1)
+      while (gi + 1 < L.ngroups && t >= tb[gi + 1]) ++gi;
     const TcGroup& q = L.g[gi];
     const unsigned nptiles = (unsigned)((q.d.P + TILE_P - 1) / TILE_P);
     const unsigned mchunks = (unsigned)((q.d.M + q.Mtile - 1) / q.Mtile);
@@ -624,83 +628,93 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      long long g = 0;
-      int li = 0;
-      bool ok = true, issued_any = false;
-      if (res && !mbar_wait(opfull, 0, budget)) ok = false;
-      int gi, pt, mc, b, s;
-      int st = 0;       // stage of K block g
-      uint32_t ph = 0;  // (g / S) & 1
-      for (; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
-        const uint32_t idesc = H16   ? idesc_f16(TILE_P, L.g[gi].Mtile)
-                               : B16 ? idesc_b16(TILE_P, L.g[gi].Mtile)
-                                     : idesc_tf32(TILE_P, L.g[gi].Mtile);
-        const int nkb = nkb_of(gi);
-        const int buf = li & 1;
-        const uint32_t use = (uint32_t)(li >> 1);
-        if (li >= 2 && !mbar_wait(&tempty[buf], (use & 1u) ^ 1u, budget)) {
+    // The whole warp walks the loop on warp-uniform values and one elected
+    // lane issues: from a lane-0 branch every MMA cost ~99 clocks of address
+    // and register moves, whatever its N; this way one of N = 128 takes the
+    // tensor pipe's 64 (measured alone).  Same MMAs in the same order.
+    int li = 0;
+    bool ok = true, issued_any = false;
+    if (res && !mbar_wait(opfull, 0, budget)) ok = false;
+    constexpr bool SW128 = !B16 || KE == 64;  // operator rows of 128 bytes
+    auto odesc = [&](const uint8_t* p) {
+      return SW128 ? sdesc(smem_u32(p)) : sdesc64(smem_u32(p));
+    };
+    const uint64_t od0 = odesc(Oh(0)), od0r = odesc(smem);
+    const uint64_t xd0 = sdesc(smem_u32(Xh(0)));
+    int gi, pt, mc, b, s;
+    int st = 0;       // stage of the current K block
+    uint32_t ph = 0;  // its use count parity
+    for (; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
+      const int mtile = __shfl_sync(0xffffffffu, L.g[gi].Mtile, 0);
+      const uint32_t idesc = H16   ? idesc_f16(TILE_P, mtile)
+                             : B16 ? idesc_b16(TILE_P, mtile)
+                                   : idesc_tf32(TILE_P, mtile);
+      const int nkb = __shfl_sync(0xffffffffu, nkb_of(gi), 0);
+      const int buf = li & 1;
+      const uint32_t use = (uint32_t)(li >> 1);
+      if (li >= 2 && !mbar_wait(&tempty[buf], (use & 1u) ^ 1u, budget)) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t acc = tmem + (uint32_t)buf * acc_stride;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait(&conv[st], ph, budget)) {
           ok = false;
           break;
         }
+        issued_any = true;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem + (uint32_t)buf * acc_stride;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
-          if (!mbar_wait(&conv[st], ph, budget)) {
-            ok = false;
-            break;
-          }
-          issued_any = true;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t oh = smem_u32(res ? OhR(kb) : Oh(st));
-          const uint32_t ol = smem_u32(res ? OlR(kb) : Ol(st));
+        const uint64_t oh =
+            res ? od0r + (((uint32_t)kb * 2 * omax) >> 4) : od0 + (((uint32_t)st * stage_bytes) >> 4);
+        const uint64_t ol = oh + (omax >> 4);
+        const uint32_t ah = tmem + (uint32_t)A_COL0 + A_SLOT * (uint32_t)st, al = ah + A_SLOT / 2;
+        const uint64_t xh = xd0 + (((uint32_t)st * stage_bytes) >> 4), xl = xh + (XBYTES >> 4);
+        if (elect_one()) {
           if (B16) {
-            const uint32_t ah = tmem + (uint32_t)A_COL0 + A_SLOT * (uint32_t)st,
-                           al = ah + A_SLOT / 2;
 #pragma unroll
             for (int kk = 0; kk < KE / 16; ++kk) {
-              const uint32_t off = kk * 32;  // 16 BF16 = 32 B of B per MMA, 8 A columns
-              const uint64_t bh = KE == 64 ? sdesc(oh + off) : sdesc64(oh + off);
-              const uint64_t bl = KE == 64 ? sdesc(ol + off) : sdesc64(ol + off);
-              mma_b16_ta(acc, ah + 8 * kk, bh, idesc, (kb | kk) ? 1u : 0u);
+              // 16 elements = 32 B of the operator per MMA, 8 A columns
+              mma_b16_ta(acc, ah + 8 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
               if (!B1) {
-                mma_b16_ta(acc, ah + 8 * kk, bl, idesc, 1u);
-                mma_b16_ta(acc, al + 8 * kk, bh, idesc, 1u);
+                mma_b16_ta(acc, ah + 8 * kk, ol + 2 * kk, idesc, 1u);
+                mma_b16_ta(acc, al + 8 * kk, oh + 2 * kk, idesc, 1u);
               }
             }
           } else if (ta) {
-            const uint32_t ah = tmem + (uint32_t)A_COL0 + A_SLOT * (uint32_t)st, al = ah + 32;
 #pragma unroll
             for (int kk = 0; kk < KB / 8; ++kk) {
-              const uint32_t off = kk * 32;  // 8 TF32 = 32 B of B per MMA, 8 A columns
-              mma_tf32_ta(acc, ah + 8 * kk, sdesc(oh + off), idesc, (kb | kk) ? 1u : 0u);
-              mma_tf32_ta(acc, ah + 8 * kk, sdesc(ol + off), idesc, 1u);
-              mma_tf32_ta(acc, al + 8 * kk, sdesc(oh + off), idesc, 1u);
+              // 8 TF32 = 32 B of the operator per MMA, 8 A columns
+              mma_tf32_ta(acc, ah + 8 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+              mma_tf32_ta(acc, ah + 8 * kk, ol + 2 * kk, idesc, 1u);
+              mma_tf32_ta(acc, al + 8 * kk, oh + 2 * kk, idesc, 1u);
             }
           } else {
-            const uint32_t xh = smem_u32(Xh(st)), xl = smem_u32(Xl(st));
 #pragma unroll
             for (int kk = 0; kk < KB / 8; ++kk) {
-              const uint32_t off = kk * 32;  // 8 TF32 = 32 B per MMA
-              mma_tf32(acc, sdesc(xh + off), sdesc(oh + off), idesc, (kb | kk) ? 1u : 0u);
-              mma_tf32(acc, sdesc(xh + off), sdesc(ol + off), idesc, 1u);
-              mma_tf32(acc, sdesc(xl + off), sdesc(oh + off), idesc, 1u);
+              // 8 TF32 = 32 B per MMA
+              mma_tf32(acc, xh + 2 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+              mma_tf32(acc, xh + 2 * kk, ol + 2 * kk, idesc, 1u);
+              mma_tf32(acc, xl + 2 * kk, oh + 2 * kk, idesc, 1u);
             }
           }
           mma_commit(&empty[st]);
-          if (++st == S) {
-            st = 0;
-            ph ^= 1u;
-          }
         }
-        if (ok) mma_commit(&tfull[buf]);
+        __syncwarp();
+        if (++st == S) {
+          st = 0;
+          ph ^= 1u;
+        }
       }
-      // after a timeout the MMAs already issued must finish before the TMEM
-      // they write is freed: one more commit tracks all of them
-      if (!ok && issued_any) {
-        mma_commit(mma_done);
-        mbar_wait(mma_done, 0, WAIT_NS);
-      }
+      if (ok && elect_one()) mma_commit(&tfull[buf]);
+      __syncwarp();
+    }
+    // after a timeout the MMAs already issued must finish before the TMEM
+    // they write is freed: one more commit tracks all of them
+    if (!ok && issued_any) {
+      if (elect_one()) mma_commit(mma_done);
+      __syncwarp();
+      mbar_wait(mma_done, 0, WAIT_NS);
     }
   } else if (warp < 6) {
     // ---------------- split staged input tiles into TF32 hi (in place) / lo ----------------

@@ -69,7 +69,10 @@ __global__ void __launch_bounds__(NTH, 1)
   uint64_t* accum = full + 2 * S;
   uint32_t* tmem_slot = (uint32_t*)(full + 2 * S + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // warp-uniform to the compiler, like the TMEM base below: the MMA issuer's
+  // descriptors then stay in uniform registers
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * TM;
   const int b0 = blockIdx.y * NB;  // first sample of this CTA
   const int nkb_all = (d.K + KBE - 1) / KBE;
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(NTH, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     if (lane == 0 && nkb > 0) {
@@ -128,8 +131,10 @@ __global__ void __launch_bounds__(NTH, 1)
         tc::mbar_wait(&full[i % S], (uint32_t)(i / S) & 1u, &g_gemm_status);
     }
   } else if (warp == 1) {
-    if (lane == 0 && nkb > 0) {
+    // the whole warp walks the K blocks, one elected lane issues
+    if (nkb > 0) {
       const uint32_t idesc = tc::idesc_bf16(TM, NB * Nt);
+      const uint64_t ad0 = tc::sdesc_sw128(tc::smem_u32(smem));
       bool ok = true;
       int st = 0;       // i % S
       uint32_t ph = 0;  // (i / S) & 1
@@ -139,21 +144,22 @@ __global__ void __launch_bounds__(NTH, 1)
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sa = tc::smem_u32(smem + (size_t)st * stage_bytes);
-        const uint32_t sb = sa + ABYTES;
+        const uint64_t ad = ad0 + (((uint32_t)st * stage_bytes) >> 4);
+        const uint64_t bd = ad + (ABYTES >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < KBE / 16; ++kk) {
-          const uint32_t off = kk * 32;  // 16 BF16 = 32 B per MMA
-          tc::mma_bf16(tmem, tc::sdesc_sw128(sa + off), tc::sdesc_sw128(sb + off), idesc,
-                       (i | kk) ? 1u : 0u);
+          for (int kk = 0; kk < KBE / 16; ++kk)  // 16 BF16 = 32 B per MMA
+            tc::mma_bf16(tmem, ad + 2 * kk, bd + 2 * kk, idesc, (i | kk) ? 1u : 0u);
+          tc::mma_commit(&empty[st]);
         }
-        tc::mma_commit(&empty[st]);
+        __syncwarp();
         if (++st == S) {
           st = 0;
           ph ^= 1u;
         }
       }
-      if (ok) tc::mma_commit(accum);
+      if (ok && elect_one()) tc::mma_commit(accum);
+      __syncwarp();
     }
   } else if (nkb > 0) {
     // ---------------- epilogue ----------------

@@ -210,6 +210,18 @@ __device__ __forceinline__ int active_count(const int* list, const int* count, i
   return c < 0 ? 0 : (c > batch ? batch : c);
 }
 
+// One lane of the (converged) warp: the tcgen05 issuers run whole warps on
+// warp-uniform values and let this lane issue.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // A zero-initialised descriptor for a single-segment pass with no epilogue.
 inline jfg_contract_desc make_desc(int batch, int M, int P, int K, Active act = Active()) {
   jfg_contract_desc d = {};
