@@ -6,6 +6,8 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ._lib import stream_handle
+
 _WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
 
 
@@ -19,6 +21,8 @@ def as_device(a, dtype=torch.float64) -> torch.Tensor:
     """Return ``a`` as a contiguous CUDA tensor of ``dtype`` (copying host arrays)."""
     if isinstance(a, torch.Tensor):
         t = a
+        if t.is_cuda and t.dtype == dtype:
+            return t.contiguous()
         if t.device.type != "cuda":
             t = t.to(device())
         if t.dtype != dtype:
@@ -33,7 +37,7 @@ def as_device(a, dtype=torch.float64) -> torch.Tensor:
 def workspace(nbytes: int, slot: int = 0) -> torch.Tensor:
     """A cached uint8 device buffer of at least ``nbytes`` for the current stream
     (calls on one stream are ordered, so reuse between calls is safe)."""
-    key = (torch.cuda.current_stream().cuda_stream, slot)
+    key = (stream_handle(), slot)
     buf = _WORKSPACES.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device())

@@ -31,34 +31,66 @@ def device_op(mat: np.ndarray, dtype=torch.float64) -> torch.Tensor:
     return t
 
 
+class _TpPlan:
+    """What every call with the same operators and type shares: their device
+    copies and the C arrays of sizes and pointers (the operators stay
+    referenced, so that their ids stay theirs).  ``ws`` is the workspace size of
+    the last batch."""
+
+    __slots__ = ("mats", "ops", "rows", "cols", "r_a", "c_a", "ptrs", "ws")
+
+    def __init__(self, mats, dtype):
+        self.mats = mats
+        self.ops = [device_op(m, dtype) for m in mats]
+        self.rows = tuple(m.shape[0] for m in mats)
+        self.cols = tuple(m.shape[1] for m in mats)
+        self.r_a, self.c_a = _lib.int_array(self.rows), _lib.int_array(self.cols)
+        self.ptrs = _lib.ptr_array([o.data_ptr() for o in self.ops])
+        self.ws = (-1, 0)
+
+    def workspace(self, batch: int, elem_bytes: int) -> torch.Tensor:
+        last, size = self.ws
+        if last != batch:
+            size = _lib.lib().jfg_tp_apply_workspace_size(len(self.rows), self.r_a, self.c_a,
+                                                          batch, elem_bytes)
+            self.ws = (batch, size)
+        return workspace(size)
+
+
+_PLANS: dict[tuple, _TpPlan] = {}
+
+
+def _tp_plan(mats, dtype) -> _TpPlan:
+    key = (tuple(map(id, mats)), dtype, torch.cuda.current_device())
+    plan = _PLANS.get(key)
+    if plan is None:
+        plan = _PLANS[key] = _TpPlan(tuple(mats), dtype)
+    return plan
+
+
 def tp_apply(mats: list[np.ndarray], x, dtype=torch.float64, df: bool = False) -> torch.Tensor:
     """out = (x_ax mats[ax]) x over the trailing len(mats) axes of ``x``.
-    ``df``: FP64 data with double-FP32 arithmetic (``jfg_tp_apply_df64``)."""
+    ``df``: FP64 data through ``jfg_tp_apply_df64``."""
     nd = len(mats)
     if df and dtype != torch.float64:
         raise ValueError("the double-FP32 engine takes FP64 data")
     x = as_device(x, dtype)
     if x.ndim < nd:
         raise ValueError(f"array of rank {x.ndim} for a {nd}-axis transform")
-    cols = [m.shape[1] for m in mats]
-    rows = [m.shape[0] for m in mats]
-    if list(x.shape[x.ndim - nd :]) != cols:
-        raise ValueError(f"trailing shape {tuple(x.shape[x.ndim - nd:])} != {tuple(cols)}")
-    lead = x.shape[: x.ndim - nd]
-    batch = int(np.prod(lead)) if lead else 1
-    out = torch.empty(lead + tuple(rows), dtype=dtype, device=x.device)
+    plan = _tp_plan(mats, dtype)
+    lead, trail = x.shape[: x.ndim - nd], x.shape[x.ndim - nd:]
+    if trail != plan.cols:
+        raise ValueError(f"trailing shape {tuple(trail)} != {plan.cols}")
+    batch = lead.numel()
+    out = torch.empty(lead + plan.rows, dtype=dtype, device=x.device)
     if batch == 0:
         return out
     L = _lib.lib()
-    r_a, c_a = _lib.int_array(rows), _lib.int_array(cols)
-    eb = 8 if dtype == torch.float64 else 4
-    ws_bytes = L.jfg_tp_apply_workspace_size(nd, r_a, c_a, batch, eb)
-    ws = workspace(ws_bytes)
-    ops = [device_op(m, dtype) for m in mats]
-    fn = (L.jfg_tp_apply_df64 if df else L.jfg_tp_apply_f64) if dtype == torch.float64 \
-        else L.jfg_tp_apply_f32
-    st = fn(nd, r_a, c_a, batch, _lib.ptr_array([o.data_ptr() for o in ops]), x.data_ptr(),
-            out.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_handle())
+    f64 = dtype == torch.float64
+    ws = plan.workspace(batch, 8 if f64 else 4)
+    fn = (L.jfg_tp_apply_df64 if df else L.jfg_tp_apply_f64) if f64 else L.jfg_tp_apply_f32
+    st = fn(nd, plan.r_a, plan.c_a, batch, plan.ptrs, x.data_ptr(), out.data_ptr(),
+            ws.data_ptr(), ws.numel(), _lib.stream_handle())
     _lib.check(st, "jfg_tp_apply")
     return out
 

@@ -144,6 +144,15 @@ class TPMatricesLUFactors:
             self._dev[dtype] = t
         return t
 
+    @staticmethod
+    def _shift(c, default: float, batch: int, device):
+        """Per-problem values of c0 or c1 on the device; None where the scalar is
+        the C ABI's own default, so that the common calls copy nothing."""
+        if isinstance(c, (int, float)):
+            return None if c == default else torch.full((batch,), float(c), dtype=torch.float64,
+                                                        device=device)
+        return as_device(np.broadcast_to(np.asarray(c, dtype=np.float64), (batch,)).copy())
+
     def solve(self, rhs, c0=None, c1=None) -> torch.Tensor:
         """U = (x W) [(x E) F / (c0 + c1 * sum lam)] for every leading-batch slice.
         ``c0``/``c1`` may be per-batch arrays (default: the factored scalars)."""
@@ -157,14 +166,12 @@ class TPMatricesLUFactors:
         if batch == 0:
             return out
         E, W, lam = self.device_factors()
-        c0 = self.c0 if c0 is None else c0
-        c1 = self.c1 if c1 is None else c1
-        c0_t = as_device(np.broadcast_to(np.asarray(c0, dtype=np.float64), (batch,)).copy())
-        c1_t = as_device(np.broadcast_to(np.asarray(c1, dtype=np.float64), (batch,)).copy())
+        c0_t = self._shift(self.c0 if c0 is None else c0, 0.0, batch, rhs.device)
+        c1_t = self._shift(self.c1 if c1 is None else c1, 1.0, batch, rhs.device)
         L = _lib.lib()
         ws = workspace(L.jfg_fd_solve_workspace_size(nd, n, batch, 8))
         st = L.jfg_fd_solve_f64(nd, n, batch, E.data_ptr(), W.data_ptr(), lam.data_ptr(),
-                                c0_t.data_ptr(), c1_t.data_ptr(), rhs.data_ptr(), out.data_ptr(),
+                                _lib.ptr(c0_t), _lib.ptr(c1_t), rhs.data_ptr(), out.data_ptr(),
                                 ws.data_ptr(), ws.numel(), _lib.stream_handle())
         _lib.check(st, "jfg_fd_solve_f64")
         return out
