@@ -192,18 +192,17 @@ void jfg_split_f16_rowscaled_host(size_t rows, size_t cols, const double* src, u
  * (MMA operand A) in TMEM, written by the split warps with tcgen05.st, so the
  * MMAs read only operand B from shared memory; 0 keeps A in shared memory. */
 int jfg_tc_set_variant(int operand_a_in_tmem);
-/* Epilogue output path of the tensor-core contractions: 1 (default) stages
- * 32 x 32 output boxes in shared memory and writes them with TMA bulk tensor
- * stores where the output rows are 16-byte aligned (and beta == 0); 0 uses
- * plain coalesced stores everywhere. */
+/* Epilogue output path of the tensor-core contractions: accepts 0 and 1 and has
+ * no effect.  Both used to differ in how the outputs were written (bulk tensor
+ * stores or plain ones); every epilogue now stores from registers. */
 int jfg_tc_set_store_path(int tma_store);
-/* Schedule of single-group launches with 16-bit operators (split BF16, scaled
- * split FP16): 0 (default) streams operator and input tiles together; 1
- * operator-stationary -- each persistent CTA serves one (segment, operator
- * chunk) slot, keeps that chunk for all K blocks in shared memory and streams
- * only input tiles, used when the chunk fits beside >= 2 input stages
- * (K <= 256 at 128 operator rows) and there are >= 2 tiles per CTA; 2
- * whenever the chunk fits.  The autotuner tries both where the chunk fits. */
+/* Schedule of single-group launches: 0 streams operator and input tiles; 1
+ * (default) operator-stationary -- each persistent CTA serves one (segment,
+ * operator chunk) slot, keeps that chunk for all K in shared memory and
+ * streams only input tiles -- where the chunk fits beside four input blocks
+ * (hi and lo: K <= 256 16-bit or 128 TF32 elements at 128 operator rows),
+ * there are >= 2 tiles per CTA and the inputs stay in L2; 2 whenever the chunk
+ * fits.  The autotuner tries both where the chunk fits. */
 int jfg_tc_set_op_resident(int on);
 /* Launch configuration of the tensor-core contraction. */
 typedef struct {
@@ -211,13 +210,13 @@ typedef struct {
   int order;             /* grouped launches: 0 groups as given, 1 by operator-tile
                             work, 2 by total work (largest first)                    */
   int ctas;              /* persistent CTAs (0: one per SM)                          */
-  int stages;            /* pipeline stages (0: as many as fit, else >= 2)           */
+  int stages;            /* input and operator blocks in flight (0: as many as fit,
+                            else at most this many of each, >= 2)                   */
   int mtile;             /* operator rows per tile = MMA N (0: up to 128, else 64)   */
-  int schedule;          /* single-group 16-bit launches: 0 the process setting
+  int schedule;          /* single-group launches: 0 the process setting
                             (jfg_tc_set_op_resident), 1 streaming, 2 operator-
                             stationary where the chunk fits                       */
-  int store;             /* epilogue: 0 the process setting (jfg_tc_set_store_path),
-                            1 TMA bulk-tensor stores where allowed, 2 plain stores */
+  int store;             /* 0, 1 or 2: no effect (see jfg_tc_set_store_path)        */
 } jfg_tc_config;
 /*
  * Grouped tensor-core contraction: ngroups independent contractions (each a
@@ -247,9 +246,8 @@ int jfg_tc_autotune(int ngroups, const jfg_contract_desc* descs, const float* co
  * signature (device, precision, batch, segments, M, P, K, epilogue, beta) has
  * no tuned configuration yet and that is made outside stream capture first
  * times the candidates -- pipeline depth (as many as fit, 3, 2) x schedule
- * (streaming, operator-stationary for 16-bit operators) x epilogue store path
- * (TMA, plain) x tile height (128, 64) x operand A placement (split TF32) --
- * with CUDA events on its own operands (the launch runs, so out is written
+ * (streaming, operator-stationary) x tile height (128, 64) x operand A
+ * placement (split TF32) -- with CUDA events on its own operands (the launch runs, so out is written
  * repeatedly), keeps the fastest for that signature and launches with it;
  * tuned signatures always launch with their configuration.  Default 0.
  */

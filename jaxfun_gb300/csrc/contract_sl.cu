@@ -72,7 +72,8 @@ constexpr int SL_NT = 64 + 32 * (NWS + NWE);
 constexpr uint32_t ABYTES = 128 * 128;  // one operator stage: 128 rows x 64 FP16
 constexpr int A_MAX = 8;          // operator stages
 constexpr int STG_LD = 9;         // epilogue staging: 32 rows x 8 columns, padded
-constexpr int RING = 4;           // input tiles whose row exponents are kept
+constexpr int RING = 8;           // input tiles whose row exponents are kept (a tile's are
+                                  // read after its accumulators are handed back)
 constexpr int COL_MAX = 3 * 512;  // column exponents (segments x K padded to 64)
 constexpr int SPECIAL = 1 << 20;  // row exponent of a row with inf or NaN
 // Sum of two row exponents from which a running FP64 sum of up to 512 products

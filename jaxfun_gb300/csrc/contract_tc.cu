@@ -10,16 +10,28 @@
 // (about 2^-22 relative per product) at three TF32 MMAs per block.
 //
 // Tile: 128 rows of p (the MMA M dimension, one TMEM lane per row) by up to 128
-// operator rows m (the MMA N dimension, one TMEM column each), K in blocks of
-// 32 FP32 (128 B rows, 128-byte swizzle), 3 pipeline stages.  The kernel is
+// operator rows m (the MMA N dimension, one TMEM column each).  The kernel is
 // persistent (one CTA per SM walking the tile list) with two TMEM accumulator
-// buffers.  Warp roles:
-//   warp 0     TMA producer (one thread)
-//   warp 1     TMEM allocator and MMA issuer (one thread)
-//   warps 2-5  split each staged input tile into TF32 hi (in place) and lo
+// buffers.  Three rings decouple the roles: input blocks (128 rows x 32 FP32,
+// 16 KB), operator blocks (a 128-byte row of K: 32 TF32 or 64 16-bit elements,
+// hi and lo; or the CTA's whole operator chunk, kept) and operand A slots in
+// TMEM.  An input block is free again as soon as it has been split, an operator
+// block and the A slots when the MMAs of its K are done (one commit for both).
+// Warp roles:
+//   warp 0     input producer (TMA, one thread)
+//   warp 1     TMEM allocator and MMA issuer
+//   warps 2-5  split each input block into hi and lo, operand A, in TMEM
+//   warps 15-18 (plain epilogue of the 16-bit paths) a second splitting group,
+//              the two taking K blocks in turn: 36.5 -> 32.6 us at K = 512
 //   warps 6-13 epilogue: two warps per TMEM lane quarter, tcgen05.ld 32 lanes
 //              x 16 columns, fused field multiply / eigenvalue divide / beta
-//              accumulate
+//              accumulate, stores from registers
+//   warp 14    operator producer (TMA, one thread)
+// With one ring of (input, operator) stages that the MMAs released, and output
+// boxes staged for bulk stores, the split-BF16 pass of 16 x 256^3 took 422 us
+// (now 365, 88 % of the measured HBM rate), the split-FP16 passes of 128
+// problems of N = 256 39 us (M = 512; now 34.5) and 64 us with the field (now
+// 49), the 3-D split-TF32 field pass of 8 x 128^3 130 us (now 104).
 // Every mbarrier wait is bounded by a global-timer budget; on expiry the
 // kernel records JFG_ERR_DEVICE_TIMEOUT in a device status word, drains its own
 // TMA copies (bounded), frees its TMEM and returns.
@@ -50,31 +62,31 @@ __device__ int g_tc_test_hold = 0;
 // Kernel variant: 1 keeps the split input tile in TMEM (default), 0 in shared
 // memory (jfg_tc_set_variant).
 static int g_operand_a_in_tmem = 1;
-// Epilogue output path: 1 TMA stores through shared memory where the layout
-// allows (default), 0 plain coalesced stores (jfg_tc_set_store_path).
-static int g_tma_store = 1;
-// Operator-stationary schedule for single-group 16-bit launches whose
-// operator chunk fits in shared memory: 0 (default) off, 1 when every CTA gets
-// >= 2 tiles, 2 whenever the chunk fits (jfg_tc_set_op_resident); a launch
-// configuration's schedule field overrides it.
-static int g_op_resident = 0;
+// Operator-stationary schedule for single-group launches whose operator chunk
+// fits in shared memory: 0 off, 1 (default) when every CTA gets >= 2 tiles, the
+// chunk leaves four input blocks and the inputs stay in L2, 2 whenever the
+// chunk fits (jfg_tc_set_op_resident); a launch configuration's schedule field
+// overrides it.  Measured against streaming (128 problems, N = 256, split
+// FP16): 34.5 against 36.5 us (M = 512), field pass 49 against 51, divide pass
+// (split BF16) 22.6 against 23.9; 3-D 8 x 128^3 split TF32: 43 against 47.5.
+// Inputs beyond L2 (3 x 8 x 128^3): 117 against 104 us, so they stream.
+static int g_op_resident = 1;
 
 namespace {
 
 constexpr int TILE_P = 128;
 constexpr int KB = 32;                     // FP32 elements per K block (128 B)
 constexpr int MT_MAX = 128;                // operator rows per tile (MMA N)
-constexpr int NTHREADS = 448;  // 14 warps
+// 15 warps; four more that split where that is what bounds the pass: the plain
+// epilogue of the 16-bit paths (their registers, 96 instead of 128 a thread,
+// cost the other kernels more than the split gains)
+__host__ __device__ constexpr int nthreads(int epi, bool beta, int prec) {
+  return prec != 0 && epi == JFG_EPI_NONE && !beta ? 608 : 480;
+}
 constexpr uint32_t XBYTES = TILE_P * KB * 4;  // 16 KB
-// K elements per block of the 16-bit operator paths (split BF16, scaled split
-// FP16): 64 (two 128-byte FP32 input rows, one 128-byte operator row; 64 KB
-// stages, three of them), except for the field-multiply epilogue: its two
-// field boxes per epilogue warp leave room for only two such stages, and with
-// 32-element blocks (one input row, a 64-byte operator row under the 64-byte
-// swizzle; 32 KB stages) five fit.  Measured on the variable-coefficient
-// passes: the field pass 74.5 -> 66.3 us with 32, every other pass slower
-// with 32 (more handshakes per unit of work).
-__host__ __device__ constexpr int b16_ke(int epi) { return epi == JFG_EPI_MUL_FIELD ? 32 : 64; }
+// K elements of one operator stage: a 128-byte row, 32 TF32 or 64 16-bit ones.
+__host__ __device__ constexpr int op_ke(bool b16) { return b16 ? 64 : 32; }
+constexpr int S_MAX = 16;                  // stages (or resident blocks) of a ring
 constexpr unsigned long long WAIT_NS = 2000000000ull;  // 2 s budget per wait
 
 constexpr int GMAX = 40;  // groups per launch of the grouped kernel
@@ -88,7 +100,6 @@ struct TcGroup {
   int bat_in_map;  // 1 if the input map has a batch dimension
   int seg_op_map;  // 1 if the operator maps have a segment dimension
   int mc_inner;    // tile order: operator chunks innermost (inputs beyond L2)
-  int tma_store;   // epilogue stores 32 x 32 boxes through shared memory with TMA
   // scaled split-FP16 variant: per-problem max |input| (float bits) that sets
   // the power-of-two input scale, per-problem max |output| recorded for the
   // next pass, and the inverse power-of-two row scales of the operator
@@ -96,34 +107,26 @@ struct TcGroup {
   unsigned* out_max;
   const float* op_inv;  // op_inv[s * op_inv_seg + m]
   long long op_inv_seg;
-  // field-multiply epilogue of a single-group launch: the field's 32 x 32
-  // boxes are fetched by TMA (L.fmap) into the warp's output staging box
-  int tma_field;
-  int fld_seg;  // the field map has a segment dimension (field_seg != 0)
-  int fld_bat;  // the field map has a batch dimension (field_batch != 0)
   // fused dot (field / divide epilogues): partials of sum(acc * out) per
   // problem at dot_part[b * DOT_NBMAX + tile-of-problem * 8 + epilogue warp]
   float* dot_part;
 };
 
 // Kernel parameter block (__grid_constant__): groups and their tensor maps
-// (input X, operator hi, operator lo, output for TMA stores).
-constexpr uint32_t STAGE_OUT = 32 * 32 * 4;  // one epilogue warp's output box (4 KB)
+// (input X, operator hi, operator lo).
 constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic shared memory (static use < 1 KB)
 template <int G>
 struct TcLaunch {
-  CUtensorMap maps[G][4];
-  CUtensorMap fmap;  // field of group 0 (TcGroup::tma_field)
+  CUtensorMap maps[G][3];
   TcGroup g[G];
   int ngroups;
-  int stages;
+  int xstages;  // input blocks (128 rows x 32 FP32) in shared memory
+  int aslots;   // split input blocks (MMA operand A): TMEM slots, or the input stages
+  int ostages;  // operator blocks in shared memory (streaming schedule)
   int tmem_cols;
   int tmem_a;   // 1: split input tile (MMA operand A) kept in TMEM, not shared memory
   int mt_max;   // largest Mtile: sets the stage layout
-  int out_stage; // 32 x 32 staging boxes per epilogue warp after the stages: 0, 1 (TMA
-                 // stores) or 2 (field-multiply launches: both of a warp's field boxes
-                 // of a tile are fetched ahead and stored from separate boxes)
-  // 1 (16-bit operators, one group): operator-stationary schedule.  CTA c
+  // 1 (one group): operator-stationary schedule.  CTA c
   // serves the operator slot c % nslots, slot = s * mchunks + mc, loads that
   // operator chunk (all K blocks, hi and lo) into shared memory once and
   // streams only the input tiles of its (problem, p-tile) pairs.
@@ -132,8 +135,8 @@ struct TcLaunch {
 };
 
 // TMEM column map when operand A lives in TMEM: accumulator buffers at
-// columns [0, 128) and [128, 256); stage s keeps A hi at 256 + 64 s and A lo
-// at 256 + 64 s + 32 (32 TF32 columns each).
+// columns [0, 128) and [128, 256); slot s of operand A at 256 + A_SLOT s, hi
+// then lo (32 TF32 columns each, or 16 columns of 16-bit pairs).
 constexpr int ACC_STRIDE_TA = 128;
 constexpr int A_COL0 = 256;
 
@@ -207,17 +210,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
-// Bulk tensor store of a shared-memory box (no swizzle) to global, tracked in
-// this thread's bulk async-group.
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0,
-                                             int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
-          reinterpret_cast<uint64_t>(map)),
-      "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row
 // core-matrix groups 1024 B apart.
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
@@ -227,17 +219,6 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
   d |= (uint64_t)(1024 >> 4) << 32;           // stride byte offset
   d |= (uint64_t)1 << 46;                     // descriptor version
   d |= (uint64_t)2 << 61;                     // SWIZZLE_128B
-  return d;
-}
-
-// The same for 64-byte rows (64-byte swizzle): 8-row groups 512 B apart.
-__device__ __forceinline__ uint64_t sdesc64(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                     // leading byte offset (unused, swizzled K-major)
-  d |= (uint64_t)(512 >> 4) << 32;            // stride byte offset
-  d |= (uint64_t)1 << 46;                     // descriptor version
-  d |= (uint64_t)4 << 61;                     // SWIZZLE_64B
   return d;
 }
 
@@ -391,7 +372,7 @@ __device__ __forceinline__ float tf32_hi(float x) {
 // tile i+1.  The tile prefix tb[] is formed on the device from the active
 // counts, so listed (active-subset) groups need no host round trip.
 template <int EPI, bool BETA, int G, int PREC>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
     k_contract_tc(const __grid_constant__ TcLaunch<G> L) {
   // PREC: 0 split TF32 (kind::tf32), 1 split BF16, 2 scaled split FP16 (both
   // kind::f16: 16-bit operator pairs, 64-element K blocks), 3 plain BF16 (one
@@ -400,13 +381,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   constexpr bool H16 = PREC == 2;
   constexpr bool B1 = PREC == 3;
   constexpr uint32_t NOP = B1 ? 1u : 2u;  // operator pieces per stage (hi, lo)
-  // K elements per block: 32 TF32 (one 128-byte row) or 64 BF16 (one 128-byte
-  // operator row; the FP32 input block then takes two TMA boxes)
-  constexpr int KE = B16 ? b16_ke(EPI) : KB;
-  constexpr uint32_t XB = B16 ? (uint32_t)(KE / KB) * XBYTES : XBYTES;
-  constexpr uint32_t OROW = B16 ? 2u * KE : 128u;  // bytes per operator row of a stage
-  // TMEM columns per stage of operand A (hi then lo)
-  constexpr uint32_t A_SLOT = B16 ? (uint32_t)KE : 2u * KB;
+  constexpr int KO = op_ke(B16);       // K elements of an operator block
+  constexpr int KXO = KO / KB;         // input blocks per operator block
+  constexpr uint32_t OROW = 128u;      // bytes per operator row of a block
+  // TMEM columns per slot of operand A (hi then lo)
+  constexpr uint32_t A_SLOT = B1 ? 16u : B16 ? 32u : 64u;
   extern __shared__ uint8_t smem_raw[];
   __shared__ long long tb[G + 1];
   __shared__ int nbs[G];
@@ -415,14 +394,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // scaled split FP16: the input bound of each stage's problem, written by the
   // producer with the stage's loads (it reads the list and the bound well
   // ahead), read by the split warps after the stage's full barrier
-  __shared__ unsigned s_xbits[16];
+  __shared__ unsigned s_xbits[S_MAX];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int S = L.stages;
+  const int SX = L.xstages, SA = L.aslots, SO = L.ostages;
   const bool ta = B16 || L.tmem_a != 0;
-  const bool res = B16 && !B1 && L.op_res != 0;
+  const bool res = L.op_res != 0;
   const uint32_t omax = (uint32_t)L.mt_max * OROW;  // Mtile operator rows (hi or lo)
-  const uint32_t xbuf = ta ? XB : 2 * XBYTES;  // X block (+ its lo part when in SMEM)
-  const uint32_t stage_bytes = res ? xbuf : xbuf + NOP * omax;
+  const uint32_t obytes_max = NOP * omax;           // an operator block
+  const uint32_t xstage = ta ? XBYTES : 2 * XBYTES;  // input block (+ its lo part when in SMEM)
   const uint32_t acc_stride = ta ? ACC_STRIDE_TA : 256;
   // operator-stationary schedule: this CTA's operator slot and tile stride
   const int r_slot = res ? (int)(blockIdx.x % (unsigned)L.nslots) : 0;
@@ -431,8 +410,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const long long r_j0 = res ? (long long)(blockIdx.x / (unsigned)L.nslots) : 0;
   const long long r_step =
       res ? (long long)((gridDim.x - (unsigned)r_slot + (unsigned)L.nslots - 1) / L.nslots) : 1;
-  const int r_nkb = res ? (L.g[0].d.K + KE - 1) / KE : 0;
-  const uint32_t res_bytes = res ? (uint32_t)r_nkb * 2 * omax : 0;
+  const int r_nko = res ? (L.g[0].d.K + KO - 1) / KO : 0;
 
   if (threadIdx.x == 0) {
     long long acc = 0;
@@ -456,19 +434,23 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (!res && (long long)blockIdx.x >= ntiles) return;  // no tile for this CTA (uniform)
   if (res && r_j0 >= r_cnt) return;
 
-  uint8_t* sbase = smem + res_bytes;                   // input (and operator) stages
-  uint8_t* ostage = sbase + (size_t)S * stage_bytes;  // epilogue output boxes (if used)
-  uint64_t* bars = (uint64_t*)(ostage + (size_t)8 * STAGE_OUT * L.out_stage);
-  uint64_t* full = bars;
-  uint64_t* conv = bars + S;
-  uint64_t* empty = bars + 2 * S;
-  uint64_t* tfull = bars + 3 * S;       // [2] accumulator ready
-  uint64_t* tempty = bars + 3 * S + 2;  // [2] accumulator drained
-  uint64_t* hold = bars + 3 * S + 4;    // test hook: nothing arrives on it
-  uint64_t* mma_done = bars + 3 * S + 5;  // MMA drain after a timeout
-  uint64_t* opfull = bars + 3 * S + 6;    // resident operator chunk landed
-  uint64_t* fbar = bars + 3 * S + 7;      // [16] field box landed (two per epilogue warp)
-  uint32_t* tmem_slot = (uint32_t*)(bars + 3 * S + 23);
+  // operator blocks (ring or resident) | input ring
+  uint8_t* obase = smem;
+  uint8_t* xbase = obase + (size_t)(res ? r_nko : SO) * obytes_max;
+  uint64_t* bars = (uint64_t*)(xbase + (size_t)SX * xstage);
+  uint64_t* xfull = bars;               // [S_MAX] input block landed
+  uint64_t* xempty = bars + S_MAX;      // [S_MAX] input block read
+  uint64_t* conv = bars + 2 * S_MAX;    // [S_MAX] operand A slot written
+  uint64_t* ofull = bars + 3 * S_MAX;   // [S_MAX] operator block landed
+  // [S_MAX] the MMAs of K block n (n % S_MAX) are done: its operator block and
+  // its operand A slots are free.  One commit per K block serves both rings
+  // (a commit costs the issuer 100-200 clocks); no ring is longer than S_MAX.
+  uint64_t* kdone = bars + 4 * S_MAX;
+  uint64_t* tfull = bars + 5 * S_MAX;       // [2] accumulator ready
+  uint64_t* tempty = bars + 5 * S_MAX + 2;  // [2] accumulator drained
+  uint64_t* hold = bars + 5 * S_MAX + 4;    // test hook: nothing arrives on it
+  uint64_t* mma_done = bars + 5 * S_MAX + 5;  // MMA drain after a timeout
+  uint32_t* tmem_slot = (uint32_t*)(bars + 5 * S_MAX + 6);
 
   // warp-uniform to the compiler, like the TMEM base below: the MMA issuer's
   // descriptors then stay in uniform registers
@@ -476,10 +458,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S; ++i) {
-      mbar_init(&full[i], 1);
+    for (int i = 0; i < S_MAX; ++i) {
+      mbar_init(&xfull[i], 1);
+      mbar_init(&xempty[i], 4);  // the split warps (operand A in TMEM)
       mbar_init(&conv[i], 4);
-      mbar_init(&empty[i], 1);
+      mbar_init(&ofull[i], 1);
+      mbar_init(&kdone[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
@@ -487,8 +471,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     mbar_init(hold, 1);
     mbar_init(mma_done, 1);
-    mbar_init(opfull, 1);
-    for (int i = 0; i < 16; ++i) mbar_init(&fbar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -503,13 +485,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  auto Xh = [&](int st) { return sbase + (size_t)st * stage_bytes; };
-  auto Xl = [&](int st) { return sbase + (size_t)st * stage_bytes + XBYTES; };
-  auto Oh = [&](int st) { return sbase + (size_t)st * stage_bytes + xbuf; };
-  auto Ol = [&](int st) { return sbase + (size_t)st * stage_bytes + xbuf + omax; };
-  // resident operator chunk: K block kb of hi at 2 kb omax, lo right after it
-  auto OhR = [&](int kb) { return smem + (size_t)kb * 2 * omax; };
-  auto OlR = [&](int kb) { return smem + (size_t)kb * 2 * omax + omax; };
+  auto Xh = [&](int st) { return xbase + (size_t)st * xstage; };
+  auto Xl = [&](int st) { return xbase + (size_t)st * xstage + XBYTES; };
+  auto Op = [&](int st) { return obase + (size_t)st * obytes_max; };  // hi, then lo
   // b = problem index (-1: an out-of-range list entry, computed but not stored);
   // roles that do not use b (need_b false) skip its list load.  Tile indices
   // below 2^32 take 32-bit division: the 64-bit one is a long software
@@ -549,7 +527,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     s = bs - slot * q.d.nseg;
     b = need_b ? active_problem(q.d.batch_list, nbs[gi], q.d.batch, slot) : 0;
   };
-  auto nkb_of = [&](int gi) { return (L.g[gi].d.K + KE - 1) / KE; };
+  // input blocks of a tile: whole operator blocks (zeros past K)
+  auto nkx_of = [&](int gi) { return (L.g[gi].d.K + KO - 1) / KO * KXO; };
+  // the MMAs of K block n are done (n < 0: there is none)
+  auto wait_done = [&](long long n) {
+    return n < 0 || mbar_wait(&kdone[n % S_MAX], (uint32_t)(n / S_MAX) & 1u, budget);
+  };
   // tile li of this CTA (false past the last one)
   auto tile_of = [&](long long li, int& gi, int& pt, int& mc, int& b, int& s,
                      bool need_b = true) -> bool {
@@ -571,60 +554,81 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   };
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
+    // ---------------- input producer ----------------
     if (lane == 0) {
-      long long g = 0, issued = 0;
+      long long issued = 0;
       bool ok = true;
-      if (res) {
-        // the operator chunk of this CTA's slot, once: every K block, hi and lo
-        const TcGroup& q = L.g[0];
-        const uint32_t obytes = (uint32_t)q.Mtile * OROW;
-        const int os = q.seg_op_map ? r_s : 0;
-        mbar_expect_tx(opfull, (uint32_t)r_nkb * 2 * obytes);
-        for (int kb = 0; kb < r_nkb; ++kb) {
-          tma_load_3d(OhR(kb), &L.maps[0][1], opfull, kb * KE, r_mc * q.Mtile, os);
-          tma_load_3d(OlR(kb), &L.maps[0][2], opfull, kb * KE, r_mc * q.Mtile, os);
-        }
-      }
       int gi, pt, mc, b, s;
-      int st = 0;       // stage of K block g (g % S, kept running: no division)
-      uint32_t ph = 0;  // (g / S) & 1
+      int st = 0;       // stage of the current block (kept running: no division)
+      uint32_t ph = 0;  // its use count parity
       for (long long li = 0; ok && tile_of(li, gi, pt, mc, b, s); ++li) {
         const TcGroup& q = L.g[gi];
         const int cs = q.seg_in_map ? s : 0;
         const int cb = (q.bat_in_map && b > 0) ? b : 0;
-        const int os = q.seg_op_map ? s : 0;
-        const uint32_t obytes = (uint32_t)q.Mtile * OROW;
-        const int nkb = nkb_of(gi);
+        const int nkx = nkx_of(gi);
         const unsigned xbits = H16 ? h16_bits(q.in_max, b) : 0u;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
-          if (g >= S && !mbar_wait(&empty[st], ph ^ 1u, budget)) {
+        for (int kx = 0; kx < nkx; ++kx) {
+          // operand A in shared memory: the MMAs read the stage itself
+          if (ta ? issued >= SX && !mbar_wait(&xempty[st], ph ^ 1u, budget)
+                 : !wait_done(issued - SX)) {
             ok = false;
             break;
           }
           if (H16) s_xbits[st] = xbits;
-          mbar_expect_tx(&full[st], res ? XB : XB + NOP * obytes);
-          tma_load_4d(Xh(st), &L.maps[gi][0], &full[st], kb * KE, pt * TILE_P, cs, cb);
-          if (B16 && KE > KB)
-            tma_load_4d(Xh(st) + XBYTES, &L.maps[gi][0], &full[st], kb * KE + KB,
-                        pt * TILE_P, cs, cb);
-          if (!res) {
-            tma_load_3d(Oh(st), &L.maps[gi][1], &full[st], kb * KE, mc * q.Mtile, os);
-            if (!B1)
-              tma_load_3d(Ol(st), &L.maps[gi][2], &full[st], kb * KE, mc * q.Mtile, os);
-          }
-          issued = g + 1;
-          if (++st == S) {
+          mbar_expect_tx(&xfull[st], XBYTES);
+          tma_load_4d(Xh(st), &L.maps[gi][0], &xfull[st], kx * KB, pt * TILE_P, cs, cb);
+          ++issued;
+          if (++st == SX) {
             st = 0;
             ph ^= 1u;
           }
         }
       }
-      // drain: the latest use of every stage (and the resident operator) must
-      // have landed before exit
-      for (long long q = (issued > S ? issued - S : 0); q < issued; ++q)
-        mbar_wait(&full[q % S], (uint32_t)(q / S) & 1u, WAIT_NS);
-      if (res) mbar_wait(opfull, 0, WAIT_NS);
+      // drain: the latest use of every stage must have landed before exit
+      for (long long q = (issued > SX ? issued - SX : 0); q < issued; ++q)
+        mbar_wait(&xfull[q % SX], (uint32_t)(q / SX) & 1u, WAIT_NS);
+    }
+  } else if (warp == 14) {
+    // ---------------- operator producer ----------------
+    if (lane == 0) {
+      if (res) {
+        // the operator chunk of this CTA's slot, once
+        const TcGroup& q = L.g[0];
+        const uint32_t obytes = (uint32_t)q.Mtile * OROW;
+        const int os = q.seg_op_map ? r_s : 0;
+        for (int ko = 0; ko < r_nko; ++ko) {
+          mbar_expect_tx(&ofull[ko], NOP * obytes);
+          tma_load_3d(Op(ko), &L.maps[0][1], &ofull[ko], ko * KO, r_mc * q.Mtile, os);
+          if (!B1)
+            tma_load_3d(Op(ko) + omax, &L.maps[0][2], &ofull[ko], ko * KO, r_mc * q.Mtile, os);
+        }
+        for (int ko = 0; ko < r_nko; ++ko) mbar_wait(&ofull[ko], 0, WAIT_NS);
+      } else {
+        long long issued = 0;
+        bool ok = true;
+        int gi, pt, mc, b, s;
+        int st = 0;
+        for (long long li = 0; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
+          const TcGroup& q = L.g[gi];
+          const int os = q.seg_op_map ? s : 0;
+          const uint32_t obytes = (uint32_t)q.Mtile * OROW;
+          const int nko = (q.d.K + KO - 1) / KO;
+          for (int ko = 0; ko < nko; ++ko) {
+            if (!wait_done(issued - SO)) {
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(&ofull[st], NOP * obytes);
+            tma_load_3d(Op(st), &L.maps[gi][1], &ofull[st], ko * KO, mc * q.Mtile, os);
+            if (!B1)
+              tma_load_3d(Op(st) + omax, &L.maps[gi][2], &ofull[st], ko * KO, mc * q.Mtile, os);
+            ++issued;
+            if (++st == SO) st = 0;
+          }
+        }
+        for (long long q = (issued > SO ? issued - SO : 0); q < issued; ++q)
+          mbar_wait(&ofull[q % SO], (uint32_t)(q / SO) & 1u, WAIT_NS);
+      }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -634,22 +638,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // tensor pipe's 64 (measured alone).  Same MMAs in the same order.
     int li = 0;
     bool ok = true, issued_any = false;
-    if (res && !mbar_wait(opfull, 0, budget)) ok = false;
-    constexpr bool SW128 = !B16 || KE == 64;  // operator rows of 128 bytes
-    auto odesc = [&](const uint8_t* p) {
-      return SW128 ? sdesc(smem_u32(p)) : sdesc64(smem_u32(p));
-    };
-    const uint64_t od0 = odesc(Oh(0)), od0r = odesc(smem);
-    const uint64_t xd0 = sdesc(smem_u32(Xh(0)));
+    const uint64_t od0 = sdesc(smem_u32(obase));
+    const uint64_t xd0 = sdesc(smem_u32(xbase));
     int gi, pt, mc, b, s;
-    int st = 0;       // stage of the current K block
-    uint32_t ph = 0;  // its use count parity
+    int sl = 0, so = 0;          // operand A slots of a block, operator stage
+    uint32_t aph = 0, oph = 0;   // their use count parities
+    unsigned kn = 0;             // K blocks so far, modulo S_MAX
     for (; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
       const int mtile = __shfl_sync(0xffffffffu, L.g[gi].Mtile, 0);
       const uint32_t idesc = H16   ? idesc_f16(TILE_P, mtile)
                              : B16 ? idesc_b16(TILE_P, mtile)
                                    : idesc_tf32(TILE_P, mtile);
-      const int nkb = __shfl_sync(0xffffffffu, nkb_of(gi), 0);
+      const int nko = __shfl_sync(0xffffffffu, nkx_of(gi) / KXO, 0);
       const int buf = li & 1;
       const uint32_t use = (uint32_t)(li >> 1);
       if (li >= 2 && !mbar_wait(&tempty[buf], (use & 1u) ^ 1u, budget)) {
@@ -658,34 +658,38 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + (uint32_t)buf * acc_stride;
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (!mbar_wait(&conv[st], ph, budget)) {
+      if (res) so = 0;
+      for (int ko = 0; ko < nko; ++ko) {
+        if (!mbar_wait(&ofull[so], res ? 0u : oph, budget) ||
+            !mbar_wait(&conv[sl], aph, budget)) {
           ok = false;
           break;
         }
         issued_any = true;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t oh =
-            res ? od0r + (((uint32_t)kb * 2 * omax) >> 4) : od0 + (((uint32_t)st * stage_bytes) >> 4);
+        const uint64_t oh = od0 + (((uint32_t)so * obytes_max) >> 4);
         const uint64_t ol = oh + (omax >> 4);
-        const uint32_t ah = tmem + (uint32_t)A_COL0 + A_SLOT * (uint32_t)st, al = ah + A_SLOT / 2;
-        const uint64_t xh = xd0 + (((uint32_t)st * stage_bytes) >> 4), xl = xh + (XBYTES >> 4);
+        const uint32_t ah = tmem + (uint32_t)A_COL0 + A_SLOT * KXO * (uint32_t)sl;
+        const uint64_t xh = xd0 + (((uint32_t)sl * xstage) >> 4), xl = xh + (XBYTES >> 4);
         if (elect_one()) {
           if (B16) {
 #pragma unroll
-            for (int kk = 0; kk < KE / 16; ++kk) {
-              // 16 elements = 32 B of the operator per MMA, 8 A columns
-              mma_b16_ta(acc, ah + 8 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+            for (int kk = 0; kk < KO / 16; ++kk) {
+              // 16 elements = 32 B of the operator per MMA, 8 A columns (two
+              // per slot of 32 elements)
+              const uint32_t a1 = ah + A_SLOT * (kk / 2) + 8 * (kk % 2), a2 = a1 + A_SLOT / 2;
+              mma_b16_ta(acc, a1, oh + 2 * kk, idesc, (ko | kk) ? 1u : 0u);
               if (!B1) {
-                mma_b16_ta(acc, ah + 8 * kk, ol + 2 * kk, idesc, 1u);
-                mma_b16_ta(acc, al + 8 * kk, oh + 2 * kk, idesc, 1u);
+                mma_b16_ta(acc, a1, ol + 2 * kk, idesc, 1u);
+                mma_b16_ta(acc, a2, oh + 2 * kk, idesc, 1u);
               }
             }
           } else if (ta) {
+            const uint32_t al = ah + A_SLOT / 2;
 #pragma unroll
             for (int kk = 0; kk < KB / 8; ++kk) {
               // 8 TF32 = 32 B of the operator per MMA, 8 A columns
-              mma_tf32_ta(acc, ah + 8 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+              mma_tf32_ta(acc, ah + 8 * kk, oh + 2 * kk, idesc, (ko | kk) ? 1u : 0u);
               mma_tf32_ta(acc, ah + 8 * kk, ol + 2 * kk, idesc, 1u);
               mma_tf32_ta(acc, al + 8 * kk, oh + 2 * kk, idesc, 1u);
             }
@@ -693,17 +697,23 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
             for (int kk = 0; kk < KB / 8; ++kk) {
               // 8 TF32 = 32 B per MMA
-              mma_tf32(acc, xh + 2 * kk, oh + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+              mma_tf32(acc, xh + 2 * kk, oh + 2 * kk, idesc, (ko | kk) ? 1u : 0u);
               mma_tf32(acc, xh + 2 * kk, ol + 2 * kk, idesc, 1u);
               mma_tf32(acc, xl + 2 * kk, oh + 2 * kk, idesc, 1u);
             }
           }
-          mma_commit(&empty[st]);
+          mma_commit(&kdone[kn]);
         }
         __syncwarp();
-        if (++st == S) {
-          st = 0;
-          ph ^= 1u;
+        if (++sl == SA / KXO) {
+          sl = 0;
+          aph ^= 1u;
+        }
+        kn = (kn + 1) % S_MAX;
+        ++so;
+        if (!res && so == SO) {
+          so = 0;
+          oph ^= 1u;
         }
       }
       if (ok && elect_one()) mma_commit(&tfull[buf]);
@@ -716,39 +726,55 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       __syncwarp();
       mbar_wait(mma_done, 0, WAIT_NS);
     }
-  } else if (warp < 6) {
+  } else if (warp < 6 || warp > 14) {
     // ---------------- split staged input tiles into TF32 hi (in place) / lo ----------------
-    const int ct = threadIdx.x - 64;  // 0..127
+    // Two groups of four warps (one per TMEM lane quarter) take K blocks in
+    // turn.  A stage must then always be the same group's (a whole number of
+    // turns per ring): a parity wait cannot skip a phase that the other group
+    // waits for.  Else the first group takes all blocks.
+    const int grp = warp < 6 ? 0 : 1;
+    const bool two = nthreads(EPI, BETA, PREC) == 608 && SX % (2 * KXO) == 0;
+    const int ct = threadIdx.x - (grp ? 480 : 64);  // 0..127
     // TMEM mode: thread = row r of the tile (its warp's lane quarter), reads
     // its 32 values from the 128-byte-swizzled tile and stores hi / lo into
     // its TMEM lane with tcgen05.st.
     const int row = 32 * (warp & 3) + lane;
     bool ok = true;
     int gi, pt, mc, b, s;
-    int st = 0;       // stage of the current K block
-    uint32_t ph = 0;  // its use count parity
+    int st = 0, sl = 0;          // input stage, operand A slot
+    uint32_t ph = 0;             // use count parity of the stage
+    long long kn = 0;            // K block
+    float xsc = 1.f, xinv = 1.f;
     for (long long li = 0; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
-      const int nkb = nkb_of(gi);
-      float xsc = 1.f, xinv = 1.f;
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (!mbar_wait(&full[st], ph, budget)) {
+      const int nkx = nkx_of(gi);
+      for (int kx = 0; kx < nkx; ++kx) {
+        if ((two ? (int)(kn & 1) : 0) != grp) {
+          if (++st == SX) {
+            st = 0;
+            ph ^= 1u;
+          }
+          if (++sl == SA) sl = 0;
+          if (kx % KXO == KXO - 1) ++kn;
+          continue;
+        }
+        if (!mbar_wait(&xfull[st], ph, budget)) {
           ok = false;
           break;
         }
-        if (H16 && kb == 0) h16_scale_bits(s_xbits[st], xsc, xinv);
-        if (H16) {
-          // 64 FP32 of this row, scaled by 2^k, -> FP16 hi / lo pairs; one
-          // 32-element half at a time (16 hi and 16 lo columns) keeps the
-          // live registers low
-          const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) +
-                                 (uint32_t)A_COL0 + A_SLOT * (uint32_t)st;
+        if (H16 && kx % KXO == 0) h16_scale_bits(s_xbits[st], xsc, xinv);
+        const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)A_COL0 +
+                               A_SLOT * (uint32_t)sl;
+        if (ta) {
+          // 32 FP32 of this row -> hi and lo: TF32 words, or 16-bit pairs
+          // packed two to a column (lower k in the lower half; FP16 scaled by
+          // the problem's power of two)
+          constexpr int W = B16 ? 16 : 32;
+          uint32_t h[W], l[W];
+          const float4* xr = (const float4*)(Xh(st) + row * 128);
 #pragma unroll
-          for (int half = 0; half < KE / KB; ++half) {
-            uint32_t h[16], l[16];
-            const float4* xr = (const float4*)(Xh(st) + half * XBYTES + row * 128);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const float4 v = xr[c ^ (row & 7)];
+          for (int c = 0; c < 8; ++c) {
+            const float4 v = xr[c ^ (row & 7)];
+            if constexpr (H16) {
               const float a0 = v.x * xsc, a1 = v.y * xsc, a2 = v.z * xsc, a3 = v.w * xsc;
               const uint32_t h0 = pack_f16x2(a0, a1), h1 = pack_f16x2(a2, a3);
               const float2 f0 = unpack_f16x2(h0), f1 = unpack_f16x2(h1);
@@ -756,25 +782,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               h[2 * c + 1] = h1;
               l[2 * c] = pack_f16x2(a0 - f0.x, a1 - f0.y);
               l[2 * c + 1] = pack_f16x2(a2 - f1.x, a3 - f1.y);
-            }
-            tmem_st16(tbase + 16 * half, h);
-            tmem_st16(tbase + A_SLOT / 2 + 16 * half, l);
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        } else if (B16) {
-          // 64 FP32 of this row (two swizzled 128-byte rows) -> BF16 hi / lo,
-          // packed in pairs (lower k in the lower half) into 32 TMEM columns
-          // each, one 32-element half (16 + 16 columns) at a time
-          const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) +
-                                 (uint32_t)A_COL0 + A_SLOT * (uint32_t)st;
-#pragma unroll
-          for (int half = 0; half < KE / KB; ++half) {
-            uint32_t h[16], l[16];
-            const float4* xr = (const float4*)(Xh(st) + half * XBYTES + row * 128);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const float4 v = xr[c ^ (row & 7)];
+            } else if constexpr (B16) {
               const uint32_t h0 = pack_bf16x2(v.x, v.y), h1 = pack_bf16x2(v.z, v.w);
               h[2 * c] = h0;
               h[2 * c + 1] = h1;
@@ -784,32 +792,32 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 l[2 * c + 1] = pack_bf16x2(v.z - __uint_as_float(h1 << 16),
                                            v.w - __uint_as_float(h1 & 0xFFFF0000u));
               }
-            }
-            tmem_st16(tbase + 16 * half, h);
-            if (!B1) tmem_st16(tbase + A_SLOT / 2 + 16 * half, l);
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        } else if (ta) {
-          const float4* xr = (const float4*)(Xh(st) + row * 128);
-          uint32_t h[32], l[32];
+            } else {
+              const float hv[4] = {tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w)};
+              const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float4 v = xr[c ^ (row & 7)];
-            const float hv[4] = {tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w)};
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              h[4 * c + e] = __float_as_uint(hv[e]);
-              l[4 * c + e] = __float_as_uint(vv[e] - hv[e]);
+              for (int e = 0; e < 4; ++e) {
+                h[4 * c + e] = __float_as_uint(hv[e]);
+                l[4 * c + e] = __float_as_uint(vv[e] - hv[e]);
+              }
             }
           }
-          const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) +
-                                 (uint32_t)A_COL0 + A_SLOT * (uint32_t)st;
-          tmem_st32(tbase, h);
-          tmem_st32(tbase + 32, l);
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          if (kx % KXO == 0 && !wait_done(kn - SA / KXO)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if constexpr (B16) {
+            tmem_st16(tbase, h);
+            if (!B1) tmem_st16(tbase + A_SLOT / 2, l);
+          } else {
+            tmem_st32(tbase, h);
+            tmem_st32(tbase + A_SLOT / 2, l);
+          }
+          if (kx % KXO == KXO - 1) {  // hand over a whole operator block's K
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          }
         } else {
           float4* xh = (float4*)Xh(st);
           float4* xl = (float4*)Xl(st);
@@ -824,18 +832,31 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&conv[st]);
-        if (++st == S) {
+        if (lane == 0) {
+          if (kx % KXO == KXO - 1) mbar_arrive(&conv[sl / KXO]);
+          // the block is read (its values are stored): its stage may be filled
+          // again while the MMAs still work on earlier slots
+          if (ta) mbar_arrive(&xempty[st]);
+        }
+        if (++st == SX) {
           st = 0;
           ph ^= 1u;
         }
+        if (++sl == SA) sl = 0;
+        if (kx % KXO == KXO - 1) ++kn;
       }
     }
   } else {
     // ---------------- epilogue: TMEM -> registers -> global ----------------
     // Eight warps: two per TMEM lane quarter, each taking every other group
-    // of 32 accumulator columns; field / eigenvalue loads of a group are all
-    // issued before its TMEM load so they are in flight together.
+    // of 32 accumulator columns in blocks of 16.  A lane holds one p of all m,
+    // so that a store (or a field load) of one m is 128 contiguous bytes of
+    // the warp: registers go straight to global memory.  Staging the tile in
+    // shared memory for bulk tensor stores cost the epilogue the copy, a proxy
+    // fence and a wait per 32 x 32 box.  Per-row factors (eigenvalues, operator
+    // scales) are held one per lane and broadcast; the field values of block
+    // k + 1 are loaded while block k is processed, those of block 0 before the
+    // accumulator wait.
     const int q4 = warp & 3;  // TMEM lane quarter this warp may access
     const int half = (warp - 6) >> 2;
     const int row = 32 * q4 + lane;
@@ -843,16 +864,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // test hook: a barrier nothing arrives on; its wait runs out (status set)
     // and this warp skips its tiles, so every other role's waits run out too
     const bool held = s_hold != 0 && !mbar_wait(hold, 0, budget);
-    const int ew = warp - 6;   // this warp's staging boxes and field barriers
-    uint32_t fph = 0;          // phase bit j of fbar[2 ew + j]
-    uint32_t fpend = 0;        // bit j: a field box load into box j is in flight
-    bool fok = true;
-    const int nbox = L.out_stage > 0 ? L.out_stage : 1;
-    auto box_of = [&](int j) {
-      return (float*)(ostage + ((size_t)ew * nbox + (j < nbox ? j : 0)) * STAGE_OUT);
-    };
+    const int ew = warp - 6;
     int gi, pt, mc, b, s;
-    for (; !held && fok && tile_of(li, gi, pt, mc, b, s); ++li) {
+    for (; !held && tile_of(li, gi, pt, mc, b, s); ++li) {
       const TcGroup& q = L.g[gi];
       const jfg_contract_desc& d = q.d;
       const int Mt = q.Mtile;
@@ -861,9 +875,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const int p = pt * TILE_P + row;
       const bool pin = p < d.P && b >= 0;
       const int bb = b < 0 ? 0 : b;
-      float* outS = q.out + (long long)bb * d.out_batch + (long long)s * d.out_seg;
+      const int mt0 = mc * Mt;
+      const bool full = mt0 + Mt <= d.M;  // no row of the tile is past M
+      float* outT = q.out + (long long)bb * d.out_batch + (long long)s * d.out_seg +
+                    (long long)mt0 * d.out_ld + p;
       float c0 = 0.f, c1 = 1.f, lp = 0.f;
-      const float* __restrict__ lam_m = (const float*)d.lam_m;
       if (EPI == JFG_EPI_DIV_EIG) {
         c0 = d.c0 ? __ldg((const float*)d.c0 + bb) : 0.f;
         c1 = d.c1 ? __ldg((const float*)d.c1 + bb) : 1.f;
@@ -871,163 +887,91 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       const float* __restrict__ fld = nullptr;
       if (EPI == JFG_EPI_MUL_FIELD)
-        fld = (const float*)d.field + (long long)bb * d.field_batch + (long long)s * d.field_seg;
-      float xsc = 1.f, xinv = 1.f, omax = 0.f, dsum = 0.f;
-      const float* __restrict__ oinv = nullptr;
-      if (H16) {
-        h16_scale(q.in_max, b, xsc, xinv);
-        oinv = q.op_inv + (long long)s * q.op_inv_seg;
-      }
+        fld = (const float*)d.field + (long long)bb * d.field_batch + (long long)s * d.field_seg +
+              (long long)mt0 * d.field_ld + p;
+      float omax = 0.f, dsum = 0.f;
       const bool fdot = EPI != JFG_EPI_NONE && q.dot_part != nullptr;
-      // This warp's 16-column blocks of the tile: cb(k) = 2 half + 4 (k / 2) +
-      // k % 2 (pairs form the 32 x 32 boxes of the TMA stores).  The per-column
-      // factors of block k+1 (field values, eigenvalues, operator scales) are
-      // loaded while block k is processed, and those of block 0 before the
-      // accumulator wait, so their latency overlaps the main loop.
       const int ncb = Mt / 16;
+      // block k: columns 16 cb(k) .. + 15; pairs of blocks are 32 columns
       auto cb_of = [&](int k) { return half * 2 + 4 * (k >> 1) + (k & 1); };
-      // field-multiply epilogue with TMA: the field's 32 x 32 box of each
-      // output box is fetched into the staging box by one bulk tensor copy
-      const bool tfld = EPI == JFG_EPI_MUL_FIELD && !BETA && q.tma_store && q.tma_field;
-      const bool dbl = tfld && nbox == 2;
-      // field box of output box j (blocks k = 2j, 2j+1) into staging box j
-      auto issue_field = [&](int j, int cbk) {
-        if (lane == 0) {
-          mbar_expect_tx(&fbar[2 * ew + j], STAGE_OUT);
-          tma_load_4d(box_of(j), &L.fmap, &fbar[2 * ew + j], pt * TILE_P + 32 * q4,
-                      mc * Mt + (cbk & ~1) * 16, q.fld_seg ? s : 0, q.fld_bat ? bb : 0);
+      // this lane's row of each pair: operator scale times the problem's, eigenvalue
+      float os0 = 0.f, os1 = 0.f, lm0 = 1.f, lm1 = 1.f;
+      if (H16 || EPI == JFG_EPI_DIV_EIG) {
+        const int ma = mt0 + 32 * half + lane, mb = ma + 64;
+        const bool oka = 32 * half + lane < Mt && ma < d.M, okb = 32 * half + lane + 64 < Mt && mb < d.M;
+        if (H16) {
+          float xsc, xinv;
+          h16_scale(q.in_max, b, xsc, xinv);
+          const float* __restrict__ oinv = q.op_inv + (long long)s * q.op_inv_seg;
+          os0 = oka ? __ldg(oinv + ma) * xinv : 0.f;
+          os1 = okb ? __ldg(oinv + mb) * xinv : 0.f;
         }
-        fpend |= 1u << j;
-      };
-      auto load_aux = [&](int cbk, float* a) {
-        const int m0 = mc * Mt + cbk * 16;
+        if (EPI == JFG_EPI_DIV_EIG) {
+          lm0 = oka ? __ldg((const float*)d.lam_m + ma) : 1.f;
+          lm1 = okb ? __ldg((const float*)d.lam_m + mb) : 1.f;
+        }
+      }
+      auto load_field = [&](int cb, float* f) {
+        const float* src = fld + (long long)(16 * cb) * d.field_ld;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const int m = m0 + j;
-          const bool ok = pin && m < d.M;
-          float v = 1.f;
-          if (EPI == JFG_EPI_MUL_FIELD && !tfld)
-            v = ok ? __ldg(fld + (long long)m * d.field_ld + p) : 0.f;
-          if (EPI == JFG_EPI_DIV_EIG) v = ok ? __ldg(lam_m + m) : 1.f;
-          if (H16 && EPI != JFG_EPI_DIV_EIG) {
-            // the row's inverse scale alone: the problem's (a power of two,
-            // xs) is applied where aux is used, so these loads stay in flight
-            // while the block before is processed
-            const float oi = ok ? __ldg(oinv + m) : 0.f;
-            v = (EPI == JFG_EPI_MUL_FIELD && !tfld) ? v * oi : oi;
-          }
-          a[j] = v;
+          f[j] = pin && (full || mt0 + 16 * cb + j < d.M) ? __ldg(src) : 0.f;
+          src += d.field_ld;
         }
       };
-      const float xs = (H16 && EPI != JFG_EPI_DIV_EIG) ? xinv : 1.f;
-      float aux[16], nxt[16];
-      if (cb_of(0) < ncb) {
-        load_aux(cb_of(0), aux);
-        if (tfld) {
-          // the staging boxes are free once the previous stores have read them
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          __syncwarp();
-          issue_field(0, cb_of(0));
-          if (dbl && cb_of(2) < ncb) issue_field(1, cb_of(2));
-        }
-      }
+      float f[16], fn[16];
+      if (EPI == JFG_EPI_MUL_FIELD && cb_of(0) < ncb) load_field(cb_of(0), f);
       if (!mbar_wait(&tfull[buf], (uint32_t)(li >> 1) & 1u, budget)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)buf * acc_stride;
-      const bool tstore = !BETA && q.tma_store;
+#pragma unroll 1
       for (int k = 0; cb_of(k) < ncb; ++k) {
         const int cb = cb_of(k);
-        const bool more = cb_of(k + 1) < ncb;
-        if (more) load_aux(cb_of(k + 1), nxt);
-        const int mh = mc * Mt + cb * 16;
-        float osc[16], prev[16];
-        if (pin) {
+        const int mh = mt0 + 16 * cb;
+        if (EPI == JFG_EPI_MUL_FIELD && cb_of(k + 1) < ncb) load_field(cb_of(k + 1), fn);
+        float* o = outT + (long long)(16 * cb) * d.out_ld;
+        float prev[16];
+        if (BETA) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int m = mh + j;
-            const bool ok = m < d.M;
-            if (H16 && EPI == JFG_EPI_DIV_EIG) osc[j] = ok ? __ldg(oinv + m) * xinv : 0.f;
-            if (BETA) prev[j] = ok ? outS[(long long)m * d.out_ld + p] : 0.f;
-          }
+          for (int j = 0; j < 16; ++j)
+            prev[j] = pin && (full || mh + j < d.M) ? o[(long long)j * d.out_ld] : 0.f;
         }
         float v[16];
         tmem_ld16(tacc + (uint32_t)(cb * 16), v);
-        float* cbox = box_of(dbl ? (k >> 1) : 0);  // this output box's staging box
-        if (tstore) {
-          // stage this warp's 32 (p) x 32 (m) box in shared memory, [m][p] with
-          // p contiguous, and store it with one bulk tensor copy (out-of-range
-          // rows and columns are clipped by the copy)
-          if ((k & 1) == 0) {
-            if (tfld) {
-              const int j = dbl ? (k >> 1) : 0;
-              if (!dbl && k > 0) {
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                __syncwarp();
-                issue_field(0, cb);
-              }
-              if (!mbar_wait(&fbar[2 * ew + j], (fph >> j) & 1u, budget)) {
-                fok = false;
-                break;
-              }
-              fph ^= 1u << j;
-              fpend &= ~(1u << j);
-            } else {
-              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-              __syncwarp();
-            }
-          }
+        const float osr = k < 2 ? os0 : os1, lmr = k < 2 ? lm0 : lm1;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float r = v[j];  // rows outside the problem are clipped by the store
-            // a = the contraction before the epilogue factor (operator and
-            // input scales applied), for the fused dot sum(a * out)
-            float a = r;
-            if (EPI != JFG_EPI_NONE || H16)
-              r *= (EPI == JFG_EPI_DIV_EIG) ? 1.f : (pin ? aux[j] * xs : 0.f);
-            if (tfld) a = r;  // aux held only the scales; the field comes next
-            if (tfld) r *= cbox[(16 * (k & 1) + j) * 32 + lane];
-            if (H16 && EPI == JFG_EPI_DIV_EIG) r *= pin ? osc[j] : 0.f;
-            if (EPI == JFG_EPI_DIV_EIG) {
-              a = r;
-              r = __fdividef(r, c0 + c1 * ((pin ? aux[j] : 1.f) + lp));
-            }
-            r *= alpha;
-            if (fdot) dsum = fmaf(a, r, dsum);
-            if (H16) omax = fmaxf(omax, fabsf(r));
-            cbox[(16 * (k & 1) + j) * 32 + lane] = r;
-          }
-          if ((k & 1) == 1 || !more || cb_of(k + 1) != cb + 1) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0 && b >= 0)
-              tma_store_4d(&L.maps[gi][3], cbox, pt * TILE_P + 32 * q4, mc * Mt + (cb & ~1) * 16,
-                           s, b);
-            if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
-        } else if (pin) {
+        for (int j = 0; j < 16; ++j) {
+          const int src = 16 * (k & 1) + j;
+          float r = v[j];
+          if (H16) r *= __shfl_sync(0xffffffffu, osr, src);
+          const float a = r;  // the contraction before the epilogue factor
+          if (EPI == JFG_EPI_MUL_FIELD) r *= f[j];
+          if (EPI == JFG_EPI_DIV_EIG)
+            r = __fdividef(r, c0 + c1 * (__shfl_sync(0xffffffffu, lmr, src) + lp));
+          r *= alpha;
+          if (fdot) dsum = fmaf(a, r, dsum);
+          if (BETA) r += beta * prev[j];
+          if (H16) omax = fmaxf(omax, fabsf(r));
+          v[j] = r;
+        }
+        if (pin) {
+          if (full) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int m = mh + j;
-            if (m < d.M) {
-              float r = v[j];
-              float a = r;  // (split FP16 with the field in aux fuses no dot)
-              if (EPI != JFG_EPI_NONE || H16) r *= (EPI == JFG_EPI_DIV_EIG) ? 1.f : aux[j] * xs;
-              if (H16 && EPI == JFG_EPI_DIV_EIG) r *= osc[j];
-              if (EPI == JFG_EPI_DIV_EIG) {
-                a = r;
-                r = __fdividef(r, c0 + c1 * (aux[j] + lp));
-              }
-              r *= alpha;
-              if (fdot) dsum = fmaf(a, r, dsum);
-              if (BETA) r += beta * prev[j];
-              if (H16) omax = fmaxf(omax, fabsf(r));
-              outS[(long long)m * d.out_ld + p] = r;
+            for (int j = 0; j < 16; ++j) {
+              *o = v[j];
+              o += d.out_ld;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (mh + j < d.M) *o = v[j];
+              o += d.out_ld;
             }
           }
         }
-        if (more) {
+        if (EPI == JFG_EPI_MUL_FIELD) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) aux[j] = nxt[j];
+          for (int j = 0; j < 16; ++j) f[j] = fn[j];
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1049,11 +993,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (lane == 0 && b >= 0) atomicMax(q.out_max + b, __float_as_uint(omax));
       }
     }
-    // field box loads still in flight (after a timeout) land before exit
-    for (int j = 0; j < 2; ++j)
-      if (fpend & (1u << j)) mbar_wait(&fbar[2 * ew + j], (fph >> j) & 1u, WAIT_NS);
-    // bulk tensor stores of this warp complete before the kernel ends
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1185,35 +1124,12 @@ int fill_group(const jfg_contract_desc& d, const void* op_hi, const void* op_lo,
                           (cuuint64_t)(q.seg_op_map ? d.nseg : 1)};
     cuuint64_t str[2] = {(cuuint64_t)d.op_ld * eb,
                          (cuuint64_t)(q.seg_op_map ? d.op_seg : d.op_ld * d.M) * eb};
-    // one operator row of a stage per box row: 128 B (TF32) or 64 B (16-bit)
-    const int orow = b16 ? 2 * b16_ke(d.epilogue) : 128;
-    cuuint32_t box[3] = {(cuuint32_t)(orow / eb), (cuuint32_t)q.Mtile, 1};
+    cuuint32_t box[3] = {(cuuint32_t)op_ke(b16), (cuuint32_t)q.Mtile, 1};
     const CUtensorMapDataType dt = prec == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                    : b16     ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                              : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    const CUtensorMapSwizzle sw =
-        orow == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-    JFG_TRY(make_map(&maps[1], op_hi, 3, dims, str, box, dt, sw));
-    if (lo) JFG_TRY(make_map(&maps[2], op_lo, 3, dims, str, box, dt, sw));
-  }
-  // output through TMA stores when its rows are 16-byte aligned and every
-  // 32-column group of a tile is full (else plain coalesced stores)
-  q.tma_store = 0;
-  if (al16(out) && (d.out_ld & 3) == 0 && (d.out_seg & 3) == 0 && (d.out_batch & 3) == 0 &&
-      q.Mtile % 32 == 0 && d.beta == 0.0) {
-    cuuint64_t dims[4] = {(cuuint64_t)d.P, (cuuint64_t)d.M, (cuuint64_t)d.nseg,
-                          (cuuint64_t)d.batch};
-    cuuint64_t str[3] = {(cuuint64_t)d.out_ld * 4,
-                         (cuuint64_t)(d.nseg > 1 ? d.out_seg : d.out_ld * d.M) * 4,
-                         (cuuint64_t)(d.batch > 1 ? d.out_batch : d.out_ld * d.M) * 4};
-    cuuint32_t box[4] = {32, 32, 1, 1};
-    EncodeTiledFn fn = encode_fn();
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (fn && fn(&maps[3], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)out, dims, str, box, estr,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                 CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-      q.tma_store = 1;
+    JFG_TRY(make_map(&maps[1], op_hi, 3, dims, str, box, dt));
+    if (lo) JFG_TRY(make_map(&maps[2], op_lo, 3, dims, str, box, dt));
   }
   return JFG_OK;
 }
@@ -1227,14 +1143,14 @@ long long group_tiles(const TcGroup& q) {
 // The scaled split-FP16 kernel exists for single-group launches only.
 template <int E, bool BETA, int G>
 void launch_h16(dim3 grid, size_t smem, cudaStream_t st, const TcLaunch<G>& L) {
-  if constexpr (G == 1) k_contract_tc<E, BETA, 1, 2><<<grid, NTHREADS, smem, st>>>(L);
+  if constexpr (G == 1) k_contract_tc<E, BETA, 1, 2><<<grid, nthreads(E, BETA, 2), smem, st>>>(L);
 }
 // ... and so does the plain BF16 kernel (the fast diagonalisation's passes:
 // no beta, no field)
 template <int E, bool BETA, int G>
 void launch_b1(dim3 grid, size_t smem, cudaStream_t st, const TcLaunch<G>& L) {
   if constexpr (G == 1 && !BETA && E != JFG_EPI_MUL_FIELD)
-    k_contract_tc<E, false, 1, 3><<<grid, NTHREADS, smem, st>>>(L);
+    k_contract_tc<E, false, 1, 3><<<grid, nthreads(E, false, 3), smem, st>>>(L);
 }
 
 // h16 (one group only): the scaled split-FP16 auxiliaries of that group.
@@ -1263,7 +1179,7 @@ int launch_groups(int ng, const jfg_contract_desc* const* ds, const void* const*
   const int epi = ds[0]->epilogue;
   const bool hb = ds[0]->beta != 0.0;
   long long tiles = 0;
-  int mt_max = 16, ostage = 0;
+  int mt_max = 16;
   for (int i = 0; i < ng; ++i) {
     if (ds[i]->epilogue != epi || (ds[i]->beta != 0.0) != hb) return JFG_ERR_ARG;
     JFG_TRY(fill_group(*ds[i], op_hi[i], op_lo[i], in[i], out[i], L.g[i], L.maps[i], prec,
@@ -1274,36 +1190,8 @@ int launch_groups(int ng, const jfg_contract_desc* const* ds, const void* const*
       L.g[i].op_inv = h16->op_inv;
       L.g[i].op_inv_seg = h16->op_inv_seg;
     }
-    if (cfg.store == 2 || (cfg.store == 0 && !g_tma_store)) L.g[i].tma_store = 0;
-    // single-group field-multiply launches fetch the field's 32 x 32 boxes
-    // by TMA into the epilogue's staging boxes (16-byte aligned rows needed)
-    TcGroup& q = L.g[i];
-    const jfg_contract_desc& d = *ds[i];
-    if (G == 1 && ng == 1 && d.epilogue == JFG_EPI_MUL_FIELD && q.tma_store && d.field &&
-        ((uintptr_t)d.field & 15u) == 0 && (d.field_ld & 3) == 0 && (d.field_seg & 3) == 0 &&
-        (d.field_batch & 3) == 0) {
-      q.fld_seg = (d.nseg > 1 && d.field_seg != 0) ? 1 : 0;
-      q.fld_bat = (d.batch > 1 && d.field_batch != 0) ? 1 : 0;
-      const cuuint64_t plane = (cuuint64_t)d.field_ld * d.M;
-      cuuint64_t dims[4] = {(cuuint64_t)d.P, (cuuint64_t)d.M,
-                            (cuuint64_t)(q.fld_seg ? d.nseg : 1),
-                            (cuuint64_t)(q.fld_bat ? d.batch : 1)};
-      cuuint64_t str[3] = {(cuuint64_t)d.field_ld * 4,
-                           (q.fld_seg ? (cuuint64_t)d.field_seg : plane) * 4,
-                           (q.fld_bat ? (cuuint64_t)d.field_batch : plane) * 4};
-      cuuint32_t box[4] = {32, 32, 1, 1};
-      cuuint32_t estr[4] = {1, 1, 1, 1};
-      EncodeTiledFn fn = encode_fn();
-      q.tma_field = (fn && fn(&L.fmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)d.field, dims,
-                              str, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-                         ? 1
-                         : 0;
-    }
     tiles += group_tiles(L.g[i]);
     if (L.g[i].Mtile > mt_max) mt_max = L.g[i].Mtile;
-    ostage |= L.g[i].tma_store;
   }
   if (tiles == 0) return JFG_OK;
   int dev = 0, nsm = 0;
@@ -1311,76 +1199,74 @@ int launch_groups(int ng, const jfg_contract_desc* const* ds, const void* const*
   JFG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   int ctas = cfg.ctas > 0 && cfg.ctas < nsm ? cfg.ctas : nsm;
   const int ta = (b16 || cfg.operand_a_in_tmem) ? 1 : 0;
-  // Operator-stationary schedule (16-bit operators, one group): each CTA keeps
-  // its operator chunk (every K block, hi and lo) in shared memory and streams
-  // only input tiles, halving the L2-to-SM traffic per tile.  Used when the
-  // chunk leaves room for >= 2 input stages and every slot gets >= 2 tiles
-  // per CTA.
+  // Shared memory: operator blocks and input blocks.  The input
+  // ring holds blocks of 16 KB (32 with the lo part beside it); the operator's
+  // blocks stream through a ring of their own, or (operator-stationary
+  // schedule, one group) each CTA keeps one chunk of it, all K of hi and lo,
+  // and streams only input tiles, halving the L2-to-SM traffic per tile.
+  const size_t oblock = (prec == 3 ? 1 : 2) * (size_t)mt_max * 128;
+  const size_t xblock = (ta ? 1 : 2) * (size_t)XBYTES;
+  const size_t fixed = 1024 + (5 * S_MAX + 8) * 8;
+  const size_t room = (size_t)SMEM_MAX - fixed;
   bool res = false;
-  int nslots = 0;
-  size_t res_bytes = 0;
+  int nslots = 0, nko = 0;
   const int sched = cfg.schedule == 1 ? 0 : cfg.schedule == 2 ? 2 : g_op_resident;
-  if (b16 && prec != 3 && ng == 1 && sched) {
+  if (ng == 1 && sched) {
     const TcGroup& q = L.g[0];
-    const int mch = (q.d.M + q.Mtile - 1) / q.Mtile;
-    nslots = q.d.nseg * mch;
-    res_bytes = (size_t)((q.d.K + b16_ke(epi) - 1) / b16_ke(epi)) * 2 * (size_t)q.Mtile * 2 *
-                b16_ke(epi);
+    nslots = q.d.nseg * ((q.d.M + q.Mtile - 1) / q.Mtile);
+    nko = (q.d.K + op_ke(b16) - 1) / op_ke(b16);
     const long long per_slot = (long long)((q.d.P + TILE_P - 1) / TILE_P) * q.d.batch;
-    const size_t room = (size_t)SMEM_MAX - 1024 - 64 * 8;
-    res = nslots <= ctas && (sched == 2 || per_slot * nslots >= 2LL * ctas) &&
-          res_bytes + 2 * (size_t)(b16_ke(epi) / KB) * XBYTES <= room;
+    res = nslots <= ctas && nko <= S_MAX &&
+          (sched == 2 ? nko * oblock + 2 * xblock <= room
+                      : !q.mc_inner && (nthreads(epi, hb, prec) != 608 || prec == 3) &&
+                            per_slot * nslots >= 2LL * ctas &&
+                            nko * oblock + 4 * xblock <= room);
   }
-  const int ke16 = b16_ke(epi);
-  const size_t xstage = (size_t)(ke16 / KB) * XBYTES;  // FP32 input of a 16-bit stage
-  const size_t stage = res ? xstage
-                           : b16 ? xstage + (prec == 3 ? 1 : 2) * (size_t)mt_max * 2 * ke16
-                                 : (ta ? 1 : 2) * (size_t)XBYTES + 2 * (size_t)mt_max * 128;
-  // field-multiply launches stage both of a warp's boxes of a tile (the
-  // field of each fetched ahead), when two pipeline stages still fit
-  int nbuf = ostage ? 1 : 0;
-  if (!res && ng == 1 && L.g[0].tma_field &&
-      (size_t)SMEM_MAX - 1024 - 64 * 8 - 16 * (size_t)STAGE_OUT >= 2 * stage)
-    nbuf = 2;
-  size_t ob = 8 * (size_t)STAGE_OUT * nbuf;
-  const size_t fixed = 1024 + (res ? res_bytes : 0) + 64 * 8;
-  int stages = (int)(((size_t)SMEM_MAX - fixed - ob) / stage);
-  if (res && stages < 3 && ostage && ((size_t)SMEM_MAX - fixed) / stage > (size_t)stages) {
-    // three input stages matter more than the TMA-store staging boxes
-    ostage = 0;
-    nbuf = 0;
-    ob = 0;
-    L.g[0].tma_store = 0;
-    stages = (int)(((size_t)SMEM_MAX - fixed) / stage);
+  // operand A in TMEM: 256 accumulator columns plus the slots
+  const int amax = ta ? (b16 ? 8 : 4) : S_MAX;
+  const size_t left = room - (res ? nko * oblock : 0);
+  int xs, os;
+  if (res) {
+    xs = (int)(left / xblock);
+    os = 0;
+  } else {
+    // as many bytes of operator as of input in flight (per 64 K of 16-bit
+    // operators 32 KB of each), at least two operator and two input blocks
+    const int xper = op_ke(b16) / KB;  // input blocks per operator block
+    os = (int)(left / (oblock + xper * xblock));
+    if (os < 2) os = 2;
+    if (os > S_MAX) os = S_MAX;
+    if (left < os * oblock + 2 * xblock) return JFG_ERR_UNSUPPORTED;
+    xs = (int)((left - os * oblock) / xblock);
   }
-  // operand A in TMEM: 256 accumulator columns plus one A slot per stage
-  const int amax = ta ? 256 / (b16 ? ke16 : 2 * KB) : 6;
-  if (stages > amax) stages = amax;  // <= 8: the kernel's per-stage tables hold 16
-  if (cfg.stages >= 2 && cfg.stages < stages) stages = cfg.stages;
-  if (stages < 2) return JFG_ERR_UNSUPPORTED;
-  L.stages = stages;
-  L.tmem_cols = 512;  // two accumulator buffers (+ operand A stages in TMEM mode)
+  if (xs > 12) xs = 12;
+  // whole turns of the two splitting groups
+  const int turn = 2 * op_ke(b16) / KB;
+  if (nthreads(epi, hb, prec) == 608 && xs >= turn) xs = xs / turn * turn;
+  if (cfg.stages >= 2 && cfg.stages < xs) xs = cfg.stages;
+  if (cfg.stages >= 2 && cfg.stages < os) os = cfg.stages;
+  if (xs < 2) return JFG_ERR_UNSUPPORTED;
+  L.xstages = xs;
+  L.ostages = os;
+  L.aslots = ta ? amax : xs;
+  L.tmem_cols = 512;  // two accumulator buffers (+ operand A slots in TMEM mode)
   L.tmem_a = ta;
   L.mt_max = mt_max;
-  L.out_stage = nbuf;
   L.op_res = res ? 1 : 0;
   L.nslots = res ? nslots : 0;
   if (dot && dot->part && ng == 1) {
-    // fused dot: field or divide epilogue, <= DOT_NBMAX partials per problem;
-    // split FP16 with the field loaded per element keeps the factors folded
-    // and fuses none
+    // fused dot: field or divide epilogue, <= DOT_NBMAX partials per problem
     TcGroup& q = L.g[0];
     const int e = q.d.epilogue;
     const long long nb = (long long)q.d.nseg * ((q.d.M + q.Mtile - 1) / q.Mtile) *
                          ((q.d.P + TILE_P - 1) / TILE_P) * 8;
-    if ((e == JFG_EPI_DIV_EIG || (e == JFG_EPI_MUL_FIELD && (prec != 2 || q.tma_field))) &&
-        q.d.beta == 0.0 && nb <= DOT_NBMAX) {
+    if ((e == JFG_EPI_DIV_EIG || e == JFG_EPI_MUL_FIELD) && q.d.beta == 0.0 &&
+        nb <= DOT_NBMAX) {
       q.dot_part = dot->part;
       if (dot->nb) *dot->nb = (int)nb;
     }
   }
-  const size_t smem = 1024 + res_bytes * (res ? 1 : 0) + stages * stage + ob +
-                      (3 * stages + 23) * 8 + 16;
+  const size_t smem = fixed + (res ? nko : os) * oblock + xs * xblock;
   if (smem > (size_t)SMEM_MAX) return JFG_ERR_UNSUPPORTED;
   long long nct = tiles < ctas ? tiles : ctas;
   if (res) nct = (long long)(ctas / nslots) * nslots;  // the same CTA count per slot
@@ -1397,14 +1283,14 @@ int launch_groups(int ng, const jfg_contract_desc* const* ds, const void* const*
       launch_b1<E, false, G>(grid, smem, st, L);                               \
     } else if (b16) {                                                          \
       if (hb)                                                                  \
-        k_contract_tc<E, true, G, 1><<<grid, NTHREADS, smem, st>>>(L);         \
+        k_contract_tc<E, true, G, 1><<<grid, nthreads(E, true, 1), smem, st>>>(L);         \
       else                                                                     \
-        k_contract_tc<E, false, G, 1><<<grid, NTHREADS, smem, st>>>(L);        \
+        k_contract_tc<E, false, G, 1><<<grid, nthreads(E, false, 1), smem, st>>>(L);        \
     } else {                                                                   \
       if (hb)                                                                  \
-        k_contract_tc<E, true, G, 0><<<grid, NTHREADS, smem, st>>>(L);         \
+        k_contract_tc<E, true, G, 0><<<grid, nthreads(E, true, 0), smem, st>>>(L);         \
       else                                                                     \
-        k_contract_tc<E, false, G, 0><<<grid, NTHREADS, smem, st>>>(L);        \
+        k_contract_tc<E, false, G, 0><<<grid, nthreads(E, false, 0), smem, st>>>(L);        \
     }                                                                          \
   } while (0)
   switch (epi) {
@@ -1473,21 +1359,20 @@ int tune_single(int prec, const jfg_contract_desc& d, const void* oh, const void
   for (int ta : {1, 0})
     for (int sched : {1, 2})
       for (int sg : {0, 3, 2})
-        for (int store : {1, 2})
-          for (int mt : {0, 64}) {
-            if ((prec != 0 && ta == 0) || ((prec == 0 || prec == 3) && sched == 2)) continue;
+        for (int mt : {0, 64}) {
+            if (prec != 0 && ta == 0) continue;
             // the operator-stationary schedule only where the chunk fits beside
-            // two input stages (else the launch would stream anyway)
-            if (sched == 2 && (size_t)((d.K + b16_ke(d.epilogue) - 1) / b16_ke(d.epilogue)) *
-                                          2 * (mt ? mt : 128) * 2 * b16_ke(d.epilogue) +
-                                      2 * (size_t)(b16_ke(d.epilogue) / KB) * XBYTES >
-                                  (size_t)SMEM_MAX - 1024 - 64 * 8)
+            // two input blocks (else the launch would stream anyway)
+            const int ke = op_ke(prec != 0);
+            if (sched == 2 && (size_t)((d.K + ke - 1) / ke) * (prec == 3 ? 1 : 2) *
+                                          (mt ? mt : 128) * 128 +
+                                      2 * (size_t)XBYTES >
+                                  (size_t)SMEM_MAX - 4096)
               continue;
             jfg_tc_config c = tc_default_config();
             c.operand_a_in_tmem = ta;
             c.schedule = sched;
             c.stages = sg;
-            c.store = store;
             c.mtile = mt;
             cands.push_back(c);
           }
@@ -1699,9 +1584,7 @@ extern "C" void jfg_split_bf16_host(size_t n, const double* src, uint16_t* hi, u
 }
 
 extern "C" int jfg_tc_set_store_path(int tma_store) {
-  if (tma_store != 0 && tma_store != 1) return JFG_ERR_ARG;
-  jfg::g_tma_store = tma_store;
-  return JFG_OK;
+  return tma_store != 0 && tma_store != 1 ? JFG_ERR_ARG : JFG_OK;
 }
 
 extern "C" int jfg_tc_set_wait_budget_ns(unsigned long long ns) {
