@@ -241,27 +241,38 @@ __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
 // the contraction
 // ---------------------------------------------------------------------------
 
-// MMAs that keep operand A in the collector buffer, or take it from there
+// FP16 MMAs with the operand A use of the collector buffer (plain: read and
+// dropped).  Issued by the lane with leader set, as one predicated instruction:
+// the warp does not branch, so that descriptors (32-bit address words, the
+// rest is constant) stay in uniform registers.
 #define JFG_MMA_COLLECT(NAME, USAGE)                                                          \
-  __device__ __forceinline__ void NAME(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,    \
-                                       uint32_t accum) {                                      \
+  __device__ __forceinline__ void NAME(uint32_t d, uint32_t a, uint32_t b, uint32_t desc_hi,  \
+                                       uint32_t idesc, uint32_t accum, uint32_t leader) {     \
     asm volatile(                                                                             \
-        "{\n\t.reg .pred p;\n\t"                                                             \
-        "setp.ne.b32 p, %4, 0;\n\t"                                                          \
-        "tcgen05.mma.cta_group::1.kind::f16.collector::a::" USAGE " [%0], %1, %2, %3, p;\n\t}" \
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accum));                                    \
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"                                       \
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"                                  \
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"                                  \
+        "@q tcgen05.mma.cta_group::1.kind::f16" USAGE " [%0], da, db, %4, p;\n\t}" ::"r"(d),  \
+        "r"(a), "r"(b), "r"(desc_hi), "r"(idesc), "r"(accum), "r"(leader));                   \
   }
-JFG_MMA_COLLECT(mma_fill, "fill")
-JFG_MMA_COLLECT(mma_use, "use")
-JFG_MMA_COLLECT(mma_lastuse, "lastuse")
+JFG_MMA_COLLECT(mma_plain, "")
+JFG_MMA_COLLECT(mma_fill, ".collector::a::fill")
+JFG_MMA_COLLECT(mma_use, ".collector::a::use")
+JFG_MMA_COLLECT(mma_lastuse, ".collector::a::lastuse")
 #undef JFG_MMA_COLLECT
-
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* r) {
+__device__ __forceinline__ void commit_if(uint64_t* bar, uint32_t leader) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(addr));
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          tc::smem_u32(bar)),
+      "r"(leader)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
 }
 // wait for the loads into r[0..31] (the operands order the uses after it)
 __device__ __forceinline__ void tmem_wait32(uint32_t* r) {
@@ -298,7 +309,7 @@ __device__ __noinline__ double plain_sum(const double* a, const double* y, int K
 
 // H + lo 2^-32 (both below 2^51 in magnitude) rounded to nearest even as a
 // double times 2^sh; rare is set when its exponent leaves the normal range.
-// No branches: the eight columns of a step run interleaved.
+// No branches: the four columns of a step run interleaved.
 __device__ __forceinline__ double level_value(long long H, long long lo, int sh, bool& rare) {
   H += lo >> 32;
   uint32_t w2 = (uint32_t)(H >> 32), w1 = (uint32_t)H, w0 = (uint32_t)lo;
@@ -400,7 +411,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
 
   // items: (problem slot, segment, p tile), all operator tiles of each; with
   // fewer of these than CTAs, every operator tile is an item of its own
-  const int nb = s_nb;
+  const int nb = __shfl_sync(0xffffffffu, s_nb, 0);
   const unsigned base_items = (unsigned)nb * d.nseg * L.nptiles;
   const int msplit = (base_items < gridDim.x) ? L.mtiles : 1;
   const unsigned items = base_items * msplit;
@@ -460,23 +471,31 @@ __global__ void __launch_bounds__(SL_NT, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    // the whole warp walks the loop, one elected lane issues
-    const uint64_t ad0 = tc::sdesc_sw128(tc::smem_u32(as));
-    const uint64_t bd0 = tc::sdesc_sw128(tc::smem_u32(bs));
+    // The whole warp walks the loop, one elected lane issues.  Every branch is
+    // on a warp-uniform value (waits through a vote): otherwise the addresses
+    // leave the uniform registers and an MMA costs 64 clocks instead of 40 (4 x
+    // 256^3 round: 4.34 ms then, 3.56 ms so; 32 x 256^2: 139 and 122 us).
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_sl_status)) != 0;
+    };
+    const uint32_t ad0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(as));
+    const uint32_t bd0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(bs));
+    const uint32_t dhi = (uint32_t)(tc::sdesc_sw128(0) >> 32);
+    const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc =  // FP16 x FP16 -> FP32, M = 128, N = 2 PT
         (1u << 4) | ((uint32_t)(2 * PT) >> 3 << 17) | ((128u >> 4) << 24);
     int st = 0, bslot = 0;
     uint32_t aph = 0, bph = 0, unit = 0;
     bool ok = true, any = false;
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
-      if (!tc::mbar_wait(&bfull[bslot], bph, &g_sl_status)) {
+      if (!wait(&bfull[bslot], bph)) {
         ok = false;
         break;
       }
-      const uint64_t bdt = bd0 + (((uint32_t)bslot * bbytes) >> 4);
+      const uint32_t bdt = bd0 + (((uint32_t)bslot * bbytes) >> 4);
       for (int mi = 0; ok && mi < mt_n; ++mi, ++unit) {
         const uint32_t db = unit & 1u;
-        if (unit >= 2 && !tc::mbar_wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u, &g_sl_status)) {
+        if (unit >= 2 && !wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
           ok = false;
           break;
         }
@@ -486,59 +505,52 @@ __global__ void __launch_bounds__(SL_NT, 1)
         for (int kb = 0; ok && kb < L.nkb; ++kb) {
           const int rest = d.K - kb * 64;
           const int n16 = rest >= 64 ? 4 : (rest + 15) / 16;
-          const uint64_t bdk = bdt + (((uint32_t)kb * KBLK) >> 4);
+          const uint32_t bdk = bdt + (((uint32_t)kb * KBLK) >> 4);
 #pragma unroll
           for (int i = 0; i < NS; ++i) {
-            if (!tc::mbar_wait(&afull[st], aph, &g_sl_status)) {
+            if (!wait(&afull[st], aph)) {
               ok = false;
               break;
             }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             any = true;
-            const uint64_t ad = ad0 + (((uint32_t)st * ABYTES) >> 4);
-            if (elect_one()) {
+            const uint32_t ad = ad0 + (((uint32_t)st * ABYTES) >> 4);
 #pragma unroll
-              for (int kk = 0; kk < 4; ++kk) {
-                if (kk >= n16) break;
-                const uint32_t more = (kb | kk | i) ? 1u : 0u;
-                // pairs h = (i + 1) / 2 .. 3 share the operator tile: it stays
-                // in the collector buffer from the first to the last
+            for (int kk = 0; kk < 4; ++kk) {
+              if (kk >= n16) break;
+              const uint32_t more = (kb | kk | i) ? 1u : 0u;
+              // pairs h = i / 2 .. 3 share the operator tile: it stays in the
+              // collector buffer from the first to the last
 #pragma unroll
-                for (int h = 3; h >= i / 2; --h) {
-                  const uint64_t bd = bdk + (((uint32_t)(2 * h - i + 1) * DBLK + 32 * kk) >> 4);
-                  const uint32_t D = acc + 2 * PT * h;
-                  if (h == 3 && h == i / 2)
-                    tc::mma_bf16(D, ad + 2 * kk, bd, idesc, more);
-                  else if (h == 3)
-                    mma_fill(D, ad + 2 * kk, bd, idesc, more);
-                  else if (h == i / 2)
-                    mma_lastuse(D, ad + 2 * kk, bd, idesc, more);
-                  else
-                    mma_use(D, ad + 2 * kk, bd, idesc, more);
-                }
+              for (int h = 3; h >= i / 2; --h) {
+                const uint32_t bd = bdk + (((uint32_t)(2 * h - i + 1) * DBLK + 32 * kk) >> 4);
+                const uint32_t D = acc + 2 * PT * h;
+                if (h == 3 && h == i / 2)
+                  mma_plain(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+                else if (h == 3)
+                  mma_fill(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+                else if (h == i / 2)
+                  mma_lastuse(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+                else
+                  mma_use(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
               }
-              if (!L.a_res) tc::mma_commit(&aempty[st]);
             }
-            __syncwarp();
+            if (!L.a_res) commit_if(&aempty[st], leader);
             if (++st == L.astages) {
               st = 0;
               if (!L.a_res) aph ^= 1u;
             }
           }
         }
-        if (ok && elect_one()) tc::mma_commit(&dfull[db]);
-        __syncwarp();
+        if (ok) commit_if(&dfull[db], leader);
       }
-      if (ok && elect_one()) tc::mma_commit(&bempty[bslot]);
-      __syncwarp();
+      if (ok) commit_if(&bempty[bslot], leader);
       if (++bslot == L.bbuf) {
         bslot = 0;
         bph ^= 1u;
       }
     }
     if (any) {  // every MMA has finished before TMEM is freed
-      if (elect_one()) tc::mma_commit(done);
-      __syncwarp();
+      commit_if(done, leader);
       tc::mbar_wait(done, 0, &g_sl_status);
     }
   } else if (warp < 2 + NWS) {
@@ -677,47 +689,47 @@ __global__ void __launch_bounds__(SL_NT, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + db * (NS * PT) + ((uint32_t)(32 * quarter) << 16);
+        if (m0 >= d.M) {  // no row of this quarter
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&dempty[db]);
+          continue;
+        }
+        // four columns of all levels at a time, staged for stores of eight
 #pragma unroll 1
-        for (int cb = 0; cb < PT / 16; ++cb) {
-          const int col0 = half * (PT / 2) + cb * 8;
-          long long H[8];
+        for (int g = 0; g < PT / 8; ++g) {
+          const int col4 = half * (PT / 2) + 4 * g;
           uint32_t r[32];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) tmem_ld8(acc + j * PT + col0, r + 8 * j);
+          for (int j = 0; j < NS; ++j) tmem_ld4(acc + j * PT + col4, r + 4 * j);
           tmem_wait32(r);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) H[c] = level_join(r[c], r[8 + c], r[16 + c], r[24 + c]);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) tmem_ld8(acc + (4 + j) * PT + col0, r + 8 * j);
-          tmem_wait32(r);
-          if (cb == PT / 16 - 1) {  // the accumulators are read: the next tile may have them
+          if (g == PT / 8 - 1) {  // the accumulators are read: the next tile may have them
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&dempty[db]);
           }
-          int Ep[8];
-#pragma unroll
-          for (int c = 0; c < 8; c += 4)
-            *reinterpret_cast<int4*>(Ep + c) =
-                *reinterpret_cast<const int4*>(row_e + ring * PT + col0 + c);
+          const int4 E4 = *reinterpret_cast<const int4*>(row_e + ring * PT + col4);
+          const int Ep[4] = {E4.x, E4.y, E4.z, E4.w};
+          double* cell = st8 + lane * STG_LD + 4 * (g & 1);
           unsigned rare = 0;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < 4; ++c) {
             bool x;
-            st8[lane * STG_LD + c] =
-                level_value(H[c], level_join(r[c], r[8 + c], r[16 + c], r[24 + c]),
-                            Ea + Ep[c] - 2080, x);
+            cell[c] = level_value(level_join(r[c], r[4 + c], r[8 + c], r[12 + c]),
+                                  level_join(r[16 + c], r[20 + c], r[24 + c], r[28 + c]),
+                                  Ea + Ep[c] - 2080, x);
             rare |= (x || Ea + Ep[c] >= BIG) ? 1u << c : 0u;
           }
           if (rare && m < d.M && b >= 0) {
             const double* a = L.op + (long long)os * d.op_seg + (long long)m * d.op_ld;
 #pragma unroll 1
-            for (int c = 0; c < 8; ++c) {
-              const int p = pt * PT + col0 + c;
+            for (int c = 0; c < 4; ++c) {
+              const int p = pt * PT + col4 + c;
               if ((rare >> c & 1u) && p < d.P)
-                st8[lane * STG_LD + c] = plain_sum(a, L.in + ib + (long long)p * d.in_ld, d.K);
+                cell[c] = plain_sum(a, L.in + ib + (long long)p * d.in_ld, d.K);
             }
           }
+          if (!(g & 1)) continue;
+          const int col0 = col4 - 4;
           __syncwarp();
           const int p = pt * PT + col0 + sc;
           if (p < d.P && b >= 0) {

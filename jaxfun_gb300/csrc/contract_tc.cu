@@ -428,9 +428,10 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
   }
   __syncthreads();
   const unsigned long long budget = s_budget;
-  const long long ntiles = tb[L.ngroups];
+  const long long ntiles = __shfl_sync(0xffffffffu, tb[L.ngroups], 0);
   const int r_nptiles = (L.g[0].d.P + TILE_P - 1) / TILE_P;
-  const long long r_cnt = res ? (long long)nbs[0] * r_nptiles : 0;  // tiles of one slot
+  const long long r_cnt =  // tiles of one slot
+      res ? (long long)__shfl_sync(0xffffffffu, nbs[0], 0) * r_nptiles : 0;
   if (!res && (long long)blockIdx.x >= ntiles) return;  // no tile for this CTA (uniform)
   if (res && r_j0 >= r_cnt) return;
 
@@ -636,6 +637,11 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
     // lane issues: from a lane-0 branch every MMA cost ~99 clocks of address
     // and register moves, whatever its N; this way one of N = 128 takes the
     // tensor pipe's 64 (measured alone).  Same MMAs in the same order.
+    // Every branch is on a warp-uniform value (waits through a vote), or the
+    // addresses would leave the uniform registers.
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget)) != 0;
+    };
     int li = 0;
     bool ok = true, issued_any = false;
     const uint64_t od0 = sdesc(smem_u32(obase));
@@ -645,6 +651,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
     uint32_t aph = 0, oph = 0;   // their use count parities
     unsigned kn = 0;             // K blocks so far, modulo S_MAX
     for (; ok && tile_of(li, gi, pt, mc, b, s, false); ++li) {
+      if (G > 1) gi = __shfl_sync(0xffffffffu, gi, 0);
       const int mtile = __shfl_sync(0xffffffffu, L.g[gi].Mtile, 0);
       const uint32_t idesc = H16   ? idesc_f16(TILE_P, mtile)
                              : B16 ? idesc_b16(TILE_P, mtile)
@@ -652,7 +659,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
       const int nko = __shfl_sync(0xffffffffu, nkx_of(gi) / KXO, 0);
       const int buf = li & 1;
       const uint32_t use = (uint32_t)(li >> 1);
-      if (li >= 2 && !mbar_wait(&tempty[buf], (use & 1u) ^ 1u, budget)) {
+      if (li >= 2 && !wait(&tempty[buf], (use & 1u) ^ 1u)) {
         ok = false;
         break;
       }
@@ -660,8 +667,8 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
       const uint32_t acc = tmem + (uint32_t)buf * acc_stride;
       if (res) so = 0;
       for (int ko = 0; ko < nko; ++ko) {
-        if (!mbar_wait(&ofull[so], res ? 0u : oph, budget) ||
-            !mbar_wait(&conv[sl], aph, budget)) {
+        if (!wait(&ofull[so], res ? 0u : oph) ||
+            !wait(&conv[sl], aph)) {
           ok = false;
           break;
         }
