@@ -353,7 +353,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
     k_contract_sl(const __grid_constant__ SlLaunch L) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_nb;
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  // aligned by an offset, so that accesses stay in the shared window for the
+  // compiler (through an integer they become generic ones, which it must order
+  // against the global stores)
+  uint8_t* smem = smem_raw + ((0u - tc::smem_u32(smem_raw)) & 1023u);
   const jfg_contract_desc& d = L.d;
   constexpr uint32_t DBLK = (uint32_t)PT * 128;        // one digit of one K block
   constexpr uint32_t KBLK = (NS + 1) * DBLK;           // zero block and digits
@@ -770,8 +773,341 @@ __global__ void __launch_bounds__(SL_NT, 1)
   }
 }
 
+// ---------------------------------------------------------------------------
+// the contraction for small operators (M <= 64, K <= 64, shared by all rows)
+// ---------------------------------------------------------------------------
+
+// The roles of the operands are swapped: 128 input rows, flattened over the
+// problems so that short ones leave no tile part empty, are the MMA's M
+// operand, and the operator's digits (in two halves of 32 rows) its resident N
+// operand.  Above, an operator of 64 rows fills half of the MMA's M, and half
+// of the TMEM lanes and with them the epilogue of two of the four schedulers:
+// 1024 problems of 64 x 62 spent 11.1k clocks per 32 rows, 8k of them in the
+// epilogue.  Lanes are input rows here, so results go straight to memory,
+// coalesced, without staging.  Two passes: 1024 x 64 x 62 167 -> 105 us, 3000 x
+// 51 x 49 465 -> 176, 3000 x 33 x 31 334 -> 103.
+//
+// One input tile fits (eight digits of 128 rows, 128 KB), so cutting a tile
+// waits for the MMAs of the one before; the epilogue of either half overlaps
+// both (two accumulator sets of 256 columns).
+constexpr int RT = 128;                            // input rows of a tile
+constexpr int RM = 32;                             // operator rows of a unit
+constexpr uint32_t RBLK = RM * 128;                // one digit of one unit
+constexpr uint32_t RUNIT = (NS + 1) * RBLK;        // zero block and digits
+constexpr size_t ROWS_SMEM = 1024 + NS * ABYTES + 2 * RUNIT + RING * RT * 4 + 64 * 4 + 16 * 8;
+
+template <int EPI, bool BETA>
+__global__ void __launch_bounds__(SL_NT, 1)
+    k_contract_sl_rows(const __grid_constant__ SlLaunch L) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int s_nb;
+  uint8_t* smem = smem_raw + ((0u - tc::smem_u32(smem_raw)) & 1023u);
+  const jfg_contract_desc& d = L.d;
+  uint8_t* as = smem;                                 // [NS][RT][64]
+  uint8_t* bs = as + NS * ABYTES;                     // [2][1 + NS][RM][64]
+  int* row_e = (int*)(bs + 2 * RUNIT);                // [RING][RT]
+  int* op_e = row_e + RING * RT;                      // [64]
+  uint64_t* bars = (uint64_t*)(op_e + 64);
+  uint64_t* ofull = bars;
+  uint64_t* bfull = bars + 1;
+  uint64_t* bempty = bars + 2;
+  uint64_t* done = bars + 3;
+  uint64_t* dfull = bars + 4;
+  uint64_t* dempty = bars + 6;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 8);
+
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  const int units = (d.M + RM - 1) / RM;  // 1 or 2
+  if (threadIdx.x == 0) {
+    s_nb = active_count(d.batch_list, d.batch_count, d.batch);
+    tc::mbar_init(ofull, 1);
+    tc::mbar_init(bfull, NWS);
+    tc::mbar_init(bempty, 1);
+    tc::mbar_init(done, 1);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&dfull[i], 1);
+      tc::mbar_init(&dempty[i], NWE);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect_tx(ofull, (uint32_t)units * NS * RBLK);
+    for (int v = 0; v < units; ++v)
+      for (int i = 0; i < NS; ++i)
+        tc::tma_load_3d(bs + v * RUNIT + (i + 1) * RBLK, &L.amap, ofull, 0, v * RM, i);
+  }
+  if (threadIdx.x < 64) op_e[threadIdx.x] = (int)threadIdx.x < d.M ? __ldg(L.row_e + threadIdx.x) : 0;
+  for (int i = threadIdx.x; i < 2 * (int)(RBLK / 16); i += SL_NT)
+    *reinterpret_cast<uint4*>(bs + (i / (RBLK / 16)) * RUNIT + (i % (RBLK / 16)) * 16) =
+        make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc::smem_u32(tmem_slot)),
+                 "r"(2 * NS * RM)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  // items: (segment, tile of RT flattened rows)
+  const int nb = __shfl_sync(0xffffffffu, s_nb, 0);
+  const unsigned R = (unsigned)nb * (unsigned)d.P;
+  const unsigned per_seg = (R + RT - 1) / RT;
+  const unsigned items = per_seg * (unsigned)d.nseg;
+  // row of an item: problem (-1: none), segment and p
+  auto locate = [&](unsigned t, int row, int& b, int& s, int& p) {
+    s = (int)(t / per_seg);
+    const unsigned r = (t - (unsigned)s * per_seg) * RT + (unsigned)row;
+    const unsigned slot = r / (unsigned)d.P;
+    p = (int)(r - slot * (unsigned)d.P);
+    b = r < R ? active_problem(d.batch_list, nb, d.batch, (int)slot) : -1;
+  };
+
+  if (warp == 0) {
+    // the operator has landed before the CTA may end
+    if (lane == 0) tc::mbar_wait(ofull, 0, &g_sl_status);
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (uniform walk as above) ----------------
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_sl_status)) != 0;
+    };
+    const uint32_t ad0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(as));
+    const uint32_t bd0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(bs));
+    const uint32_t dhi = (uint32_t)(tc::sdesc_sw128(0) >> 32);
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc =  // FP16 x FP16 -> FP32, M = 128, N = 2 RM
+        (1u << 4) | ((uint32_t)(2 * RM) >> 3 << 17) | ((128u >> 4) << 24);
+    const int n16 = (d.K + 15) / 16;
+    uint32_t unit = 0, ph = 0;
+    bool any = false;
+    bool ok = blockIdx.x >= items || wait(ofull, 0);
+    for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x, ph ^= 1u) {
+      if (!wait(bfull, ph)) break;
+      for (int v = 0; v < units; ++v, ++unit) {
+        const uint32_t db = unit & 1u;
+        if (unit >= 2 && !wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        any = true;
+        const uint32_t acc = tmem + db * (NS * RM);
+        const uint32_t bdv = bd0 + (((uint32_t)v * RUNIT) >> 4);
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+          const uint32_t ad = ad0 + (((uint32_t)i * ABYTES) >> 4);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            if (kk >= n16) break;
+            const uint32_t more = (kk | i) ? 1u : 0u;
+#pragma unroll
+            for (int h = 3; h >= i / 2; --h) {
+              const uint32_t bd = bdv + (((uint32_t)(2 * h - i + 1) * RBLK + 32 * kk) >> 4);
+              const uint32_t D = acc + 2 * RM * h;
+              if (h == 3 && h == i / 2)
+                mma_plain(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+              else if (h == 3)
+                mma_fill(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+              else if (h == i / 2)
+                mma_lastuse(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+              else
+                mma_use(D, ad + 2 * kk, bd, dhi, idesc, more, leader);
+            }
+          }
+        }
+        commit_if(&dfull[db], leader);
+      }
+      if (ok) commit_if(bempty, leader);
+    }
+    if (any) {  // every MMA has finished before TMEM is freed
+      commit_if(done, leader);
+      tc::mbar_wait(done, 0, &g_sl_status);
+    }
+  } else if (warp < 2 + NWS) {
+    // ---------------- cut the input rows into digits ----------------
+    // a lane takes 8 consecutive elements of four rows 32 apart; the chunk
+    // order lets a quarter-warp store to different 16-byte columns
+    const int u = lane >> 2;
+    const int cu = (u >> 1) | ((u & 1) << 2);
+    const int k0 = 8 * cu;
+    const int row0 = 4 * (warp - 2) + (lane & 3);
+    const uint4 ce = __ldg((const uint4*)(L.col_e + k0));
+    uint8_t* dst = as + row0 * 128 + ((cu ^ (row0 & 7)) << 4);
+    double x[4][8];
+    auto load = [&](unsigned t) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        int b, s, p;
+        locate(t, 32 * i + row0, b, s, p);
+        const double* src = L.in + (long long)(b < 0 ? 0 : b) * d.in_batch +
+                            (long long)s * d.in_seg + (long long)p * d.in_ld + k0;
+        if (b >= 0 && k0 + 8 <= d.K) {
+          if (L.vec2) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              const double2 v = __ldg((const double2*)(src + e));
+              x[i][e] = v.x;
+              x[i][e + 1] = v.y;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[i][e] = __ldg(src + e);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[i][e] = b >= 0 && k0 + e < d.K ? __ldg(src + e) : 0.0;
+        }
+      }
+    };
+    uint32_t n = 0;
+    if (blockIdx.x < items) load(blockIdx.x);
+    for (unsigned t = blockIdx.x; t < items; t += gridDim.x, ++n) {
+      int E[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        E[i] = -(1 << 19);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int v = not_finite(x[i][e]) ? SPECIAL : elem_e(x[i][e], short_of(ce, e));
+          if (!is_zero(x[i][e])) E[i] = max(E[i], v);
+        }
+      }
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) E[i] = max(E[i], __shfl_xor_sync(0xffffffffu, E[i], o));
+      if (n >= 1 && !tc::mbar_wait(bempty, (n & 1u) ^ 1u, &g_sl_status)) break;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (E[i] < -(1 << 18)) E[i] = 0;
+        if (u == 0) row_e[(n & (RING - 1)) * RT + 32 * i + row0] = E[i];
+        unsigned long long f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          f[e] = biased_fixed(x[i][e], elem_e(x[i][e], short_of(ce, e)), E[i]);
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          uint4 v;
+          v.x = digit_pair(f[0], f[1], j);
+          v.y = digit_pair(f[2], f[3], j);
+          v.z = digit_pair(f[4], f[5], j);
+          v.w = digit_pair(f[6], f[7], j);
+          *reinterpret_cast<uint4*>(dst + i * (32 * 128) + j * ABYTES) = v;
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bfull);
+      if (t + gridDim.x < items) load(t + gridDim.x);
+    }
+  } else {
+    // ---------------- epilogue: a lane is an input row ----------------
+    const int quarter = warp & 3, half = (warp - 2 - NWS) >> 2;
+    const int row = 32 * quarter + lane;
+    uint32_t unit = 0, n = 0;
+    bool ok = true;
+    for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x, ++n) {
+      int b, s, p;
+      locate(t, row, b, s, p);
+      const long long ib = (long long)(b < 0 ? 0 : b);
+      double* outP = L.out + ib * d.out_batch + (long long)s * d.out_seg + p;
+      const double* f = (const double*)d.field + ib * d.field_batch + (long long)s * d.field_seg + p;
+      double c0 = 0.0, c1 = 1.0, lp = 0.0;
+      if (EPI == JFG_EPI_DIV_EIG && b >= 0) {
+        if (d.c0) c0 = ((const double*)d.c0)[b];
+        if (d.c1) c1 = ((const double*)d.c1)[b];
+        lp = __ldg((const double*)d.lam_p + p);
+      }
+      int Ep = 0;
+      for (int v = 0; v < units; ++v, ++unit) {
+        const uint32_t db = unit & 1u;
+        if (!tc::mbar_wait(&dfull[db], (unit >> 1) & 1u, &g_sl_status)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // read before any accumulator of the tile is handed back: the ring
+        // may be written again three tiles on
+        if (v == 0) Ep = row_e[(n & (RING - 1)) * RT + row];
+        const uint32_t acc = tmem + db * (NS * RM) + ((uint32_t)(32 * quarter) << 16);
+        const int col0 = half * (RM / 2);
+        const int live = min(RM / 2, d.M - v * RM - col0);  // columns with an operator row
+        const int steps = live > 0 ? (live + 3) / 4 : 0;
+        if (steps == 0) {
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&dempty[db]);
+        }
+#pragma unroll 1
+        for (int g = 0; g < steps; ++g) {
+          const int col4 = col0 + 4 * g, m = v * RM + col4;
+          uint32_t r[32];
+#pragma unroll
+          for (int j = 0; j < NS; ++j) tmem_ld4(acc + j * RM + col4, r + 4 * j);
+          tmem_wait32(r);
+          if (g == steps - 1) {  // the accumulators are read: the next unit may have them
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&dempty[db]);
+          }
+          const int4 A4 = *reinterpret_cast<const int4*>(op_e + m);
+          const int Ea[4] = {A4.x, A4.y, A4.z, A4.w};
+          double val[4];
+          unsigned rare = 0;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            bool xr;
+            val[c] = level_value(level_join(r[c], r[4 + c], r[8 + c], r[12 + c]),
+                                 level_join(r[16 + c], r[20 + c], r[24 + c], r[28 + c]),
+                                 Ea[c] + Ep - 2080, xr);
+            rare |= (xr || Ea[c] + Ep >= BIG) ? 1u << c : 0u;
+          }
+          if (b < 0) continue;
+          if (rare) {
+            const double* y = L.in + ib * d.in_batch + (long long)s * d.in_seg + (long long)p * d.in_ld;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if ((rare >> c & 1u) && m + c < d.M)
+                val[c] = plain_sum(L.op + (long long)(m + c) * d.op_ld, y, d.K);
+          }
+          double* o = outP + (long long)m * d.out_ld;
+          const double* fm = f + (long long)m * d.field_ld;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (m + c < d.M) {
+              double w = val[c];
+              if (EPI == JFG_EPI_MUL_FIELD)
+                w *= __ldg(fm);
+              else if (EPI == JFG_EPI_DIV_EIG)
+                w = w / (c0 + c1 * (__ldg((const double*)d.lam_m + m + c) + lp));
+              if (L.scaled) w *= d.alpha;
+              if (BETA) w += d.beta * *o;
+              *o = w;
+            }
+            o += d.out_ld;
+            if (EPI == JFG_EPI_MUL_FIELD) fm += d.field_ld;
+          }
+        }
+      }
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(2 * NS * RM));
+  }
+}
+
 template <int EPI, bool BETA>
 int set_attr() {
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl_rows<EPI, BETA>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ROWS_SMEM));
   JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, BETA, 32>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)SMEM_LIMIT - 1024));
@@ -813,6 +1149,29 @@ int launch(const SlLaunch& L, dim3 grid, size_t smem, cudaStream_t st) {
     k_contract_sl<E, true, PT><<<grid, SL_NT, smem, st>>>(L);            \
   else                                                                   \
     k_contract_sl<E, false, PT><<<grid, SL_NT, smem, st>>>(L)
+  switch (L.d.epilogue) {
+    case JFG_EPI_NONE:
+      JFG_SL(JFG_EPI_NONE);
+      break;
+    case JFG_EPI_MUL_FIELD:
+      JFG_SL(JFG_EPI_MUL_FIELD);
+      break;
+    default:
+      JFG_SL(JFG_EPI_DIV_EIG);
+      break;
+  }
+#undef JFG_SL
+  JFG_LAUNCHED();
+  return JFG_OK;
+}
+
+int launch_rows(const SlLaunch& L, dim3 grid, cudaStream_t st) {
+  const bool beta = L.d.beta != 0.0;
+#define JFG_SL(E)                                                            \
+  if (beta)                                                                  \
+    k_contract_sl_rows<E, true><<<grid, SL_NT, ROWS_SMEM, st>>>(L);          \
+  else                                                                       \
+    k_contract_sl_rows<E, false><<<grid, SL_NT, ROWS_SMEM, st>>>(L)
   switch (L.d.epilogue) {
     case JFG_EPI_NONE:
       JFG_SL(JFG_EPI_NONE);
@@ -938,11 +1297,20 @@ int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, do
   const int Kp = kp8(d.K);
   const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)op.M, (cuuint64_t)(op.nseg * NS)};
   const cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * op.M};
-  const cuuint32_t box[3] = {64, 128, 1}, estr[3] = {1, 1, 1};
+  // Small operators: 128 flattened rows per tile, unless so few that the SMs
+  // are better spread over 32-row tiles.  Two passes and the digits take about
+  // 27 + 20 us per wave of 128-row tiles and 22 + 10.5 us per wave of 32-row
+  // ones (64 x 62; less on either side for smaller ones): 150 problems (1 wave
+  // to 2) 47 and 43 us, 200 (1 to 3) 47 and 52, 1024 (4 to 14) 105 and 167.
+  const long long row_tiles = d.nseg * (((long long)d.batch * d.P + RT - 1) / RT);
+  const bool rows = L.op_segs == 1 && d.M <= 64 && d.K <= 64 && row_tiles <= 0xFFFFFF &&
+                    (items + sms - 1) / sms > 2 * ((row_tiles + sms - 1) / sms);
+  const cuuint32_t box[3] = {64, rows ? (cuuint32_t)RM : 128u, 1}, estr[3] = {1, 1, 1};
   if (enc(&L.amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)op.dig, dims, strides, box, estr,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return JFG_ERR_ARG;
+  if (rows) return launch_rows(L, dim3((unsigned)(row_tiles < sms ? row_tiles : sms)), st);
   const dim3 grid((unsigned)(items < sms ? items : sms));
   const size_t smem = fixed + (size_t)L.astages * ABYTES;
   return PT == 32 ? launch<32>(L, grid, smem, st) : launch<16>(L, grid, smem, st);
