@@ -45,9 +45,10 @@
 // operator digits fit in the stages (M <= 128, K <= 64) they are loaded once
 // per CTA.
 //
-// The epilogue uses integers throughout: on the FP64 pipe (a warp instruction
-// holds its scheduler's share for 64 clocks) even the two additions that would
-// round a result cost more than the 35 integer instructions.
+// The epilogue keeps FP64 instructions to the two that round a result: a warp
+// instruction holds its scheduler's share of that pipe for 64 clocks.  alpha
+// and beta are a template flag (LIN) for the same reason: as run-time
+// conditions the product by alpha was computed and dropped.
 //
 // Warps: 0 TMA producer, 1 TMEM allocator and MMA issuer, 2-9 cut the input,
 // 10-17 epilogue (two per TMEM lane quarter).  Every wait is bounded
@@ -98,7 +99,6 @@ struct SlLaunch {
   int astages;
   int a_res;             // 1: every operator tile has its own stage, loaded once
   int vec2;              // input rows are 16-byte aligned
-  int scaled;            // alpha != 1
   int nptiles, mtiles;
 };
 
@@ -307,48 +307,24 @@ __device__ __noinline__ double plain_sum(const double* a, const double* y, int K
   return v;
 }
 
-// H + lo 2^-32 (both below 2^51 in magnitude) rounded to nearest even as a
-// double times 2^sh; rare is set when its exponent leaves the normal range.
-// No branches: the four columns of a step run interleaved.
+// H + lo 2^-32 (integers below 2^51 in magnitude) rounded to nearest even as
+// a double times 2^sh; rare is set when its exponent leaves the normal range.
+// H and lo become doubles of 1.5 2^52 + H and + lo by one integer addition
+// each; H - 1.5 2^20 is exact, and in the one fused multiply-add the offsets
+// cancel.  The two FP64 instructions hold the scheduler's share of that pipe
+// for 64 clocks each, but next to the MMAs it is idle: in integers (shifts,
+// carries, leading zeros: some 60 instructions) 8 x 128^3 took 588 us, so 510.
 __device__ __forceinline__ double level_value(long long H, long long lo, int sh, bool& rare) {
-  H += lo >> 32;
-  uint32_t w2 = (uint32_t)(H >> 32), w1 = (uint32_t)H, w0 = (uint32_t)lo;
-  const uint32_t s = (uint32_t)((int)w2 >> 31);
-  // magnitude of the 96-bit number: ones' complement and 1 if negative
-  asm("{\n\t"
-      "xor.b32 %0, %0, %3;\n\txor.b32 %1, %1, %3;\n\txor.b32 %2, %2, %3;\n\t"
-      "add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;\n\t}"
-      : "+r"(w0), "+r"(w1), "+r"(w2)
-      : "r"(s), "r"(s & 1u));
-  int e = sh + 1086;  // biased exponent of a number whose top bit is bit 95
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {  // whole words of leading zeros
-    const bool z = w2 == 0;
-    w2 = z ? w1 : w2;
-    w1 = z ? w0 : w1;
-    w0 = z ? 0u : w0;
-    e = z ? e - 32 : e;
-  }
-  const int z = __clz((int)w2);
-  w2 = __funnelshift_l(w1, w2, z);
-  w1 = __funnelshift_l(w0, w1, z);
-  w1 |= __funnelshift_l(0u, w0, z) != 0 ? 1u : 0u;  // what is cut off stays visible
-  e -= z;
-  // to 53 bits, ties to even; a carry out of the top leaves 2^64
-  uint32_t c;
-  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, 0, 0;"
-      : "+r"(w1), "+r"(w2), "=r"(c)
-      : "r"(0x3FFu + ((w1 >> 11) & 1u)));
-  w2 |= c << 31;
-  e += (int)c;
-  const bool nz = w2 != 0;
-  rare = nz && (unsigned)(e - 1) >= 2046u;
-  // the leading bit adds the 1 that the exponent field is short of
-  const uint32_t hi = ((w2 >> 11) + ((uint32_t)(e - 1) << 20)) | (s & 0x80000000u);
-  return __hiloint2double(nz ? (int)hi : 0, (int)__funnelshift_r(w1, w2, 11));
+  const double h = __longlong_as_double(H + 0x4338000000000000ll);
+  const double l = __longlong_as_double(lo + 0x4338000000000000ll);
+  const double v = __fma_rn(__dadd_rn(h, -6755399442628608.0), 4294967296.0, l);
+  const int hi = __double2hiint(v);
+  const int ex = (hi >> 20) & 0x7FF;  // 0: the sum is zero
+  rare = ex != 0 && (unsigned)(ex + sh - 33) >= 2046u;
+  return __hiloint2double(ex ? hi + ((sh - 32) << 20) : 0, __double2loint(v));
 }
 
-template <int EPI, bool BETA, int PT>
+template <int EPI, bool LIN, int PT>
 __global__ void __launch_bounds__(SL_NT, 1)
     k_contract_sl(const __grid_constant__ SlLaunch L) {
   extern __shared__ uint8_t smem_raw[];
@@ -749,8 +725,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
                   v *= __ldg(f);
                 else if (EPI == JFG_EPI_DIV_EIG)
                   v = v / (c0 + c1 * (__ldg((const double*)d.lam_m + mm) + lp));
-                if (L.scaled) v *= d.alpha;
-                if (BETA) v += d.beta * *o;
+                if (LIN) {
+                  v *= d.alpha;
+                  if (d.beta != 0.0) v += d.beta * *o;
+                }
                 *o = v;
               }
               o += 4 * d.out_ld;
@@ -796,7 +774,7 @@ constexpr uint32_t RBLK = RM * 128;                // one digit of one unit
 constexpr uint32_t RUNIT = (NS + 1) * RBLK;        // zero block and digits
 constexpr size_t ROWS_SMEM = 1024 + NS * ABYTES + 2 * RUNIT + RING * RT * 4 + 64 * 4 + 16 * 8;
 
-template <int EPI, bool BETA>
+template <int EPI, bool LIN>
 __global__ void __launch_bounds__(SL_NT, 1)
     k_contract_sl_rows(const __grid_constant__ SlLaunch L) {
   extern __shared__ uint8_t smem_raw[];
@@ -1082,8 +1060,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
                 w *= __ldg(fm);
               else if (EPI == JFG_EPI_DIV_EIG)
                 w = w / (c0 + c1 * (__ldg((const double*)d.lam_m + m + c) + lp));
-              if (L.scaled) w *= d.alpha;
-              if (BETA) w += d.beta * *o;
+              if (LIN) {
+                w *= d.alpha;
+                if (d.beta != 0.0) w += d.beta * *o;
+              }
               *o = w;
             }
             o += d.out_ld;
@@ -1103,15 +1083,15 @@ __global__ void __launch_bounds__(SL_NT, 1)
   }
 }
 
-template <int EPI, bool BETA>
+template <int EPI, bool LIN>
 int set_attr() {
-  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl_rows<EPI, BETA>,
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl_rows<EPI, LIN>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)ROWS_SMEM));
-  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, BETA, 32>,
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, LIN, 32>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)SMEM_LIMIT - 1024));
-  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, BETA, 16>,
+  JFG_CUDA_TRY(cudaFuncSetAttribute(k_contract_sl<EPI, LIN, 16>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)SMEM_LIMIT - 1024));
   return JFG_OK;
@@ -1143,9 +1123,9 @@ inline int kp64(int K) { return (K + 63) / 64 * 64; }
 
 template <int PT>
 int launch(const SlLaunch& L, dim3 grid, size_t smem, cudaStream_t st) {
-  const bool beta = L.d.beta != 0.0;
+  const bool lin = L.d.alpha != 1.0 || L.d.beta != 0.0;
 #define JFG_SL(E)                                                        \
-  if (beta)                                                              \
+  if (lin)                                                               \
     k_contract_sl<E, true, PT><<<grid, SL_NT, smem, st>>>(L);            \
   else                                                                   \
     k_contract_sl<E, false, PT><<<grid, SL_NT, smem, st>>>(L)
@@ -1166,9 +1146,9 @@ int launch(const SlLaunch& L, dim3 grid, size_t smem, cudaStream_t st) {
 }
 
 int launch_rows(const SlLaunch& L, dim3 grid, cudaStream_t st) {
-  const bool beta = L.d.beta != 0.0;
+  const bool lin = L.d.alpha != 1.0 || L.d.beta != 0.0;
 #define JFG_SL(E)                                                            \
-  if (beta)                                                                  \
+  if (lin)                                                                   \
     k_contract_sl_rows<E, true><<<grid, SL_NT, ROWS_SMEM, st>>>(L);          \
   else                                                                       \
     k_contract_sl_rows<E, false><<<grid, SL_NT, ROWS_SMEM, st>>>(L)
@@ -1293,7 +1273,6 @@ int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, do
   if (L.astages < 2) return JFG_ERR_UNSUPPORTED;
   L.a_res = L.op_segs == 1 && L.mtiles * L.nkb * NS <= L.astages ? 1 : 0;
   L.vec2 = ((uintptr_t)in & 15) == 0 && !(d.in_ld & 1) && !(d.in_seg & 1) && !(d.in_batch & 1);
-  L.scaled = d.alpha != 1.0;
   const int Kp = kp8(d.K);
   const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)op.M, (cuuint64_t)(op.nseg * NS)};
   const cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * op.M};
