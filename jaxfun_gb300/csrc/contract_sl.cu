@@ -72,7 +72,7 @@ constexpr int NWE = 8;            // epilogue warps
 constexpr int SL_NT = 64 + 32 * (NWS + NWE);
 constexpr uint32_t ABYTES = 128 * 128;  // one operator stage: 128 rows x 64 FP16
 constexpr int A_MAX = 8;          // operator stages
-constexpr int STG_LD = 9;         // epilogue staging: 32 rows x 8 columns, padded
+constexpr int STG_LD = 5;         // epilogue staging: 32 rows x 4 columns, padded
 constexpr int RING = 8;           // input tiles whose row exponents are kept (a tile's are
                                   // read after its accumulators are handed back)
 constexpr int COL_MAX = 3 * 512;  // column exponents (segments x K padded to 64)
@@ -543,6 +543,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
     // quarter-warp store to different 16-byte columns of the swizzled rows
     const int cu = PT == 32 ? ((u >> 1) | ((u & 1) << 2))
                             : (((u & 3) << 1) | ((u >> 2) & 1) | (u & 8));
+    const int steps = (L.kpad + 8 * UPR - 1) / (8 * UPR);  // with any elements
     double x[STEPS][8];
     auto load = [&](unsigned t) {
       int mt0, pt, slot, s;
@@ -554,6 +555,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       const bool live = b >= 0 && p < d.P;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
+        if (i >= steps) break;
         const int k0 = 8 * (cu + UPR * i);
         if (live && k0 + 8 <= d.K) {
           if (L.vec2) {
@@ -586,6 +588,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       bool bad = false;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
+        if (i >= steps) break;
         const int k0 = 8 * (cu + UPR * i);
         if (k0 < L.kpad) {
           const uint4 c = *reinterpret_cast<const uint4*>(ce + k0);
@@ -608,6 +611,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       uint8_t* dst = bs + (uint32_t)bslot * bbytes + DBLK + row * 128;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
+        if (i >= steps) break;
         const int q = cu + UPR * i, k0 = 8 * q;
         if (k0 < L.kpad) {
           const uint4 c = *reinterpret_cast<const uint4*>(ce + k0);
@@ -640,8 +644,8 @@ __global__ void __launch_bounds__(SL_NT, 1)
     // ---------------- epilogue ----------------
     const int ew = warp - 2 - NWS;
     const int quarter = warp & 3, half = ew >> 2;
-    double* st8 = stg + ew * 32 * STG_LD;
-    const int sr = lane >> 3, sc = lane & 7;
+    double* st4 = stg + ew * 32 * STG_LD;
+    const int sr = lane >> 2, sc = lane & 3;
     int ring = 0;
     uint32_t unit = 0;
     bool ok = true;
@@ -673,7 +677,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
           if (lane == 0) tc::mbar_arrive(&dempty[db]);
           continue;
         }
-        // four columns of all levels at a time, staged for stores of eight
+        // four columns of all levels at a time, staged for stores of 32 bytes a row
 #pragma unroll 1
         for (int g = 0; g < PT / 8; ++g) {
           const int col4 = half * (PT / 2) + 4 * g;
@@ -688,7 +692,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
           }
           const int4 E4 = *reinterpret_cast<const int4*>(row_e + ring * PT + col4);
           const int Ep[4] = {E4.x, E4.y, E4.z, E4.w};
-          double* cell = st8 + lane * STG_LD + 4 * (g & 1);
+          double* cell = st4 + lane * STG_LD;
           unsigned rare = 0;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -707,20 +711,18 @@ __global__ void __launch_bounds__(SL_NT, 1)
                 cell[c] = plain_sum(a, L.in + ib + (long long)p * d.in_ld, d.K);
             }
           }
-          if (!(g & 1)) continue;
-          const int col0 = col4 - 4;
           __syncwarp();
-          const int p = pt * PT + col0 + sc;
+          const int p = pt * PT + col4 + sc;
           if (p < d.P && b >= 0) {
             const double lp = EPI == JFG_EPI_DIV_EIG ? __ldg((const double*)d.lam_p + p) : 0.0;
             double* o = outS + (long long)(m0 + sr) * d.out_ld + p;
             const double* f = (const double*)d.field + (long long)b * d.field_batch +
                               (long long)s * d.field_seg + (long long)(m0 + sr) * d.field_ld + p;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int mm = m0 + 4 * i + sr;
+            for (int i = 0; i < 4; ++i) {
+              const int mm = m0 + 8 * i + sr;
               if (mm < d.M) {
-                double v = st8[(4 * i + sr) * STG_LD + sc];
+                double v = st4[(8 * i + sr) * STG_LD + sc];
                 if (EPI == JFG_EPI_MUL_FIELD)
                   v *= __ldg(f);
                 else if (EPI == JFG_EPI_DIV_EIG)
@@ -731,8 +733,8 @@ __global__ void __launch_bounds__(SL_NT, 1)
                 }
                 *o = v;
               }
-              o += 4 * d.out_ld;
-              if (EPI == JFG_EPI_MUL_FIELD) f += 4 * d.field_ld;
+              o += 8 * d.out_ld;
+              if (EPI == JFG_EPI_MUL_FIELD) f += 8 * d.field_ld;
             }
           }
           __syncwarp();
@@ -835,13 +837,15 @@ __global__ void __launch_bounds__(SL_NT, 1)
   const unsigned R = (unsigned)nb * (unsigned)d.P;
   const unsigned per_seg = (R + RT - 1) / RT;
   const unsigned items = per_seg * (unsigned)d.nseg;
-  // row of an item: problem (-1: none), segment and p
-  auto locate = [&](unsigned t, int row, int& b, int& s, int& p) {
-    s = (int)(t / per_seg);
+  // row of an item: segment, problem slot and p
+  auto locate = [&](unsigned t, int row, int& s, unsigned& slot, unsigned& p) {
+    s = d.nseg > 1 ? (int)(t / per_seg) : 0;
     const unsigned r = (t - (unsigned)s * per_seg) * RT + (unsigned)row;
-    const unsigned slot = r / (unsigned)d.P;
-    p = (int)(r - slot * (unsigned)d.P);
-    b = r < R ? active_problem(d.batch_list, nb, d.batch, (int)slot) : -1;
+    slot = r / (unsigned)d.P;
+    p = r - slot * (unsigned)d.P;
+  };
+  auto problem = [&](unsigned slot) {  // -1: past the last
+    return active_problem(d.batch_list, nb, d.batch, (int)slot);
   };
 
   if (warp == 0) {
@@ -914,12 +918,15 @@ __global__ void __launch_bounds__(SL_NT, 1)
     const int row0 = 4 * (warp - 2) + (lane & 3);
     const uint4 ce = __ldg((const uint4*)(L.col_e + k0));
     uint8_t* dst = as + row0 * 128 + ((cu ^ (row0 & 7)) << 4);
+    const unsigned q32 = 32u / (unsigned)d.P, r32 = 32u - q32 * (unsigned)d.P;  // 32 rows on
     double x[4][8];
     auto load = [&](unsigned t) {
+      int s;
+      unsigned slot, p;
+      locate(t, row0, s, slot, p);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        int b, s, p;
-        locate(t, 32 * i + row0, b, s, p);
+        const int b = problem(slot);
         const double* src = L.in + (long long)(b < 0 ? 0 : b) * d.in_batch +
                             (long long)s * d.in_seg + (long long)p * d.in_ld + k0;
         if (b >= 0 && k0 + 8 <= d.K) {
@@ -937,6 +944,12 @@ __global__ void __launch_bounds__(SL_NT, 1)
         } else {
 #pragma unroll
           for (int e = 0; e < 8; ++e) x[i][e] = b >= 0 && k0 + e < d.K ? __ldg(src + e) : 0.0;
+        }
+        slot += q32;
+        p += r32;
+        if (p >= (unsigned)d.P) {
+          p -= (unsigned)d.P;
+          ++slot;
         }
       }
     };
@@ -988,8 +1001,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
     uint32_t unit = 0, n = 0;
     bool ok = true;
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x, ++n) {
-      int b, s, p;
-      locate(t, row, b, s, p);
+      int s;
+      unsigned slot, up;
+      locate(t, row, s, slot, up);
+      const int b = problem(slot), p = (int)up;
       const long long ib = (long long)(b < 0 ? 0 : b);
       double* outP = L.out + ib * d.out_batch + (long long)s * d.out_seg + p;
       const double* f = (const double*)d.field + ib * d.field_batch + (long long)s * d.field_seg + p;
