@@ -12,111 +12,201 @@ namespace {
 
 constexpr int MAXC = 64;  // channel width limit of the mode-mixing kernels
 
-// out[b][co][q] = sum_ci R[q][co][ci] x[b][q][ci]
+// Per-mode channel mixing.  Forward: out[b][co][q] = sum_ci R[q][co][ci] x[b][q][ci].
+// Backward: dx[b][ci][q] = sum_co R[q][co][ci] dy[b][q][co] and
+// dR[q][co][ci] = sum_b dy[b][q][co] x[b][q][ci].  Sums run in ascending order.
 //
-// A block owns MM_Q consecutive modes and a slice of the samples; thread
-// (co, ql) keeps the row R[q0+ql][co][:] in registers for the whole slice.
-// Per sample the block stages x[b][q0 .. q0+MM_Q)[:] (contiguous, one float
-// per thread) in shared memory, double-buffered so one barrier per sample
-// suffices, and the MM_Q threads of one output channel write MM_Q
-// consecutive modes (16 bytes).  The number of modes must be a multiple of
-// MM_Q (checked by the launcher).
-constexpr int MM_Q = 8;
+// A block owns MB neighbouring modes and works through (32 samples, mode)
+// steps: the mode's R and the samples' rows are copied to shared memory one
+// step ahead (cp.async), 256 threads hold 2 x 4 (sample, channel) and 4 x 4
+// (dR) register tiles, and bf16 results of the MB modes are gathered in shared
+// memory so that each (sample, channel) gets MB modes in one store.  Bound by
+// shared-memory reads, about 10 wavefronts per 32 FMA instructions.  32 samples,
+// 1024 modes, 64 channels: forward 78 -> 21 us, backward 108 -> 32 us against
+// one mode (forward: eight) at a time with a barrier or two per sample.
+constexpr int MM_B = 32;             // samples per step
+constexpr int MM_T = 256;
+constexpr int MM_LD = MAXC + 4;      // 16-byte rows, neighbouring rows 4 banks apart
+constexpr int MM_Q = 8;              // the forward call takes multiples of this
 
-constexpr int MM_LD = MAXC + 4;  // 16-byte rows; the MM_Q rows of a warp's float4 reads hit distinct banks
+struct MixStage {
+  float R[MAXC][MM_LD];
+  float x[MM_B][MM_LD];
+  float d[MM_B][MM_LD];
+};
+template <int MB>
+struct MixSmem {
+  MixStage st[2];
+  __nv_bfloat16 o[MM_B * MAXC][MB];
+};
 
-__global__ void __launch_bounds__(MM_Q * MAXC) k_modemix_fwd(
-    int batch, int nq, int C, int per_block, const float* __restrict__ R,
-    const float* __restrict__ x, __nv_bfloat16* __restrict__ out) {
-  __shared__ __align__(16) float xs[2][MM_Q][MM_LD];
-  const int t = threadIdx.x;
-  // channels ci >= C stay zero (their R entries are zero too)
-  for (int i = t; i < 2 * MM_Q * MM_LD; i += blockDim.x) (&xs[0][0][0])[i] = 0.f;
-  __syncthreads();
-  const int ql = t % MM_Q;
-  const int co = t / MM_Q;
-  const int q0 = blockIdx.x * MM_Q;
-  const int b0 = blockIdx.y * per_block;
-  const int b1 = min(batch, b0 + per_block);
-  const bool active = co < C;
-  float r[MAXC];
-  const float* Rrow = R + ((long long)(q0 + ql) * C + (active ? co : 0)) * C;
-#pragma unroll
-  for (int ci = 0; ci < MAXC; ++ci) r[ci] = (active && ci < C) ? __ldg(Rrow + ci) : 0.f;
-  const int nload = MM_Q * C;
-  // each thread's element of the next PF samples is loaded ahead, so the
-  // loop over samples does not wait on a load every iteration
-  constexpr int PF = 4;
-  float nxt[PF];
-#pragma unroll
-  for (int u = 0; u < PF; ++u)
-    nxt[u] = (t < nload && b0 + u < b1) ? x[((long long)(b0 + u) * nq + q0) * C + t] : 0.f;
-  for (int b = b0; b < b1; ++b) {
-    float (*xb)[MM_LD] = xs[b & 1];
-    if (t < nload) xb[t / C][t % C] = nxt[0];
-#pragma unroll
-    for (int u = 0; u + 1 < PF; ++u) nxt[u] = nxt[u + 1];
-    nxt[PF - 1] =
-        (t < nload && b + PF < b1) ? x[((long long)(b + PF) * nq + q0) * C + t] : 0.f;
-    __syncthreads();
-    if (active) {
-      const float4* xv = reinterpret_cast<const float4*>(xb[ql]);
-      float s = 0.f;
-#pragma unroll
-      for (int c4 = 0; c4 < MAXC / 4; ++c4) {
-        const float4 v = xv[c4];
-        s = fmaf(r[4 * c4], v.x, s);
-        s = fmaf(r[4 * c4 + 1], v.y, s);
-        s = fmaf(r[4 * c4 + 2], v.z, s);
-        s = fmaf(r[4 * c4 + 3], v.w, s);
-      }
-      out[((long long)b * C + co) * nq + q0 + ql] = __float2bfloat16(s);
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+// rows of C floats at src + r * ld into dst[r][0..C)
+__device__ __forceinline__ void mix_copy(float (*dst)[MM_LD], const float* src, long long ld,
+                                         int rows, int C, bool vec) {
+  if (vec) {
+    const int c4 = C / 4;
+    for (int i = threadIdx.x; i < rows * c4; i += MM_T) {
+      const int r = i / c4, c = (i - r * c4) * 4;
+      cp16(&dst[r][c], src + r * ld + c);
+    }
+  } else {
+    for (int i = threadIdx.x; i < rows * C; i += MM_T) {
+      const int r = i / C, c = i - r * C;
+      dst[r][c] = src[r * ld + c];
     }
   }
 }
 
-// dx[b][ci][q] = sum_co R[q][co][ci] dy[b][q][co];  dR[q][co][ci] = sum_b dy[b][q][co] x[b][q][ci]
-__global__ void k_modemix_bwd(int batch, int nq, int C, const float* __restrict__ R,
-                              const float* __restrict__ x, const float* __restrict__ dy,
-                              __nv_bfloat16* __restrict__ dx, float* __restrict__ dR) {
-  __shared__ float Rs[MAXC * (MAXC + 1)];
-  __shared__ float xs[MAXC], ds[MAXC];
-  const int q = blockIdx.x;
+template <int MB, bool BWD>
+__global__ void __launch_bounds__(MM_T, 2)
+    k_modemix(int batch, int nq, int C, int per_block, int vec, int wide,
+              const float* __restrict__ R,
+              const float* __restrict__ x, const float* __restrict__ dy,
+              __nv_bfloat16* __restrict__ out, float* __restrict__ dR) {
+  extern __shared__ __align__(16) uint8_t mix_smem[];
+  MixSmem<MB>& sm = *reinterpret_cast<MixSmem<MB>*>(mix_smem);
   const int t = threadIdx.x;
-  for (int i = t; i < C * C; i += blockDim.x) Rs[(i / C) * (C + 1) + i % C] = R[(long long)q * C * C + i];
-  float acc[MAXC / 2];  // dR row co = t, columns [0, C): two halves processed in turn
-  for (int half = 0; half < 2; ++half) {
-    const int c0 = half * (C / 2 > 0 ? (C + 1) / 2 : C);
-    const int cn = half == 0 ? (C + 1) / 2 : C - (C + 1) / 2;
-#pragma unroll 4
-    for (int j = 0; j < MAXC / 2; ++j) acc[j] = 0.f;
-    __syncthreads();
-    for (int b = 0; b < batch; ++b) {
-      if (t < C) {
-        xs[t] = x[((long long)b * nq + q) * C + t];
-        ds[t] = dy[((long long)b * nq + q) * C + t];
-      }
-      __syncthreads();
-      if (t < C) {
-        const float dyt = ds[t];
+  const int q0 = blockIdx.x * MB;
+  const int b0 = blockIdx.y * per_block, b1 = min(batch, b0 + per_block);
+  const int nm = min(MB, nq - q0);
+  const int steps = (b1 - b0 + MM_B - 1) / MM_B * nm;  // (samples, mode), modes inside
+  // channels past C are zero
+  for (int i = t; i < (int)(sizeof(sm.st) / 16); i += MM_T)
+    reinterpret_cast<float4*>(&sm.st[0])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  auto fetch = [&](int step) {
+    MixStage& s = sm.st[step & 1];
+    const int b = b0 + step / nm * MM_B, q = q0 + step % nm;
+    const int n = min(MM_B, b1 - b);
+    mix_copy(s.R, R + (long long)q * C * C, C, C, C, vec);
+    mix_copy(s.x, x + ((long long)b * nq + q) * C, (long long)nq * C, n, C, vec);
+    if (BWD) mix_copy(s.d, dy + ((long long)b * nq + q) * C, (long long)nq * C, n, C, vec);
+  };
+  float acc[BWD ? MB : 1][4][4];
 #pragma unroll
-        for (int j = 0; j < MAXC / 2; ++j)
-          if (j < cn) acc[j] += dyt * xs[c0 + j];
-        if (half == 0) {
-          float s = 0.f;
-          for (int co = 0; co < C; ++co) s += Rs[co * (C + 1) + t] * ds[co];
-          dx[((long long)b * C + t) * nq + q] = __float2bfloat16(s);
+  for (int m = 0; m < (BWD ? MB : 1); ++m)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[m][i / 4][i % 4] = 0.f;
+  const int lo = t & 15, hi = t >> 4;
+  if (steps > 0) fetch(0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int bb = b0, step = 0; bb < b1; bb += MM_B) {
+    const int n = min(MM_B, b1 - bb);
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      if (m >= nm) break;
+      if (step + 1 < steps) fetch(step + 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      const MixStage& s = sm.st[step & 1];
+      ++step;
+      // samples 2 hi, 2 hi + 1; channels 4 lo + j (backward), lo + 16 j (forward:
+      // rows of R that lie in different banks)
+      float v[2][4] = {};
+      const float(*in)[MM_LD] = BWD ? s.d : s.x;
+#pragma unroll 4
+      for (int c = 0; c < MAXC; c += 4) {
+        if (c >= C) break;
+        float y[2][4], r[4][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          *reinterpret_cast<float4*>(y[u]) = *reinterpret_cast<const float4*>(&in[2 * hi + u][c]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<float4*>(r[j]) = *reinterpret_cast<const float4*>(
+              BWD ? &s.R[c + j][4 * lo] : &s.R[lo + 16 * j][c]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[u][j] = fmaf(BWD ? r[k][j] : r[j][k], y[u][k], v[u][j]);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          sm.o[(2 * hi + u) * MAXC + (BWD ? 4 * lo + j : lo + 16 * j)][m] = __float2bfloat16(v[u][j]);
+      if (BWD) {
+#pragma unroll 4
+        for (int b = 0; b < n; ++b) {
+          float xv[4], dv[4];
+          *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(&s.x[b][4 * lo]);
+          *reinterpret_cast<float4*>(dv) = *reinterpret_cast<const float4*>(&s.d[b][4 * hi]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[m][i][j] = fmaf(dv[i], xv[j], acc[m][i][j]);
         }
       }
-      __syncthreads();
+      __syncthreads();  // the stage may be filled again
     }
-    if (t < C) {
+    // MB modes of every (sample, channel); the next results come after a barrier
+    for (int i = t; i < n * C; i += MM_T) {
+      const int b = i / C, c = i - b * C;
+      const __nv_bfloat16* o = sm.o[b * MAXC + c];
+      __nv_bfloat16* g = out + ((long long)(bb + b) * C + c) * nq + q0;
+      if (MB == 4 && wide)
+        *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(o);
+      else
+        for (int m = 0; m < nm; ++m) g[m] = o[m];
+    }
+  }
+  if (BWD) {
 #pragma unroll
-      for (int j = 0; j < MAXC / 2; ++j)
-        if (j < cn) dR[((long long)q * C + t) * C + c0 + j] = acc[j];
+    for (int m = 0; m < MB; ++m) {
+      if (m >= nm) break;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int co = 4 * hi + i;
+        if (co >= C) continue;
+        float* g = dR + ((long long)(q0 + m) * C + co) * C + 4 * lo;
+        if (vec) {
+          if (4 * lo < C)
+            *reinterpret_cast<float4*>(g) =
+                make_float4(acc[m][i][0], acc[m][i][1], acc[m][i][2], acc[m][i][3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (4 * lo + j < C) g[j] = acc[m][i][j];
+        }
+      }
     }
   }
 }
+
+template <int MB, bool BWD>
+int mix_launch(int groups, int per_block, int batch, int nq, int C, const float* R, const float* x,
+               const float* dy, void* out, float* dR, cudaStream_t st) {
+  static bool set[64] = {};  // per device; call before a capture
+  int dev = 0;
+  JFG_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
+  if (!set[dev]) {
+    JFG_CUDA_TRY(cudaFuncSetAttribute(k_modemix<MB, BWD>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(MixSmem<MB>)));
+    set[dev] = true;
+  }
+  // copies of 16 bytes; stores of MB modes at once
+  const int vec = C % 4 == 0 && (((uintptr_t)R | (uintptr_t)x | (uintptr_t)dy | (uintptr_t)dR) & 15) == 0;
+  const int wide = nq % MB == 0 && ((uintptr_t)out & 7) == 0;
+  k_modemix<MB, BWD><<<dim3((nq + MB - 1) / MB, groups), MM_T, sizeof(MixSmem<MB>), st>>>(
+      batch, nq, C, per_block, vec, wide, R, x, dy, (__nv_bfloat16*)out, dR);
+  JFG_LAUNCHED();
+  return JFG_OK;
+}
+
+// Four modes a block (8-byte stores), one where that would leave SMs idle.
+constexpr int MM_FEW = 512;
 
 __global__ void k_colsum_bf16(long long rows, int n, const __nv_bfloat16* __restrict__ src,
                               float* __restrict__ out, long long rows_per_block) {
@@ -196,16 +286,13 @@ extern "C" int jfg_sno_modemix_fwd(int batch, int nmodes, int C, const float* R,
   if (batch < 0 || nmodes < 0 || C < 1 || C > MAXC || !R || !x || !out) return JFG_ERR_ARG;
   if (batch == 0 || nmodes == 0) return JFG_OK;
   if (nmodes % MM_Q != 0) return JFG_ERR_ARG;
-  // enough blocks for every SM, at least 8 samples per block
-  const int mblocks = nmodes / MM_Q;
-  int groups = (2 * 152 + mblocks - 1) / mblocks;
-  groups = std::max(1, std::min(groups, (batch + 7) / 8));
+  // samples spread over the blocks' second index where modes are few
+  const int mblocks = nmodes >= MM_FEW ? nmodes / 4 : nmodes;
+  const int groups = std::max(1, std::min((2 * 152 + mblocks - 1) / mblocks, (batch + MM_B - 1) / MM_B));
   const int per_block = (batch + groups - 1) / groups;
-  groups = (batch + per_block - 1) / per_block;
-  k_modemix_fwd<<<dim3(mblocks, groups), MM_Q * MAXC, 0, (cudaStream_t)stream>>>(
-      batch, nmodes, C, per_block, R, x, (__nv_bfloat16*)out);
-  JFG_LAUNCHED();
-  return JFG_OK;
+  auto* f = nmodes >= MM_FEW ? mix_launch<4, false> : mix_launch<1, false>;
+  return f((batch + per_block - 1) / per_block, per_block, batch, nmodes, C, R, x, nullptr, out,
+           nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int jfg_sno_modemix_bwd(int batch, int nmodes, int C, const float* R, const float* x,
@@ -213,10 +300,8 @@ extern "C" int jfg_sno_modemix_bwd(int batch, int nmodes, int C, const float* R,
   if (batch < 0 || nmodes < 0 || C < 1 || C > MAXC || !R || !x || !dy || !dx || !dR)
     return JFG_ERR_ARG;
   if (nmodes == 0) return JFG_OK;
-  k_modemix_bwd<<<nmodes, ((C + 31) / 32) * 32, 0, (cudaStream_t)stream>>>(
-      batch, nmodes, C, R, x, dy, (__nv_bfloat16*)dx, dR);
-  JFG_LAUNCHED();
-  return JFG_OK;
+  auto* f = nmodes >= MM_FEW ? mix_launch<4, true> : mix_launch<1, true>;
+  return f(1, batch, batch, nmodes, C, R, x, dy, dx, dR, (cudaStream_t)stream);
 }
 
 extern "C" int jfg_colsum_bf16(long long rows, int n, const void* src, float* out,
