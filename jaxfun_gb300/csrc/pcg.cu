@@ -107,6 +107,30 @@ __device__ __forceinline__ T sum_part(const T* part, int b, int nb) {
   return s;
 }
 
+// The sums of one problem's NSETS sets of partials for a block: the partials
+// are loaded by all threads at once and added from shared memory by one thread
+// per set, in sum_part's order.  One thread loading them in turn waited for L2
+// every few partials, up to 128 of them per launch: 8 FP64 solves of 128^2
+// 17.97 -> 17.82 ms, 128 mixed ones of 256^2 41.00 -> 40.74 ms.
+template <int NSETS, typename T>
+__device__ __forceinline__ void block_parts(const T* const (&part)[NSETS], const int (&nb)[NSETS],
+                                            int b, T (&sum)[NSETS]) {
+  __shared__ T s_part[NSETS][PS];
+#pragma unroll
+  for (int i = 0; i < NSETS; ++i)
+    for (int j = threadIdx.x; j < nb[i]; j += blockDim.x) s_part[i][j] = part[i][b * PS + j];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NSETS; ++i)
+    if (threadIdx.x == 32 * i) {
+      T s = T(0);
+#pragma unroll 8
+      for (int j = 0; j < nb[i]; ++j) s += s_part[i][j];
+      sum[i] = s;
+    }
+  __syncthreads();
+}
+
 template <typename T>
 __device__ __forceinline__ bool is_active(T rz, T rz0, double tol) {
   return rz0 > T(0) && rz > T(0) && (double)rz > tol * tol * (double)rz0;
@@ -163,14 +187,15 @@ __global__ void k_update_r(T* __restrict__ r, const T* __restrict__ q, long long
                            const T* __restrict__ rz0, const double* __restrict__ tolp,
                            const int* __restrict__ list, const int* count, int batch,
                            unsigned* __restrict__ slots, int nb_pq, int nb_rz) {
-  __shared__ T s_alpha;
+  __shared__ T s_alpha, s_sum[2];
   __shared__ int s_act;
   const int b = active_problem(list, active_count(list, count, batch), batch, blockIdx.y);
   if (b < 0) return;
+  block_parts<2, T>({rz_prev, pq_part}, {nb_rz, nb_pq}, b, s_sum);
   if (threadIdx.x == 0) {
-    const T rz = sum_part(rz_prev, b, nb_rz);
+    const T rz = s_sum[0];
     s_act = is_active(rz, rz0[b], tolp[b]) ? 1 : 0;
-    s_alpha = s_act ? rz / sum_part(pq_part, b, nb_pq) : T(0);
+    s_alpha = s_act ? rz / s_sum[1] : T(0);
     if (s_act && slots && blockIdx.x == 0)
       for (int k = 0; k < H16_SLOTS; ++k) slots[(long long)k * batch + b] = 0u;
   }
@@ -203,17 +228,18 @@ __global__ void k_update_xp(T* __restrict__ x, T* __restrict__ p, const T* __res
                             const int* count, int batch, unsigned* __restrict__ pmax, int nb_pq,
                             int nb_rz, int* __restrict__ inner_it, int maxit,
                             int* __restrict__ keep) {
-  __shared__ T s_alpha, s_beta;
+  __shared__ T s_alpha, s_beta, s_sum[3];
   __shared__ int s_act;
   const int b = active_problem(list, active_count(list, count, batch), batch, blockIdx.y);
   if (b < 0) return;
+  block_parts<3, T>({rz_prev_part, rz_new_part, pq_part}, {nb_rz, nb_rz, nb_pq}, b, s_sum);
   if (threadIdx.x == 0) {
-    const T rzp = sum_part(rz_prev_part, b, nb_rz);
+    const T rzp = s_sum[0];
     s_act = is_active(rzp, rz0[b], tolp[b]) ? 1 : 0;
     int kp = 0;
     if (s_act) {
-      const T rzn = sum_part(rz_new_part, b, nb_rz);
-      s_alpha = rzp / sum_part(pq_part, b, nb_pq);
+      const T rzn = s_sum[1];
+      s_alpha = rzp / s_sum[2];
       s_beta = rzn / rzp;
       // whether the problem stays in the active list (read by k_compact)
       kp = is_active(rzn, rz0[b], tolp[b]) ? 1 : 0;
