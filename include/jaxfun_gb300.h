@@ -294,7 +294,8 @@ size_t jfg_tp_apply_workspace_size(int ndim, const int* rows, const int* cols, i
 int jfg_tp_apply_f64(int ndim, const int* rows, const int* cols, int batch,
                      const double* const* mats, const double* in, double* out,
                      void* work, size_t work_bytes, void* stream);
-/* FP64 data in double-FP32 arithmetic (jfg_contract_df64 per pass, about
+/* FP64 data: passes large enough for it as jfg_tp_apply_f64 runs them on the
+ * tensor cores, else double-FP32 arithmetic (jfg_contract_df64 per pass, about
  * 1e-14 relative per contraction, ~3x the FP64 pipe's rate on GB300): for
  * FP64-class right-hand sides, e.g. the scalar product of a forcing. */
 int jfg_tp_apply_df64(int ndim, const int* rows, const int* cols, int batch,
@@ -563,7 +564,8 @@ typedef struct {
   const float* ops32;    /* packed padded operators rounded to FP32, or NULL: used for
                             r -= ||r|| A d once ||r|| <= 1e-4 ||rhs|| (else FP64 r = b - A x) */
   int residual;          /* arithmetic of r = b - A x: 0 FP64 (DFMA), 1 double-FP32
-                            (jfg_contract_df64 passes)                                */
+                            (jfg_contract_df64 passes); large 2-D batches take FP64 on
+                            the tensor cores with either                              */
   int precond_bf16;      /* 1: the inner preconditioner's FD passes use split-BF16
                             operators (E/W_hi16, _lo16: jfg_split_bf16_host of the
                             padded factors), 2: plain BF16 (E/W_hi16 only; the

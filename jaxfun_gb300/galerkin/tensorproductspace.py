@@ -294,7 +294,8 @@ class TensorProductSpace:
         return W
 
     # ---- transforms (tensorproductspace.py:330-417) -------------------------
-    # precision: "f64" (FP64 CUDA cores, parity path), "df64" (FP64 data,
+    # precision: "f64" (FP64, parity path: the tensor cores' exact digit products
+    # or FP64 FMAs, by size), "df64" (FP64 data, the same for large passes, else
     # double-FP32 arithmetic on the FP32 pipe, ~1e-14), "bf16x3" (FP32 data,
     # split-BF16 operators, three BF16 MMAs per product) or "tc" (FP32 data,
     # split-TF32 tcgen05 contractions)

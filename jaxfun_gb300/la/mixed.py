@@ -86,7 +86,8 @@ class MixedVarCoefSolver:
                  precond: str | None = None, apply: str | None = None, fused_dots: bool = True,
                  schedule: str = "sync"):
         """``residual``: arithmetic of the refinement residual r = b - A x,
-        "df64" (double-FP32 on the FP32 units) or "f64" (FP64 FMAs).
+        "df64" (double-FP32 on the FP32 units) or "f64" (FP64 FMAs); large
+        2-D batches take FP64 on the tensor cores with either.
         ``fp32_updates``: once ||r|| <= 1e-4 ||b||, update r -= ||r|| A d in FP32
         instead of recomputing it (default: in 2-D only; in 3-D the operator's
         conditioning turns the FP32 update error into > 1e-10 solution error).
