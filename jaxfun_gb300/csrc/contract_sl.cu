@@ -269,6 +269,12 @@ __device__ __forceinline__ void commit_if(uint64_t* bar, uint32_t leader) {
       : "memory");
 }
 
+// The wait of a whole warp: one answer for all lanes, which are converged after
+// it, as the aligned TMEM instructions and the issuers' uniform walk need.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_sl_status)) != 0;
+}
+
 __device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -454,9 +460,6 @@ __global__ void __launch_bounds__(SL_NT, 1)
     // on a warp-uniform value (waits through a vote): otherwise the addresses
     // leave the uniform registers and an MMA costs 64 clocks instead of 40 (4 x
     // 256^3 round: 4.34 ms then, 3.56 ms so; 32 x 256^2: 139 and 122 us).
-    auto wait = [&](uint64_t* bar, uint32_t parity) {
-      return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_sl_status)) != 0;
-    };
     const uint32_t ad0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(as));
     const uint32_t bd0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(bs));
     const uint32_t dhi = (uint32_t)(tc::sdesc_sw128(0) >> 32);
@@ -467,14 +470,14 @@ __global__ void __launch_bounds__(SL_NT, 1)
     uint32_t aph = 0, bph = 0, unit = 0;
     bool ok = true, any = false;
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
-      if (!wait(&bfull[bslot], bph)) {
+      if (!warp_wait(&bfull[bslot], bph)) {
         ok = false;
         break;
       }
       const uint32_t bdt = bd0 + (((uint32_t)bslot * bbytes) >> 4);
       for (int mi = 0; ok && mi < mt_n; ++mi, ++unit) {
         const uint32_t db = unit & 1u;
-        if (unit >= 2 && !wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
+        if (unit >= 2 && !warp_wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
           ok = false;
           break;
         }
@@ -487,7 +490,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
           const uint32_t bdk = bdt + (((uint32_t)kb * KBLK) >> 4);
 #pragma unroll
           for (int i = 0; i < NS; ++i) {
-            if (!wait(&afull[st], aph)) {
+            if (!warp_wait(&afull[st], aph)) {
               ok = false;
               break;
             }
@@ -606,7 +609,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       }
       if (E < -(1 << 18)) E = 0;
       if (bad) E = SPECIAL;
-      if (n >= (unsigned)L.bbuf && !tc::mbar_wait(&bempty[bslot], bph ^ 1u, &g_sl_status)) break;
+      if (n >= (unsigned)L.bbuf && !warp_wait(&bempty[bslot], bph ^ 1u)) break;
       if (u == 0) row_e[ring * PT + row] = E;
       uint8_t* dst = bs + (uint32_t)bslot * bbytes + DBLK + row * 128;
 #pragma unroll
@@ -666,7 +669,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
         const int m = m0 + lane;
         const int Ea = m < d.M ? __ldg(L.row_e + (long long)os * L.row_ld + m) : 0;
         const uint32_t db = unit & 1u;
-        if (!tc::mbar_wait(&dfull[db], (unit >> 1) & 1u, &g_sl_status)) {
+        if (!warp_wait(&dfull[db], (unit >> 1) & 1u)) {
           ok = false;
           break;
         }
@@ -853,9 +856,6 @@ __global__ void __launch_bounds__(SL_NT, 1)
     if (lane == 0) tc::mbar_wait(ofull, 0, &g_sl_status);
   } else if (warp == 1) {
     // ---------------- MMA issuer (uniform walk as above) ----------------
-    auto wait = [&](uint64_t* bar, uint32_t parity) {
-      return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_sl_status)) != 0;
-    };
     const uint32_t ad0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(as));
     const uint32_t bd0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(bs));
     const uint32_t dhi = (uint32_t)(tc::sdesc_sw128(0) >> 32);
@@ -865,12 +865,12 @@ __global__ void __launch_bounds__(SL_NT, 1)
     const int n16 = (d.K + 15) / 16;
     uint32_t unit = 0, ph = 0;
     bool any = false;
-    bool ok = blockIdx.x >= items || wait(ofull, 0);
+    bool ok = blockIdx.x >= items || warp_wait(ofull, 0);
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x, ph ^= 1u) {
-      if (!wait(bfull, ph)) break;
+      if (!warp_wait(bfull, ph)) break;
       for (int v = 0; v < units; ++v, ++unit) {
         const uint32_t db = unit & 1u;
-        if (unit >= 2 && !wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
+        if (unit >= 2 && !warp_wait(&dempty[db], ((unit >> 1) & 1u) ^ 1u)) {
           ok = false;
           break;
         }
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       for (int o = 4; o < 32; o <<= 1)
 #pragma unroll
         for (int i = 0; i < 4; ++i) E[i] = max(E[i], __shfl_xor_sync(0xffffffffu, E[i], o));
-      if (n >= 1 && !tc::mbar_wait(bempty, (n & 1u) ^ 1u, &g_sl_status)) break;
+      if (n >= 1 && !warp_wait(bempty, (n & 1u) ^ 1u)) break;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (E[i] < -(1 << 18)) E[i] = 0;
@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       int Ep = 0;
       for (int v = 0; v < units; ++v, ++unit) {
         const uint32_t db = unit & 1u;
-        if (!tc::mbar_wait(&dfull[db], (unit >> 1) & 1u, &g_sl_status)) {
+        if (!warp_wait(&dfull[db], (unit >> 1) & 1u)) {
           ok = false;
           break;
         }
@@ -1057,33 +1057,36 @@ __global__ void __launch_bounds__(SL_NT, 1)
                                  Ea[c] + Ep - 2080, xr);
             rare |= (xr || Ea[c] + Ep >= BIG) ? 1u << c : 0u;
           }
-          if (b < 0) continue;
-          if (rare) {
-            const double* y = L.in + ib * d.in_batch + (long long)s * d.in_seg + (long long)p * d.in_ld;
+          if (b >= 0) {
+            if (rare) {
+              const double* y =
+                  L.in + ib * d.in_batch + (long long)s * d.in_seg + (long long)p * d.in_ld;
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if ((rare >> c & 1u) && m + c < d.M)
-                val[c] = plain_sum(L.op + (long long)(m + c) * d.op_ld, y, d.K);
-          }
-          double* o = outP + (long long)m * d.out_ld;
-          const double* fm = f + (long long)m * d.field_ld;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (m + c < d.M) {
-              double w = val[c];
-              if (EPI == JFG_EPI_MUL_FIELD)
-                w *= __ldg(fm);
-              else if (EPI == JFG_EPI_DIV_EIG)
-                w = w / (c0 + c1 * (__ldg((const double*)d.lam_m + m + c) + lp));
-              if (LIN) {
-                w *= d.alpha;
-                if (d.beta != 0.0) w += d.beta * *o;
-              }
-              *o = w;
+              for (int c = 0; c < 4; ++c)
+                if ((rare >> c & 1u) && m + c < d.M)
+                  val[c] = plain_sum(L.op + (long long)(m + c) * d.op_ld, y, d.K);
             }
-            o += d.out_ld;
-            if (EPI == JFG_EPI_MUL_FIELD) fm += d.field_ld;
+            double* o = outP + (long long)m * d.out_ld;
+            const double* fm = f + (long long)m * d.field_ld;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (m + c < d.M) {
+                double w = val[c];
+                if (EPI == JFG_EPI_MUL_FIELD)
+                  w *= __ldg(fm);
+                else if (EPI == JFG_EPI_DIV_EIG)
+                  w = w / (c0 + c1 * (__ldg((const double*)d.lam_m + m + c) + lp));
+                if (LIN) {
+                  w *= d.alpha;
+                  if (d.beta != 0.0) w += d.beta * *o;
+                }
+                *o = w;
+              }
+              o += d.out_ld;
+              if (EPI == JFG_EPI_MUL_FIELD) fm += d.field_ld;
+            }
           }
+          __syncwarp();  // the next step's TMEM loads take the whole warp
         }
       }
     }

@@ -534,6 +534,11 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
   auto wait_done = [&](long long n) {
     return n < 0 || mbar_wait(&kdone[n % S_MAX], (uint32_t)(n / S_MAX) & 1u, budget);
   };
+  // the wait of a whole warp: one answer for all lanes, which are converged
+  // after it, as the aligned TMEM instructions need
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget)) != 0;
+  };
   // tile li of this CTA (false past the last one)
   auto tile_of = [&](long long li, int& gi, int& pt, int& mc, int& b, int& s,
                      bool need_b = true) -> bool {
@@ -639,9 +644,6 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
     // tensor pipe's 64 (measured alone).  Same MMAs in the same order.
     // Every branch is on a warp-uniform value (waits through a vote), or the
     // addresses would leave the uniform registers.
-    auto wait = [&](uint64_t* bar, uint32_t parity) {
-      return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget)) != 0;
-    };
     int li = 0;
     bool ok = true, issued_any = false;
     const uint64_t od0 = sdesc(smem_u32(obase));
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
       const int nko = __shfl_sync(0xffffffffu, nkx_of(gi) / KXO, 0);
       const int buf = li & 1;
       const uint32_t use = (uint32_t)(li >> 1);
-      if (li >= 2 && !wait(&tempty[buf], (use & 1u) ^ 1u)) {
+      if (li >= 2 && !warp_wait(&tempty[buf], (use & 1u) ^ 1u)) {
         ok = false;
         break;
       }
@@ -667,8 +669,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
       const uint32_t acc = tmem + (uint32_t)buf * acc_stride;
       if (res) so = 0;
       for (int ko = 0; ko < nko; ++ko) {
-        if (!wait(&ofull[so], res ? 0u : oph) ||
-            !wait(&conv[sl], aph)) {
+        if (!warp_wait(&ofull[so], res ? 0u : oph) || !warp_wait(&conv[sl], aph)) {
           ok = false;
           break;
         }
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
           if (kx % KXO == KXO - 1) ++kn;
           continue;
         }
-        if (!mbar_wait(&xfull[st], ph, budget)) {
+        if (!warp_wait(&xfull[st], ph)) {
           ok = false;
           break;
         }
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
               }
             }
           }
-          if (kx % KXO == 0 && !wait_done(kn - SA / KXO)) {
+          if (kx % KXO == 0 && !__all_sync(0xffffffffu, wait_done(kn - SA / KXO))) {
             ok = false;
             break;
           }
@@ -928,7 +929,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
       };
       float f[16], fn[16];
       if (EPI == JFG_EPI_MUL_FIELD && cb_of(0) < ncb) load_field(cb_of(0), f);
-      if (!mbar_wait(&tfull[buf], (uint32_t)(li >> 1) & 1u, budget)) break;
+      if (!warp_wait(&tfull[buf], (uint32_t)(li >> 1) & 1u)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)buf * acc_stride;
 #pragma unroll 1
@@ -980,6 +981,7 @@ __global__ void __launch_bounds__(nthreads(EPI, BETA, PREC), 1)
 #pragma unroll
           for (int j = 0; j < 16; ++j) f[j] = fn[j];
         }
+        __syncwarp();  // the next block's TMEM load takes the whole warp
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
