@@ -8,7 +8,7 @@ import torch
 
 from ._lib import stream_handle
 
-_WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
+_WORKSPACES: dict[tuple[int, int, int], torch.Tensor] = {}
 
 
 def device() -> torch.device:
@@ -36,8 +36,9 @@ def as_device(a, dtype=torch.float64) -> torch.Tensor:
 
 def workspace(nbytes: int, slot: int = 0) -> torch.Tensor:
     """A cached uint8 device buffer of at least ``nbytes`` for the current stream
-    (calls on one stream are ordered, so reuse between calls is safe)."""
-    key = (stream_handle(), slot)
+    of the current device (calls on one stream are ordered, so reuse between
+    calls is safe; the default stream has the same handle on every device)."""
+    key = (torch.cuda.current_device(), stream_handle(), slot)
     buf = _WORKSPACES.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device())
