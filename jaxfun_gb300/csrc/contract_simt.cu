@@ -195,16 +195,6 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
-int sm_count(int* n) {
-  static int nsm[64] = {};
-  int dev = 0;
-  JFG_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
-  if (!nsm[dev]) JFG_CUDA_TRY(cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev));
-  *n = nsm[dev];
-  return JFG_OK;
-}
-
 // largest tile (16 R) that still gives two CTAs per SM (the list-restricted
 // launches count their full batch: the active count is not known here)
 int tile_r(const jfg_contract_desc& d, bool f32, int sms) {
@@ -311,6 +301,16 @@ int validate_desc(const jfg_contract_desc& d) {
   if (d.epilogue == JFG_EPI_DIV_EIG && (!d.lam_m || !d.lam_p)) return JFG_ERR_ARG;
   if (d.epilogue < 0 || d.epilogue > 2) return JFG_ERR_ARG;
   if ((d.batch_list == nullptr) != (d.batch_count == nullptr)) return JFG_ERR_ARG;
+  return JFG_OK;
+}
+
+int sm_count(int* n) {
+  static int nsm[64] = {};
+  int dev = 0;
+  JFG_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
+  if (!nsm[dev]) JFG_CUDA_TRY(cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev));
+  *n = nsm[dev];
   return JFG_OK;
 }
 

@@ -57,24 +57,73 @@ __device__ __forceinline__ void fill_tab(int family, int m, HelmTab& T) {
 // Rows: U1 = M x and U2 = K x in a single backward sweep i = n+1 .. 0 over
 // t_i = x_i - x_{i-2}, w = diag(h) t or -(D2 t), y_i = w_i - w_{i+2}.  The two
 // parity classes are independent recurrences, each with its state in registers.
-constexpr int SW = 8;  // steps per chunk of the columns' sweep (even: a chunk
-                       // starts on the class of n+1)
+constexpr int SW = 8;  // steps per chunk of a lane's own sweep, loads first (even:
+                       // a chunk starts on the class of n+1)
 
 struct RowClass {
   double S = 0.0, V = 0.0, x = 0.0;  // suffix sums and the class's pending x_i
 };
+
+// One line by one lane, straight from and to memory.
+__device__ __forceinline__ void helm_row(const HelmTab& T, int n, const double* __restrict__ x,
+                                         double* __restrict__ U1, double* __restrict__ U2) {
+  RowClass A, B;  // A: the parity of n+1, B: the other
+  double wm1 = 0.0, wm2 = 0.0, wk1 = 0.0, wk2 = 0.0;  // w at i+1, i+2
+  for (int i0 = n + 1; i0 >= 0; i0 -= SW) {
+    double xl[SW];
+#pragma unroll
+    for (int k = 0; k < SW; ++k) {
+      const int i = i0 - k;
+      xl[k] = i >= 2 ? x[i - 2] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < SW; ++k) {
+      const int i = i0 - k;
+      if (i < 0) break;
+      RowClass& c = (k & 1) ? B : A;
+      const double t = c.x - xl[k];  // c.x = x_i (loaded as x_{(i+2)-2}); 0 beyond n-1
+      c.x = xl[k];
+      const double wm = __dmul_rn(T.h[i], t);
+      c.V = fma(T.c[i], c.S, c.V);
+      c.S = fma(T.s[i], t, c.S);
+      const double wk = c.V;
+      if (i < n) {
+        U1[i] = wm - wm2;
+        U2[i] = wk - wk2;
+      }
+      wm2 = wm1;
+      wm1 = wm;
+      wk2 = wk1;
+      wk1 = wk;
+    }
+  }
+}
 
 // A warp takes 32 lines, one per lane (off: its first element, n: its length,
 // 0 for a line to leave alone).  The lines are contiguous, so a lane walking
 // its own would touch 32 sectors per access; instead 16 columns of the 32
 // lines at a time are moved through shared memory with coalesced accesses (128
 // bytes of two lines per instruction), counted from each line's own end so
-// that lines of different length go together.  1024 uneven problems (N = 32
-// to 512): 2.75 -> 1.25 ms; 6 FP64 instructions per element bound it at 1.0.
+// that lines of different length go together.  The next 16 are in flight while
+// the present ones are summed; 6 FP64 instructions per element bound the sweep.
 constexpr int RT = 16;           // columns per step of the tiles
 constexpr int RLD = RT + 1;      // their padded rows
-constexpr int ROW_WARPS = 8;     // warps per block
-constexpr size_t ROW_SMEM = (size_t)ROW_WARPS * 2 * 32 * RLD * sizeof(double);
+constexpr int ROW_WARPS = 8;     // most warps per block
+constexpr size_t ROW_TILE = (size_t)2 * 32 * RLD * sizeof(double);  // of a warp
+
+// Warps (of 32 lines) per block of a row launch.  Four keep one warp on each
+// scheduler, and a warp has its share of the FP64 pipe to itself; eight would
+// share it by twos while other SMs stand idle.  Eight where blocks of four would
+// not all be resident (three per SM).
+int row_warps(long long lines, int sms) {
+  return lines > 3LL * 32 * (ROW_WARPS / 2) * sms ? ROW_WARPS : ROW_WARPS / 2;
+}
+// Lines up to which every lane walks its own (TILES false): with two blocks of four
+// warps per SM nothing hides the tiles' copies, and the sectors of uncoalesced
+// accesses hardly hold each other up.  Both sweeps of the operator, 152 SMs:
+// lines of 510, 16320 of them 379 us (tiles 435), 32640 632 (603), 48960 994
+// (812), 65280 1335 (1050); of 126, 8064 86 (96), 32256 149 (160), 50400 234 (214).
+bool row_tiled(long long lines, int sms) { return lines > 64LL * (ROW_WARPS / 2) * sms; }
 
 __device__ __forceinline__ void helm_rows_warp(const HelmTab& T, int n, long long off,
                                                const double* __restrict__ x,
@@ -82,7 +131,7 @@ __device__ __forceinline__ void helm_rows_warp(const HelmTab& T, int n, long lon
                                                double* tiles) {
   const int lane = threadIdx.x & 31;
   double* X = tiles;              // x, then U1 in its place
-  double* Y = tiles + 32 * RLD;   // U2
+  const double* Y = tiles + 32 * RLD;  // U2
   int top = n;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
@@ -90,37 +139,54 @@ __device__ __forceinline__ void helm_rows_warp(const HelmTab& T, int n, long lon
   const int half = lane >> 4, col = lane & 15;
   RowClass A, B;  // A: the parity of n+1, B: the other
   double wm1 = 0.0, wm2 = 0.0, wk1 = 0.0, wk2 = 0.0;  // w at i+1, i+2
-  for (int k0 = 0; k0 < top + 2; k0 += RT) {
-    // step k of a line is i = n + 1 - k and reads x_{i-2}, x_{n-1-k}: column
-    // j of the tile holds step k0 + RT - 1 - j, ascending in memory
+  // step k of a line is i = n + 1 - k and reads x_{i-2}, x_{n-1-k}: column
+  // j of the tile holds step k0 + RT - 1 - j, ascending in memory
+  double next[16];
+  auto fetch = [&](int k0) {
 #pragma unroll
     for (int r2 = 0; r2 < 16; ++r2) {
       const int r = 2 * r2 + half;
       const int nr = __shfl_sync(0xffffffffu, n, r);
       const long long orr = __shfl_sync(0xffffffffu, off, r);
       const int c = nr - k0 - RT + col;  // n - 1 - k
-      X[r * RLD + col] = (c >= 0 && c < nr) ? x[orr + c] : 0.0;
+      next[r2] = (c >= 0 && c < nr) ? x[orr + c] : 0.0;
     }
-    __syncwarp();
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < top + 2; k0 += RT) {
 #pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      const int i = n + 1 - k0 - k;
-      double* cell = X + lane * RLD + (RT - 1 - k);
-      if (i >= 0 && n > 0) {
+    for (int r2 = 0; r2 < 16; ++r2) X[(2 * r2 + half) * RLD + col] = next[r2];
+    __syncwarp();
+    if (k0 + RT < top + 2) fetch(k0 + RT);
+    // eight steps at a time between the tile's loads and stores, so that neither
+    // waits for the other's arithmetic; past a line's end (i < 0) nothing is kept
+#pragma unroll
+    for (int h = 0; h < RT; h += 8) {
+      double* cell = X + lane * RLD + (RT - 1 - h);
+      double xl[8], y1[8], y2[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) xl[k] = cell[-k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int i = max(n + 1 - k0 - h - k, 0);
         RowClass& c = (k & 1) ? B : A;
-        const double xl = *cell;
-        const double t = c.x - xl;  // c.x = x_i (loaded as x_{(i+2)-2}); 0 beyond n-1
-        c.x = xl;
-        const double wm = T.h[i] * t;
+        const double t = c.x - xl[k];  // c.x = x_i (loaded as x_{(i+2)-2}); 0 beyond n-1
+        c.x = xl[k];
+        const double wm = __dmul_rn(T.h[i], t);
         c.V = fma(T.c[i], c.S, c.V);
         c.S = fma(T.s[i], t, c.S);
         const double wk = c.V;
-        *cell = wm - wm2;
-        Y[lane * RLD + (RT - 1 - k)] = wk - wk2;
+        y1[k] = wm - wm2;
+        y2[k] = wk - wk2;
         wm2 = wm1;
         wm1 = wm;
         wk2 = wk1;
         wk1 = wk;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        cell[-k] = y1[k];
+        cell[32 * RLD - k] = y2[k];
       }
     }
     __syncwarp();
@@ -182,6 +248,7 @@ __device__ __forceinline__ void helm_col(const HelmTab& T, int n, const double* 
 }
 
 // axis 1 (contiguous): U1 = rows through M, U2 = rows through K
+template <bool TILES>
 __global__ void __launch_bounds__(32 * ROW_WARPS)
     k_helm_rows(int family, int n, long long nlines, const double* __restrict__ u,
                 double* __restrict__ U1, double* __restrict__ U2) {
@@ -189,8 +256,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS)
   __shared__ HelmTab T;
   fill_tab(family, n + 2, T);
   const long long line = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (!TILES) {
+    if (line < nlines) helm_row(T, n, u + line * n, U1 + line * n, U2 + line * n);
+    return;
+  }
   helm_rows_warp(T, line < nlines ? n : 0, line * n, u, U1, U2,
-                 row_tiles + (threadIdx.x >> 5) * (2 * 32 * RLD));
+                 row_tiles + (threadIdx.x >> 5) * (ROW_TILE / sizeof(double)));
 }
 
 // axis 0 (stride n): v = (alpha2 M + K) U1 + M U2 (columns), optionally r = b - v
@@ -214,8 +285,8 @@ int row_setup() {
   JFG_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
   if (!done[dev])
-    JFG_CUDA_TRY(cudaFuncSetAttribute(k_helm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)ROW_SMEM));
+    JFG_CUDA_TRY(cudaFuncSetAttribute(k_helm_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(ROW_WARPS * ROW_TILE)));
   done[dev] = true;
   return JFG_OK;
 }
@@ -239,10 +310,16 @@ extern "C" int jfg_helmholtz_apply_f64(int family, int n, int batch, const doubl
   double* U2 = (double*)((char*)work + need / 2);
   const long long nl = (long long)batch * n;
   const int blocks = (int)((nl + 127) / 128);
-  const int rblocks = (int)((nl + 32 * jfg::ROW_WARPS - 1) / (32 * jfg::ROW_WARPS));
+  int sms = 0;
+  JFG_TRY(jfg::sm_count(&sms));
+  const int rw = jfg::row_warps(nl, sms);
+  const int rblocks = (int)((nl + 32 * rw - 1) / (32 * rw));
   cudaStream_t st = (cudaStream_t)stream;
   JFG_TRY(jfg::row_setup());
-  jfg::k_helm_rows<<<rblocks, 32 * jfg::ROW_WARPS, jfg::ROW_SMEM, st>>>(family, n, nl, u, U1, U2);
+  if (jfg::row_tiled(nl, sms))
+    jfg::k_helm_rows<true><<<rblocks, 32 * rw, rw * jfg::ROW_TILE, st>>>(family, n, nl, u, U1, U2);
+  else
+    jfg::k_helm_rows<false><<<rblocks, 32 * rw, 0, st>>>(family, n, nl, u, U1, U2);
   JFG_LAUNCHED();
   jfg::k_helm_cols<<<blocks, 128, 0, st>>>(family, n, batch, U1, U2, alpha2, b, v);
   JFG_LAUNCHED();
@@ -481,6 +558,7 @@ __device__ __forceinline__ int find_prob(const HelmProb* tb, int nprob, long lon
 }
 
 // rows (contiguous axis) of every problem: U1 = rows through M, U2 through K
+template <bool TILES>
 __global__ void __launch_bounds__(32 * ROW_WARPS)
     k_rag_rows(int family, int nprob, int mmax, long long nlines,
                const HelmProb* __restrict__ tb, const double* __restrict__ gate,
@@ -497,7 +575,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS)
     off = q.off64 + (line - q.line0) * q.n;
     n = gate[p] == 0.0 ? 0 : q.n;  // x unchanged: its residual stands
   }
-  helm_rows_warp(T, n, off, u, U1, U2, row_tiles + (threadIdx.x >> 5) * (2 * 32 * RLD));
+  if (!TILES) {
+    if (n > 0) helm_row(T, n, u + off, U1 + off, U2 + off);
+    return;
+  }
+  helm_rows_warp(T, n, off, u, U1, U2,
+                 row_tiles + (threadIdx.x >> 5) * (ROW_TILE / sizeof(double)));
 }
 
 // shared-memory opt-in of k_rag_rows, once per device (call before a capture)
@@ -507,8 +590,8 @@ int rag_row_setup() {
   JFG_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return JFG_ERR_UNSUPPORTED;
   if (!done[dev])
-    JFG_CUDA_TRY(cudaFuncSetAttribute(k_rag_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)ROW_SMEM));
+    JFG_CUDA_TRY(cudaFuncSetAttribute(k_rag_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(ROW_WARPS * ROW_TILE)));
   done[dev] = true;
   return JFG_OK;
 }
@@ -685,7 +768,10 @@ extern "C" int jfg_helmholtz_solve_grouped(
   const long long avg32 = Lo.tot32 / np + 1;
   const dim3 vgrid((unsigned)((avg32 + 255) / 256 < 64 ? (avg32 + 255) / 256 : 64), np);
   const unsigned lblocks = (unsigned)((Lo.lines + 127) / 128);
-  const unsigned rblocks = (unsigned)((Lo.lines + 32 * ROW_WARPS - 1) / (32 * ROW_WARPS));
+  int sms = 0;
+  JFG_TRY(sm_count(&sms));
+  const int rw = row_warps(Lo.lines, sms);
+  const unsigned rblocks = (unsigned)((Lo.lines + 32 * rw - 1) / (32 * rw));
 
   auto step = [&]() -> int {
     k_rag_pad<<<vgrid, 256, 0, st>>>(tb, r64, hin, r32);
@@ -700,8 +786,11 @@ extern "C" int jfg_helmholtz_solve_grouped(
                                 out3.data(), tc, st));
     k_rag_axpy<<<vgrid, 256, 0, st>>>(tb, d32, hout, x, nref);
     JFG_LAUNCHED();
-    k_rag_rows<<<rblocks, 32 * ROW_WARPS, ROW_SMEM, st>>>(family, np, mmax, Lo.lines, tb, hout, x,
-                                                           U1, U2);
+    if (row_tiled(Lo.lines, sms))
+      k_rag_rows<true><<<rblocks, 32 * rw, rw * ROW_TILE, st>>>(family, np, mmax, Lo.lines, tb, hout,
+                                                               x, U1, U2);
+    else
+      k_rag_rows<false><<<rblocks, 32 * rw, 0, st>>>(family, np, mmax, Lo.lines, tb, hout, x, U1, U2);
     JFG_LAUNCHED();
     k_rag_cols<<<lblocks, 128, 0, st>>>(family, np, mmax, Lo.lines, tb, hout, U1, U2, alpha2, rhs,
                                         r64);

@@ -88,6 +88,7 @@ struct DotOut {
   int* nb = nullptr;
 };
 
+int sm_count(int* n);  // SMs of the current device
 // tile of the FP64 CUDA-core launch (64, 32 or 16)
 int contract_f64_tile(const jfg_contract_desc& d);
 int contract_f64(const jfg_contract_desc& d, const double* op, const double* in, double* out,
