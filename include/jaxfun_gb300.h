@@ -201,8 +201,9 @@ int jfg_tc_set_store_path(int tma_store);
  * operator chunk) slot, keeps that chunk for all K in shared memory and
  * streams only input tiles -- where the chunk fits beside four input blocks
  * (hi and lo: K <= 256 16-bit or 128 TF32 elements at 128 operator rows),
- * there are >= 2 tiles per CTA and the inputs stay in L2; 2 whenever the chunk
- * fits.  The autotuner tries both where the chunk fits. */
+ * there are >= 2 tiles per CTA, the inputs stay in L2 and it is not a split
+ * 16-bit launch without field, divide or beta (those gain by some sizes and lose
+ * by others); 2 whenever the chunk fits.  The autotuner tries both where the chunk fits. */
 int jfg_tc_set_op_resident(int on);
 /* Launch configuration of the tensor-core contraction. */
 typedef struct {

@@ -64,12 +64,16 @@ __device__ int g_tc_test_hold = 0;
 static int g_operand_a_in_tmem = 1;
 // Operator-stationary schedule for single-group launches whose operator chunk
 // fits in shared memory: 0 off, 1 (default) when every CTA gets >= 2 tiles, the
-// chunk leaves four input blocks and the inputs stay in L2, 2 whenever the
-// chunk fits (jfg_tc_set_op_resident); a launch configuration's schedule field
-// overrides it.  Measured against streaming (128 problems, N = 256, split
-// FP16): 34.5 against 36.5 us (M = 512), field pass 49 against 51, divide pass
-// (split BF16) 22.6 against 23.9; 3-D 8 x 128^3 split TF32: 43 against 47.5.
-// Inputs beyond L2 (3 x 8 x 128^3): 117 against 104 us, so they stream.
+// chunk leaves four input blocks, the inputs stay in L2 and the kernel has one
+// splitting group, 2 whenever the chunk fits (jfg_tc_set_op_resident); a launch
+// configuration's schedule field overrides it.  Measured against streaming (128
+// problems, N = 256): field pass (split FP16) 49.8 against 53.0 us, plain BF16
+// 16.4 against 18.4; 3-D 8 x 128^3 split TF32: 43 against 47.5.  Inputs beyond
+// L2 (3 x 8 x 128^3): 117 against 104 us, so they stream.  The kernels with two
+// splitting groups (plain epilogue of the split 16-bit paths) gain or lose by
+// the size and stream by default, the autotuner tries both: split FP16, M = 512,
+// 128 problems 35.5 against 34.9 us, 64 problems 21.7 against 22.6; split BF16
+// 19.2 against 20.5 for 128 problems, 10.8 against 10.3 for 32.
 static int g_op_resident = 1;
 
 namespace {
