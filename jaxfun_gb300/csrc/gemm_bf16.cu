@@ -340,7 +340,8 @@ extern "C" int jfg_gemm_bf16(const jfg_gemm_desc* dp, const void* A, const void*
   // (fewer where the CTAs would leave a quarter of the SMs idle: a CTA is bound
   // by what its SM can take in from L2; 32 samples, M = 1024, K = 4096: 64 CTAs
   // of four samples 36.7 us, 128 of two 31.0)
-  const int sms = 152;
+  int sms = 0;
+  JFG_TRY(sm_count(&sms));
   const long long mtiles = (d.M + TM - 1) / TM;
   prm.nb = 1;
   if (prm.b_bat && !prm.a_bat && d.ksplit == 1 && d.N % 16 == 0)

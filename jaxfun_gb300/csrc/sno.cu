@@ -288,7 +288,9 @@ extern "C" int jfg_sno_modemix_fwd(int batch, int nmodes, int C, const float* R,
   if (nmodes % MM_Q != 0) return JFG_ERR_ARG;
   // samples spread over the blocks' second index where modes are few
   const int mblocks = nmodes >= MM_FEW ? nmodes / 4 : nmodes;
-  const int groups = std::max(1, std::min((2 * 152 + mblocks - 1) / mblocks, (batch + MM_B - 1) / MM_B));
+  int sms = 0;
+  JFG_TRY(sm_count(&sms));
+  const int groups = std::max(1, std::min((2 * sms + mblocks - 1) / mblocks, (batch + MM_B - 1) / MM_B));
   const int per_block = (batch + groups - 1) / groups;
   auto* f = nmodes >= MM_FEW ? mix_launch<4, false> : mix_launch<1, false>;
   return f((batch + per_block - 1) / per_block, per_block, batch, nmodes, C, R, x, nullptr, out,
