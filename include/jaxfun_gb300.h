@@ -289,9 +289,21 @@ int jfg_tc_test_hold(int on);
  * operators of OrthogonalSpace/Composite/Chebyshev (src/jaxfun/galerkin/
  * orthogonal.py:214-277, composite.py:205-349, Chebyshev.py:225-279).
  * ndim in {1,2,3}.  Workspace: jfg_tp_apply_workspace_size bytes.
+ *
+ * FP64 with that workspace: passes large enough for it take their products from
+ * FP16 digits on the tensor cores where the operator is dense (nearly all of its
+ * entries within 2^7 of their row's largest, once its columns have been scaled
+ * to one size: the transforms of the spaces are); banded, triangular, diagonal
+ * and graded operators are summed by FP64 FMAs in the same launch.  A digit sum
+ * of K terms is off by about sqrt(7 K) 2^-63.6 times the largest scaled entries
+ * of its operator row and its input row, and by its rounding to FP64.  With
+ * jfg_tp_apply_fma_workspace_size bytes every pass is summed by FP64 FMAs, which
+ * is the faster way where no operator is dense.
  */
 size_t jfg_tp_apply_workspace_size(int ndim, const int* rows, const int* cols, int batch,
                                    int elem_bytes);
+size_t jfg_tp_apply_fma_workspace_size(int ndim, const int* rows, const int* cols, int batch,
+                                       int elem_bytes);
 int jfg_tp_apply_f64(int ndim, const int* rows, const int* cols, int batch,
                      const double* const* mats, const double* in, double* out,
                      void* work, size_t work_bytes, void* stream);
@@ -356,6 +368,11 @@ int jfg_banded_lu_solve_f64(int nsys, int n, int p, int q, const double* lu, con
  * Same n x n E (= W^{-1} M^{-1}; W^T for symmetric pairs), W and lam on
  * every axis (square tensor-product space, n per axis), rhs/out
  * (batch, n^ndim).  lam has length n.  ndim in {2,3}.
+ * FP64 with jfg_fd_solve_workspace_size bytes: large solves take the products
+ * from FP16 digits (see jfg_tp_apply_f64) unless a factor is sparse (fewer than
+ * 9/32 of its entries large); W's columns and their inputs are scaled by half of
+ * the eigenvalues' exponents, which keeps the small entries of the solution as
+ * near as FMAs do.
  */
 size_t jfg_fd_solve_workspace_size(int ndim, int n, int batch, int elem_bytes);
 int jfg_fd_solve_f64(int ndim, int n, int batch, const double* E, const double* W,

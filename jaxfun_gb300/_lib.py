@@ -108,6 +108,7 @@ SIGNATURES = {
     "jfg_tc_set_wait_budget_ns": (_i, [C.c_ulonglong]),
     "jfg_tc_test_hold": (_i, [_i]),
     "jfg_tp_apply_workspace_size": (_sz, [_i, C.POINTER(_i), C.POINTER(_i), _i, _i]),
+    "jfg_tp_apply_fma_workspace_size": (_sz, [_i, C.POINTER(_i), C.POINTER(_i), _i, _i]),
     "jfg_tp_apply_f64": (_i, [_i, C.POINTER(_i), C.POINTER(_i), _i, C.POINTER(_vp), _vp, _vp,
                               _vp, _sz, _vp]),
     "jfg_tp_apply_f32": (_i, [_i, C.POINTER(_i), C.POINTER(_i), _i, C.POINTER(_vp), _vp, _vp,

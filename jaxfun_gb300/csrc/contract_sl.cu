@@ -4,7 +4,7 @@
 //
 // with FP64 operands and FP64 results.  GB300 issues about 2 FP64 FMAs per
 // clock per SM, so the CUDA-core contraction (contract_simt.cu) is bound by
-// that pipe at ~1.24 TFLOP/s.  Here every operand row becomes a 62-bit
+// that pipe at ~1.24 TFLOP/s.  Here every operand row becomes a 63-bit
 // fixed-point number per element (one power-of-two scale per row), cut into
 // eight signed base-256 digits that FP16 holds exactly; products of digits are
 // accumulated exactly by the tensor cores (kind::f16, FP32 accumulators that
@@ -17,9 +17,12 @@
 // Accuracy.  The operator's columns are first scaled by powers of two to a
 // largest entry in [1, 2) and the input's columns by the inverse, so that a
 // column of large entries against small coefficients (derivatives of spectral
-// bases) does not cost digits.  An element then keeps 61 bits below its
-// scaled row's largest one, and the digit products left out (weights 2^-64
-// and below) are as small.  Level d sums at most d + 1 digit pairs, each
+// bases) does not cost digits.  An element then keeps 62 bits below its
+// scaled row's largest one; the digit products left out are larger: 7 K of
+// level 8, about sqrt(7 K) 2^-63.6 of the two rows' largest entries' product.
+// So a sum is as accurate as by FMAs where the operator meets the input's
+// largest entries with entries not far below its row's largest one, which
+// k_sl_split judges by the operator.  Level d sums at most d + 1 digit pairs, each
 // below 2^14 K: levels 0..3 cannot pass 2^24 for K <= 256 (0 and 1 for
 // K <= 512), and a level that did could only lose its last bits, which weigh
 // 2^-8d.  Rows with an infinity or a NaN (in the operator or the input) are
@@ -57,6 +60,8 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "jfg_internal.cuh"
 #include "tc_common.cuh"
 
@@ -91,6 +96,8 @@ struct SlLaunch {
   double* out;
   const int* row_e;      // [segments][M]
   const int16_t* col_e;  // [segments][kpad]
+  const int* use;        // [segments] 0: FP64 FMAs instead of digits
+  int ctas;              // CTAs that digits take; the others serve FMA sums alone
   int op_segs;           // segments of the operator (1: shared by all)
   int row_ld;            // row exponents per segment
   int kpad;              // K padded to 64
@@ -120,12 +127,21 @@ __device__ __forceinline__ int short_of(const uint4& v, int e) {
   return (e & 1) ? (int)w >> 16 : (int)(w << 16) >> 16;
 }
 
-// x 2^(61 - E) truncated to an integer (|.| < 2^62; e = elem_e(x) <= E, E its
-// row's maximum), plus 0x80 in every byte: byte 7 - j is then digit j + 128.
+// The same with six bits of the mantissa below it; a row's exponent is row_e_of
+// of the largest key: one more than the largest element's where its mantissa is
+// within 2^-6 of 2.
+__device__ __forceinline__ int elem_key(double x, int ce) {
+  return max((__double2hiint(x) >> 14) & 0x1FFFF, 64) + 64 * ce;
+}
+constexpr int NO_KEY = -(1 << 25);  // a row of zeros
+__device__ __forceinline__ int row_e_of(int key) { return (key + 1) >> 6; }
+// x 2^(62 - E) truncated to an integer (|.| < 2^63 (1 - 2^-7), e = elem_e(x) <= E,
+// E its row's exponent), plus 0x80 in every byte: byte 7 - j is then
+// digit j + 128, and the sum has not passed 64 bits.
 __device__ __forceinline__ unsigned long long biased_fixed(double x, int e, int E) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   const uint32_t mh = (hi & 0xFFFFFu) | ((hi & 0x7FF00000u) ? 0x100000u : 0u);
-  const unsigned long long m = ((unsigned long long)mh << 32 | lo) << 9;
+  const unsigned long long m = ((unsigned long long)mh << 32 | lo) << 10;
   const unsigned s = min((unsigned)(E - e), 63u);  // a zero with e > E wraps to 63
   const unsigned long long v = m >> s;
   const unsigned long long sg = (unsigned long long)((long long)((unsigned long long)hi << 32) >> 63);
@@ -147,24 +163,50 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned lo
 // operator digits
 // ---------------------------------------------------------------------------
 
-constexpr int SPLIT_T = 256;
+constexpr int SPLIT_T = 512;
 constexpr int SPLIT_CL = 8;
+static_assert(SPLIT_T == SL_KMAX, "a thread per column");
 
 struct SlSeg {
   const double* src;
+  const double* lam;
   long long ld;
   int M, K, Kp, kpad;
   uint16_t* dig;  // [NS][M][Kp]
   int* row_e;
   int16_t* col_e;
+  int* use;
+  SlRule rule;
 };
 struct SlSplitArgs {
   SlSeg s[SL_MAX_SEGS];
 };
 
+// Whether digits keep what FP64 sums keep of every entry.  A digit sum is off by
+// about sqrt(7 K) 2^-63.6 of (row's largest scaled entry) x (input row's largest),
+// an FP64 sum by 2^-53 of the terms' magnitudes: the two compare when the
+// operator meets the input's largest entries with entries of its own that are
+// not far below their row's largest.  "Large" is an entry whose first digit is
+// not zero: within 2^7 to 2^8 of it.
+// SL_DENSE asks for large entries nearly everywhere (15/16 of all, 3/8 of every
+// row and column: the transforms of the spaces have 0.98 or more and 0.49 or
+// more, N = 24 to 256, both families), so that it does not matter which entries
+// of the input are the largest.  Banded, triangular, diagonal and graded
+// operators fall short of it: an identity on e^-k keeps nothing from k = 45 on.
+// SL_FACTORS (eigenvector factors, the variable-coefficient operator) turns away
+// the sparse ones alone (large entries: half of each factor is zero by parity,
+// 0.335 or more are large for N = 17 to 400); those factors were measured entry
+// by entry through the whole call instead.
+__device__ __forceinline__ bool dense_enough(SlRule rule, long long large, long long rows,
+                                             long long cols) {
+  return rule == SL_DENSE ? 16 * large >= 15 * rows * cols : 32 * large >= 9 * rows * cols;
+}
+__device__ __forceinline__ bool line_dense(int large, int len) { return 8 * large >= 3 * len; }
+
 // One cluster of 8 CTAs per operator segment: column maxima over each CTA's
 // rows, combined through distributed shared memory; then one warp per row
-// finds the row's exponent and writes its digits.  A few microseconds, bound
+// finds the row's exponent, writes its digits and counts its large entries, for
+// *use: whether the contraction is to take the digits.  A few microseconds, bound
 // by the latency of two reads of the rows (256 x 256: 4 rows per warp).
 __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
     k_sl_split(const __grid_constant__ SlSplitArgs A) {
@@ -172,32 +214,56 @@ __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
   cg::cluster_group cl = cg::this_cluster();
   __shared__ int cmax[512];
   __shared__ int16_t ce[512];
+  // large entries of each column in this CTA's rows ([element][chunk], so that a
+  // warp's adds lie in different banks) and, in rank 0, in all rows
+  __shared__ int clarge[512], call[512];
+  // columns that are not zero; rank 0: regular rows, their large entries, and
+  // whether a row has too few
+  __shared__ int cols, rows, large, thin;
   const SlSeg& q = A.s[blockIdx.x / SPLIT_CL];
   const int rank = (int)cl.block_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int k = threadIdx.x; k < q.K; k += SPLIT_T) {
+  cmax[threadIdx.x] = -1;
+  clarge[threadIdx.x] = call[threadIdx.x] = 0;
+  if (threadIdx.x == 0) cols = rows = large = thin = 0;
+  __syncthreads();
+  // as many threads as fit take rows of a column in turn
+  const int kc = q.K <= 128 ? 128 : q.K <= 256 ? 256 : SPLIT_T, k1 = threadIdx.x % kc;
+  if (k1 < q.K) {
     int mx = -1;
-    for (int m = rank; m < q.M; m += SPLIT_CL) {
-      const double x = q.src[(long long)m * q.ld + k];
+    for (int m = rank + SPLIT_CL * (threadIdx.x / kc); m < q.M; m += SPLIT_CL * (SPLIT_T / kc)) {
+      const double x = q.src[(long long)m * q.ld + k1];
       if (!is_zero(x) && !not_finite(x)) mx = max(mx, elem_e(x, 0));
     }
-    cmax[k] = mx;
+    if (mx >= 0) atomicMax(&cmax[k1], mx);
   }
   cl.sync();
-  for (int k = threadIdx.x; k < q.kpad; k += SPLIT_T) {
+  if (const int k = threadIdx.x; k < q.kpad) {  // whole warps: kpad is a multiple of 64
     int c = 0;
     if (k < q.K) {
       int mx = -1;
+#pragma unroll
       for (int r = 0; r < SPLIT_CL; ++r) mx = max(mx, cl.map_shared_rank(cmax, r)[k]);
       c = mx < 0 ? NO_COLUMN : mx - 1023;
+      if (mx >= 0) {
+        // half of the eigenvalue's exponent: the inputs fall off like its
+        // inverse, so that it evens out both sides
+        if (q.lam && !is_zero(q.lam[k]) && !not_finite(q.lam[k]))
+          c += (elem_e(q.lam[k], 0) - 1023) >> 1;
+      }
     }
-    if (k < 512) ce[k] = (int16_t)c;
+    const unsigned any = __ballot_sync(0xffffffffu, c != NO_COLUMN && k < q.K);
+    if (lane == 0) atomicAdd(&cols, __popc(any));
+    ce[k] = (int16_t)c;
     if (rank == 0) q.col_e[k] = (int16_t)c;
   }
   cl.sync();  // also keeps cmax alive until every peer has read it
+  const int ncol = cols;
+  int cnt[2][8] = {}, nrow = 0, nlarge = 0;
+  bool short_row = false;
   for (int m = rank + SPLIT_CL * warp; m < q.M; m += SPLIT_CL * (SPLIT_T / 32)) {
     const double* row = q.src + (long long)m * q.ld;
-    int E = -(1 << 19);
+    int key = NO_KEY;
     bool bad = false;
     double x[2][8];
 #pragma unroll
@@ -208,14 +274,15 @@ __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
         x[i][e] = k < q.K ? row[k] : 0.0;
         if (not_finite(x[i][e])) bad = true;
         // the column's exponent moves to the input: subtract it here
-        else if (!is_zero(x[i][e])) E = max(E, elem_e(x[i][e], -(int)ce[k]));
+        else if (!is_zero(x[i][e])) key = max(key, elem_key(x[i][e], -(int)ce[k]));
       }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+    int E = row_e_of(__reduce_max_sync(0xffffffffu, key));
     bad = __any_sync(0xffffffffu, bad);
     if (bad) E = SPECIAL;
+    const bool regular = E > -(1 << 18) && !bad;
     if (lane == 0) q.row_e[m] = E < -(1 << 18) ? 0 : E;
     if (E < -(1 << 18)) E = 0;
+    int n = 0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int k0 = 8 * (lane + 32 * i);
@@ -224,6 +291,14 @@ __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
 #pragma unroll
       for (int e = 0; e < 8; ++e)
         f[e] = biased_fixed(x[i][e], elem_e(x[i][e], k0 + e < q.K ? -(int)ce[k0 + e] : 0), E);
+      if (regular) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int l = (uint32_t)(f[e] >> 56) != 0x80u;
+          n += l;
+          cnt[i][e] += l;
+        }
+      }
 #pragma unroll
       for (int j = 0; j < NS; ++j) {
         uint4 v;
@@ -234,6 +309,39 @@ __global__ void __cluster_dims__(SPLIT_CL, 1, 1) __launch_bounds__(SPLIT_T)
         *reinterpret_cast<uint4*>(q.dig + ((long long)j * q.M + m) * q.Kp + k0) = v;
       }
     }
+    if (regular) {
+      n = __reduce_add_sync(0xffffffffu, n);
+      ++nrow;
+      nlarge += n;
+      short_row = short_row || !line_dense(n, ncol);
+    }
+  }
+  // all counts to rank 0, which judges
+  if (q.rule == SL_DENSE) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (cnt[i][e]) atomicAdd(clarge + 64 * e + lane + 32 * i, cnt[i][e]);
+    __syncthreads();
+    const int c = clarge[threadIdx.x];
+    if (c) atomicAdd(cl.map_shared_rank(call, 0) + threadIdx.x, c);
+  }
+  if (lane == 0) {
+    atomicAdd(cl.map_shared_rank(&rows, 0), nrow);
+    atomicAdd(cl.map_shared_rank(&large, 0), nlarge);
+    if (short_row) atomicOr(cl.map_shared_rank(&thin, 0), 1);
+  }
+  cl.sync();
+  if (rank == 0) {
+    bool ok = dense_enough(q.rule, large, rows, ncol);
+    if (q.rule == SL_DENSE) {
+      const int k = threadIdx.x;
+      ok = ok && !thin && (k >= q.K || ce[k] == NO_COLUMN ||
+                           line_dense(call[64 * (k & 7) + (k >> 3)], rows));
+      ok = __syncthreads_and(ok) != 0;
+    }
+    if (threadIdx.x == 0) *q.use = ok ? 1 : 0;
   }
 }
 
@@ -330,11 +438,112 @@ __device__ __forceinline__ double level_value(long long H, long long lo, int sh,
   return __hiloint2double(ex ? hi + ((sh - 32) << 20) : 0, __double2loint(v));
 }
 
+// whether every operator segment of the launch is to be taken as digits
+__device__ __forceinline__ bool use_digits(const SlLaunch& L) {
+  int u = 1;
+  for (int s = 0; s < L.op_segs; ++s) u &= __ldg(L.use + s);
+  return u != 0;
+}
+
+// The whole launch by FP64 FMAs, for an operator whose digits would lose entries:
+// tiles of 16 R operator rows by 32 R input rows over the CTAs, summed in the
+// order of the CUDA-core contraction (the same bits).  Bound by the FP64 pipe:
+// a thread reads 2 R values from shared memory per R^2 FMAs of 64 clocks.  R = 1
+// unless there are many tiles of R = 2, for less idling in the last round.  The
+// next 32 K are in registers while the present ones are multiplied.
+constexpr int FMA_K = 32;
+template <int EPI, int R>
+__device__ __forceinline__ void fma_tiles_r(const SlLaunch& L, int nb, double* sm) {
+  constexpr int TM = 16 * R, TP = 32 * R, T = 512;  // warps 0-15 multiply
+  constexpr int LA = TM + 1, LB = TP + 1, NA = TM * FMA_K / T, NB = TP * FMA_K / T;
+  const jfg_contract_desc& d = L.d;
+  double* As = sm;                // [FMA_K][LA]
+  double* Bs = sm + FMA_K * LA;   // [FMA_K][LB]
+  const int t = threadIdx.x, tx = t & 31, ty = t >> 5, kk = t % FMA_K, r0 = t / FMA_K;
+  const unsigned mt = (unsigned)((d.M + TM - 1) / TM), ptl = (unsigned)((d.P + TP - 1) / TP);
+  const long long tiles = (long long)nb * d.nseg * ptl * mt;
+  for (long long i = blockIdx.x; i < tiles; i += gridDim.x) {
+    const int m0 = (int)(i % mt) * TM, p0 = (int)(i / mt % ptl) * TP;
+    const int bs = (int)(i / ((long long)mt * ptl)), slot = bs / d.nseg, s = bs - slot * d.nseg;
+    const int b = active_problem(d.batch_list, nb, d.batch, slot);
+    if (b < 0) continue;  // the same for the whole CTA
+    const double* a = L.op + (L.op_segs > 1 ? (long long)s * d.op_seg : 0);
+    const double* y = L.in + (long long)b * d.in_batch + (long long)s * d.in_seg;
+    double av[NA], bv[NB], acc[R][R] = {};
+    auto load = [&](int k) {
+#pragma unroll
+      for (int j = 0; j < NA; ++j) {
+        const int m = m0 + r0 + j * (T / FMA_K);
+        av[j] = t < T && m < d.M && k < d.K ? __ldg(a + (long long)m * d.op_ld + k) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        const int p = p0 + r0 + j * (T / FMA_K);
+        bv[j] = t < T && p < d.P && k < d.K ? __ldg(y + (long long)p * d.in_ld + k) : 0.0;
+      }
+    };
+    load(kk);
+    for (int k0 = 0; k0 < d.K; k0 += FMA_K) {
+      __syncthreads();
+      if (t < T) {
+#pragma unroll
+        for (int j = 0; j < NA; ++j) As[kk * LA + r0 + j * (T / FMA_K)] = av[j];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) Bs[kk * LB + r0 + j * (T / FMA_K)] = bv[j];
+      }
+      __syncthreads();
+      if (k0 + FMA_K < d.K) load(k0 + FMA_K + kk);
+      if (t < T) {
+#pragma unroll 8
+        for (int k = 0; k < FMA_K; ++k)
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+#pragma unroll
+            for (int v = 0; v < R; ++v)
+              acc[u][v] = fma(As[k * LA + ty + 16 * u], Bs[k * LB + tx + 32 * v], acc[u][v]);
+      }
+    }
+    if (t >= T) continue;
+    double c0 = 0.0, c1 = 1.0;
+    if (EPI == JFG_EPI_DIV_EIG) {
+      if (d.c0) c0 = ((const double*)d.c0)[b];
+      if (d.c1) c1 = ((const double*)d.c1)[b];
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u)
+#pragma unroll
+      for (int v = 0; v < R; ++v) {
+        const int m = m0 + ty + 16 * u, p = p0 + tx + 32 * v;
+        if (m >= d.M || p >= d.P) continue;
+        double w = acc[u][v];
+        if (EPI == JFG_EPI_MUL_FIELD)
+          w *= ((const double*)d.field)[(long long)b * d.field_batch + (long long)s * d.field_seg +
+                                        (long long)m * d.field_ld + p];
+        else if (EPI == JFG_EPI_DIV_EIG)
+          w = w / (c0 + c1 * (((const double*)d.lam_m)[m] + ((const double*)d.lam_p)[p]));
+        double* o = L.out + (long long)b * d.out_batch + (long long)s * d.out_seg +
+                    (long long)m * d.out_ld + p;
+        w = d.alpha * w;
+        if (d.beta != 0.0) w += d.beta * *o;
+        *o = w;
+      }
+  }
+}
+template <int EPI>
+__device__ __noinline__ void fma_tiles(const SlLaunch& L, int nb, double* sm) {
+  const jfg_contract_desc& d = L.d;
+  if ((long long)nb * d.nseg * ((d.M + 31) / 32) * ((d.P + 63) / 64) >= 8LL * gridDim.x)
+    fma_tiles_r<EPI, 2>(L, nb, sm);
+  else
+    fma_tiles_r<EPI, 1>(L, nb, sm);
+}
+constexpr size_t FMA_SMEM = FMA_K * (33 + 65) * 8;
+
 template <int EPI, bool LIN, int PT>
 __global__ void __launch_bounds__(SL_NT, 1)
     k_contract_sl(const __grid_constant__ SlLaunch L) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int s_nb;
+  __shared__ int s_nb, s_dig;
   // aligned by an offset, so that accesses stay in the shared window for the
   // compiler (through an integer they become generic ones, which it must order
   // against the global stores)
@@ -362,6 +571,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
   // uniform registers
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
+  if (blockIdx.x >= (unsigned)L.ctas && use_digits(L)) return;
   if (threadIdx.x == 0) {
     s_nb = active_count(d.batch_list, d.batch_count, d.batch);
     for (int i = 0; i < A_MAX; ++i) {
@@ -413,6 +623,8 @@ __global__ void __launch_bounds__(SL_NT, 1)
     s = (int)t - slot * d.nseg;
   };
 
+  // The digits are summed whether they are to be taken or not, so that nothing
+  // waits for the verdict; results are stored only if they are.
   if (warp == 0) {
     // ---------------- operator producer ----------------
     if (lane == 0) {
@@ -453,6 +665,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
         for (long long q = issued > L.astages ? issued - L.astages : 0; q < issued; ++q)
           tc::mbar_wait(&afull[q % L.astages], (uint32_t)(q / L.astages) & 1u, &g_sl_status);
       }
+      s_dig = use_digits(L) ? 1 : 0;
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -587,7 +800,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
     if (blockIdx.x < items) s = load(blockIdx.x);
     for (unsigned t = blockIdx.x; t < items; t += gridDim.x, ++n) {
       const int16_t* ce = col_e + (L.op_segs > 1 ? s : 0) * L.kpad;
-      int E = -(1 << 19);
+      int key = NO_KEY;
       bool bad = false;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
@@ -598,15 +811,16 @@ __global__ void __launch_bounds__(SL_NT, 1)
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             bad = bad || not_finite(x[i][e]);
-            if (!is_zero(x[i][e])) E = max(E, elem_e(x[i][e], short_of(c, e)));
+            if (!is_zero(x[i][e])) key = max(key, elem_key(x[i][e], short_of(c, e)));
           }
         }
       }
 #pragma unroll
       for (int o = RW; o < 32; o <<= 1) {
-        E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+        key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
         bad = __shfl_xor_sync(0xffffffffu, (int)bad, o) || bad;
       }
+      int E = row_e_of(key);
       if (E < -(1 << 18)) E = 0;
       if (bad) E = SPECIAL;
       if (n >= (unsigned)L.bbuf && !warp_wait(&bempty[bslot], bph ^ 1u)) break;
@@ -649,13 +863,14 @@ __global__ void __launch_bounds__(SL_NT, 1)
     const int quarter = warp & 3, half = ew >> 2;
     double* st4 = stg + ew * 32 * STG_LD;
     const int sr = lane >> 2, sc = lane & 3;
+    const bool take = use_digits(L);
     int ring = 0;
     uint32_t unit = 0;
     bool ok = true;
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x) {
       int mt0, pt, slot, s;
       decode(t, mt0, pt, slot, s);
-      const int b = active_problem(d.batch_list, nb, d.batch, slot);
+      const int b = take ? active_problem(d.batch_list, nb, d.batch, slot) : -1;
       const int os = L.op_segs > 1 ? s : 0;
       const long long ib = (long long)(b < 0 ? 0 : b) * d.in_batch + (long long)s * d.in_seg;
       double* outS = L.out + (long long)(b < 0 ? 0 : b) * d.out_batch + (long long)s * d.out_seg;
@@ -702,7 +917,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
             bool x;
             cell[c] = level_value(level_join(r[c], r[4 + c], r[8 + c], r[12 + c]),
                                   level_join(r[16 + c], r[20 + c], r[24 + c], r[28 + c]),
-                                  Ea + Ep[c] - 2080, x);
+                                  Ea + Ep[c] - 2082, x);
             rare |= (x || Ea + Ep[c] >= BIG) ? 1u << c : 0u;
           }
           if (rare && m < d.M && b >= 0) {
@@ -749,6 +964,8 @@ __global__ void __launch_bounds__(SL_NT, 1)
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (!s_dig) fma_tiles<EPI>(L, nb, (double*)smem);  // every copy has landed
+  __syncwarp();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -783,7 +1000,7 @@ template <int EPI, bool LIN>
 __global__ void __launch_bounds__(SL_NT, 1)
     k_contract_sl_rows(const __grid_constant__ SlLaunch L) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int s_nb;
+  __shared__ int s_nb, s_dig;
   uint8_t* smem = smem_raw + ((0u - tc::smem_u32(smem_raw)) & 1023u);
   const jfg_contract_desc& d = L.d;
   uint8_t* as = smem;                                 // [NS][RT][64]
@@ -802,6 +1019,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int units = (d.M + RM - 1) / RM;  // 1 or 2
+  if (blockIdx.x >= (unsigned)L.ctas && use_digits(L)) return;
   if (threadIdx.x == 0) {
     s_nb = active_count(d.batch_list, d.batch_count, d.batch);
     tc::mbar_init(ofull, 1);
@@ -853,7 +1071,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
 
   if (warp == 0) {
     // the operator has landed before the CTA may end
-    if (lane == 0) tc::mbar_wait(ofull, 0, &g_sl_status);
+    if (lane == 0) {
+      tc::mbar_wait(ofull, 0, &g_sl_status);
+      s_dig = use_digits(L) ? 1 : 0;
+    }
   } else if (warp == 1) {
     // ---------------- MMA issuer (uniform walk as above) ----------------
     const uint32_t ad0 = (uint32_t)tc::sdesc_sw128(tc::smem_u32(as));
@@ -959,10 +1180,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
       int E[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        E[i] = -(1 << 19);
+        E[i] = NO_KEY;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const int v = not_finite(x[i][e]) ? SPECIAL : elem_e(x[i][e], short_of(ce, e));
+          const int v = not_finite(x[i][e]) ? 64 * SPECIAL : elem_key(x[i][e], short_of(ce, e));
           if (!is_zero(x[i][e])) E[i] = max(E[i], v);
         }
       }
@@ -973,6 +1194,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
       if (n >= 1 && !warp_wait(bempty, (n & 1u) ^ 1u)) break;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
+        E[i] = row_e_of(E[i]);
         if (E[i] < -(1 << 18)) E[i] = 0;
         if (u == 0) row_e[(n & (RING - 1)) * RT + 32 * i + row0] = E[i];
         unsigned long long f[8];
@@ -998,13 +1220,14 @@ __global__ void __launch_bounds__(SL_NT, 1)
     // ---------------- epilogue: a lane is an input row ----------------
     const int quarter = warp & 3, half = (warp - 2 - NWS) >> 2;
     const int row = 32 * quarter + lane;
+    const bool take = use_digits(L);
     uint32_t unit = 0, n = 0;
     bool ok = true;
     for (unsigned t = blockIdx.x; ok && t < items; t += gridDim.x, ++n) {
       int s;
       unsigned slot, up;
       locate(t, row, s, slot, up);
-      const int b = problem(slot), p = (int)up;
+      const int b = take ? problem(slot) : -1, p = (int)up;
       const long long ib = (long long)(b < 0 ? 0 : b);
       double* outP = L.out + ib * d.out_batch + (long long)s * d.out_seg + p;
       const double* f = (const double*)d.field + ib * d.field_batch + (long long)s * d.field_seg + p;
@@ -1054,7 +1277,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
             bool xr;
             val[c] = level_value(level_join(r[c], r[4 + c], r[8 + c], r[12 + c]),
                                  level_join(r[16 + c], r[20 + c], r[24 + c], r[28 + c]),
-                                 Ea[c] + Ep - 2080, xr);
+                                 Ea[c] + Ep - 2082, xr);
             rare |= (xr || Ea[c] + Ep >= BIG) ? 1u << c : 0u;
           }
           if (b >= 0) {
@@ -1094,6 +1317,8 @@ __global__ void __launch_bounds__(SL_NT, 1)
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (!s_dig) fma_tiles<EPI>(L, nb, (double*)smem);  // every copy has landed
+  __syncwarp();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -1191,12 +1416,16 @@ int launch_rows(const SlLaunch& L, dim3 grid, cudaStream_t st) {
 size_t sl_op_bytes(int nseg, int M, int K) {
   if (K < 1 || K > SL_KMAX || M < 1 || nseg < 1) return 0;
   return align_up((size_t)nseg * NS * M * kp8(K) * 2, 256) + align_up((size_t)nseg * M * 4, 256) +
-         align_up((size_t)nseg * kp64(K) * 2, 256);
+         align_up((size_t)nseg * kp64(K) * 2, 256) +
+         align_up((size_t)nseg * 4, 256);
 }
 
-SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, void* work) {
+SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, SlRule rule,
+           void* work, const double* lam) {
   SlOp o;
   o.src = src;
+  o.lam = lam;
+  o.rule = rule;
   o.ld = ld;
   o.seg = seg;
   o.nseg = nseg;
@@ -1209,6 +1438,8 @@ SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int 
   o.row_e = (int*)w;
   w += align_up((size_t)nseg * M * 4, 256);
   o.col_e = (int16_t*)w;
+  w += align_up((size_t)nseg * kp64(K) * 2, 256);
+  o.use = (int*)w;
   return o;
 }
 
@@ -1223,6 +1454,7 @@ int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st) {
     for (int s = 0; s < o.nseg; ++s) {
       if (n == SL_MAX_SEGS) return JFG_ERR_ARG;
       A.s[n++] = SlSeg{o.src + s * o.seg,
+                       o.lam,
                        o.ld,
                        o.M,
                        o.K,
@@ -1230,7 +1462,9 @@ int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st) {
                        kpad,
                        o.dig + (size_t)s * NS * o.M * Kp,
                        o.row_e + (size_t)s * o.M,
-                       o.col_e + (size_t)s * kpad};
+                       o.col_e + (size_t)s * kpad,
+                       o.use + s,
+                       o.rule};
     }
   }
   if (n == 0) return JFG_OK;
@@ -1269,6 +1503,7 @@ int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, do
   L.out = out;
   L.row_e = op.row_e;
   L.col_e = op.col_e;
+  L.use = op.use;
   L.op_segs = d.nseg > 1 && op.nseg > 1 ? d.nseg : 1;
   L.row_ld = op.M;
   L.kpad = kp64(d.K);
@@ -1307,9 +1542,16 @@ int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, do
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return JFG_ERR_ARG;
-  if (rows) return launch_rows(L, dim3((unsigned)(row_tiles < sms ? row_tiles : sms)), st);
-  const dim3 grid((unsigned)(items < sms ? items : sms));
+  // a CTA per tile of the FMA sums too, should the operator's digits not be taken
+  // (of eigenvector factors and packed operators they are)
+  const long long fma_ctas = (long long)d.batch * d.nseg * ((d.M + 15) / 16) * ((d.P + 31) / 32);
+  const long long tiles = rows ? row_tiles : items;
+  const long long most = op.rule == SL_DENSE ? std::max(tiles, fma_ctas) : tiles;
+  L.ctas = (int)(tiles < sms ? tiles : sms);
+  const dim3 grid((unsigned)(most < sms ? most : sms));
+  if (rows) return launch_rows(L, grid, st);
   const size_t smem = fixed + (size_t)L.astages * ABYTES;
+  static_assert(FMA_SMEM <= 2 * ABYTES && FMA_SMEM <= ROWS_SMEM, "the FMA tiles fit");
   return PT == 32 ? launch<32>(L, grid, smem, st) : launch<16>(L, grid, smem, st);
 }
 

@@ -137,13 +137,19 @@ constexpr int SL_MAX_SEGS = 8;    // operator segments cut in one launch
 // 25.4 us, of which the cut is ~9 us.
 constexpr double SL_MIN_WORK = 8e6;
 constexpr double SL_MIN_WORK_CUT = 4e6;
+// How an operator must look for its digits to be taken (contract_sl.cu); where
+// it does not, the same launch sums it by FP64 FMAs.
+enum SlRule { SL_DENSE = 0, SL_FACTORS = 1 };
 struct SlOp {
   const double* src = nullptr;
+  const double* lam = nullptr;  // eigenvalues that the inputs were divided by, or null
   long long ld = 0, seg = 0;
   int nseg = 0, M = 0, K = 0;
+  SlRule rule = SL_DENSE;
   uint16_t* dig = nullptr;  // null: not cut, the CUDA-core contraction serves it
   int* row_e = nullptr;
   int16_t* col_e = nullptr;
+  int* use = nullptr;  // per segment: 1 digits, 0 FMAs (written by the cut)
   // segment s alone
   SlOp segment(int s) const {
     SlOp o = *this;
@@ -153,12 +159,14 @@ struct SlOp {
       o.dig += (size_t)s * 8 * M * ((K + 7) / 8 * 8);
       o.row_e += (size_t)s * M;
       o.col_e += (size_t)s * ((K + 63) / 64 * 64);
+      o.use += s;
     }
     return o;
   }
 };
 size_t sl_op_bytes(int nseg, int M, int K);  // 0 when K > SL_KMAX
-SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, void* work);
+SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, SlRule rule,
+           void* work, const double* lam = nullptr);
 int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st);  // operators without dig are skipped
 bool sl_pays(const jfg_contract_desc& d, double min_work = SL_MIN_WORK);
 int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, double* out,
@@ -268,7 +276,7 @@ int varcoef_apply(Engine e, int ndim, int n, int nq, int batch, OpRef<T> ops, co
 // varcoef_apply (SL_VARCOEF); sl_split_ops cuts them.
 constexpr int SL_VARCOEF = 4;
 size_t fd_sl_bytes(int n);
-void fd_sl_ops(int n, const double* E, const double* W, void* work, SlOp* out);
+void fd_sl_ops(int n, const double* E, const double* W, const double* lam, void* work, SlOp* out);
 // whether a varcoef_apply is large enough to cut its operators for it
 bool varcoef_pays(int ndim, int n, int nq, int batch, double min_work);
 size_t varcoef_sl_bytes(int ndim, int n, int nq);

@@ -655,7 +655,7 @@ int PcgCtx<T>::init(const PcgProblem<T>& problem, T* x_, void* work, size_t work
       inner_bytes -= cut;
       char* c = (char*)work + need;
       varcoef_sl_ops(ndim, n, nq, pb.ops.hi, c, sl_a);
-      fd_sl_ops(n, pb.E.hi, pb.W.hi, c + varcoef_sl_bytes(ndim, n, nq), sl_m);
+      fd_sl_ops(n, pb.E.hi, pb.W.hi, pb.lam, c + varcoef_sl_bytes(ndim, n, nq), sl_m);
       sl = true;
       JFG_TRY(sl_setup());  // before the iterations are captured
     }

@@ -31,13 +31,27 @@ def device_op(mat: np.ndarray, dtype=torch.float64) -> torch.Tensor:
     return t
 
 
+def _dense(mat: np.ndarray) -> bool:
+    """Whether FP64 passes of ``mat`` can run on digits (nearly all entries within
+    2^8 of their row's largest, columns scaled to one size).  The library judges
+    by itself; this spares banded and triangular operators the attempt."""
+    a = np.abs(mat)
+    top = a.max(axis=0, initial=0.0)
+    cols = (top > 0) & np.isfinite(top)
+    if not cols.any():
+        return False
+    a = np.ldexp(a[:, cols], -np.frexp(top[cols])[1])
+    large = a >= a.max(axis=1, keepdims=True) * 2.0**-8
+    return bool(large.mean() >= 15 / 16)
+
+
 class _TpPlan:
     """What every call with the same operators and type shares: their device
     copies and the C arrays of sizes and pointers (the operators stay
     referenced, so that their ids stay theirs).  ``ws`` is the workspace size of
-    the last batch."""
+    the last batch, ``size`` the function that says it."""
 
-    __slots__ = ("mats", "ops", "rows", "cols", "r_a", "c_a", "ptrs", "ws")
+    __slots__ = ("mats", "ops", "rows", "cols", "r_a", "c_a", "ptrs", "ws", "size")
 
     def __init__(self, mats, dtype):
         self.mats = mats
@@ -47,14 +61,16 @@ class _TpPlan:
         self.r_a, self.c_a = _lib.int_array(self.rows), _lib.int_array(self.cols)
         self.ptrs = _lib.ptr_array([o.data_ptr() for o in self.ops])
         self.ws = (-1, 0)
+        L = _lib.lib()
+        digits = dtype == torch.float64 and any(map(_dense, mats))
+        self.size = L.jfg_tp_apply_workspace_size if digits else L.jfg_tp_apply_fma_workspace_size
 
-    def workspace(self, batch: int, elem_bytes: int) -> torch.Tensor:
+    def workspace(self, batch: int, elem_bytes: int) -> tuple[torch.Tensor, int]:
         last, size = self.ws
         if last != batch:
-            size = _lib.lib().jfg_tp_apply_workspace_size(len(self.rows), self.r_a, self.c_a,
-                                                          batch, elem_bytes)
+            size = self.size(len(self.rows), self.r_a, self.c_a, batch, elem_bytes)
             self.ws = (batch, size)
-        return workspace(size)
+        return workspace(size), size
 
 
 _PLANS: dict[tuple, _TpPlan] = {}
@@ -87,10 +103,10 @@ def tp_apply(mats: list[np.ndarray], x, dtype=torch.float64, df: bool = False) -
         return out
     L = _lib.lib()
     f64 = dtype == torch.float64
-    ws = plan.workspace(batch, 8 if f64 else 4)
+    ws, ws_bytes = plan.workspace(batch, 8 if f64 else 4)
     fn = (L.jfg_tp_apply_df64 if df else L.jfg_tp_apply_f64) if f64 else L.jfg_tp_apply_f32
     st = fn(nd, plan.r_a, plan.c_a, batch, plan.ptrs, x.data_ptr(), out.data_ptr(),
-            ws.data_ptr(), ws.numel(), _lib.stream_handle())
+            ws.data_ptr(), ws_bytes, _lib.stream_handle())
     _lib.check(st, "jfg_tp_apply")
     return out
 
@@ -294,8 +310,8 @@ class TensorProductSpace:
         return W
 
     # ---- transforms (tensorproductspace.py:330-417) -------------------------
-    # precision: "f64" (FP64, parity path: the tensor cores' exact digit products
-    # or FP64 FMAs, by size), "df64" (FP64 data, the same for large passes, else
+    # precision: "f64" (FP64, parity path: digit products on the tensor cores or
+    # FP64 FMAs, by size and operator), "df64" (FP64 data, the same for large passes, else
     # double-FP32 arithmetic on the FP32 pipe, ~1e-14), "bf16x3" (FP32 data,
     # split-BF16 operators, three BF16 MMAs per product) or "tc" (FP32 data,
     # split-TF32 tcgen05 contractions)
