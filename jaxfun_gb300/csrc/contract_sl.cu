@@ -24,8 +24,8 @@
 // largest entries with entries not far below its row's largest one, which
 // k_sl_split judges by the operator.  Level d sums at most d + 1 digit pairs, each
 // below 2^14 K: levels 0..3 cannot pass 2^24 for K <= 256 (0 and 1 for
-// K <= 512), and a level that did could only lose its last bits, which weigh
-// 2^-8d.  Rows with an infinity or a NaN (in the operator or the input) are
+// K <= 512; sums whose level 2 or 3 did are redone by FMAs), and the others
+// could only lose their last bits, which weigh 2^-8d.  Rows with an infinity or a NaN (in the operator or the input) are
 // summed by plain FP64 FMAs in the epilogue.
 //
 // Tile.  A CTA takes PT input rows (p) of one problem and segment, cuts them
@@ -919,6 +919,10 @@ __global__ void __launch_bounds__(SL_NT, 1)
                                   level_join(r[16 + c], r[20 + c], r[24 + c], r[28 + c]),
                                   Ea + Ep[c] - 2082, x);
             rare |= (x || Ea + Ep[c] >= BIG) ? 1u << c : 0u;
+            // K > 256 (PT 16): levels 2 and 3 may have lost bits past 2^24
+            if (PT == 16 && fmaxf(fabsf(__uint_as_float(r[8 + c])),
+                                  fabsf(__uint_as_float(r[12 + c]))) >= 16777216.f)
+              rare |= 1u << c;
           }
           if (rare && m < d.M && b >= 0) {
             const double* a = L.op + (long long)os * d.op_seg + (long long)m * d.op_ld;

@@ -120,3 +120,20 @@ def test_mantissas_near_two(n, B):
     got, ref = tp([A, V], x), tp([A, V], x, cut=False)
     mag = torch.einsum("ma,nb,iab->imn", A.abs(), V.abs(), x.abs())
     assert ((got - ref).abs() <= 4 * (2 * n + 2) * 2.0**-53 * mag).all()
+
+
+def test_levels_past_their_exact_range():
+    """K = 512 terms whose first three digits are all 120: the levels' FP32 sums
+    pass 2^24, and the results are still those of FP64 sums."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(10)
+    K, M, B = 512, 130, 40
+
+    def near(*shape):
+        u = torch.rand(*shape, dtype=torch.float64, device="cuda", generator=g) - 0.5
+        return (float(0x787878) + 0.8 * u) * 2.0**-23
+
+    I, A, x = near(16, 16), near(M, K), near(B, 16, K)
+    got, ref = tp([I, A], x), tp([I, A], x, cut=False)
+    mag = torch.einsum("ma,nb,iab->imn", I, A, x)
+    assert ((got - ref).abs() <= 4 * (K + 16 + 2) * 2.0**-53 * mag).all()
