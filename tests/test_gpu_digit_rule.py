@@ -122,16 +122,20 @@ def test_mantissas_near_two(n, B):
     assert ((got - ref).abs() <= 4 * (2 * n + 2) * 2.0**-53 * mag).all()
 
 
-def test_levels_past_their_exact_range():
-    """K = 512 terms whose first three digits are all 120: the levels' FP32 sums
-    pass 2^24, and the results are still those of FP64 sums."""
+@pytest.mark.parametrize("K", [256, 257, 512])
+def test_levels_past_their_exact_range(K):
+    """K terms whose first three digits lie between 104 and 125: above 256 terms
+    the FP32 sums of levels that count pass 2^24, on values of every parity, and
+    the results are still those of FP64 sums."""
     g = torch.Generator(device="cuda")
     g.manual_seed(10)
-    K, M, B = 512, 130, 40
+    M, B = 130, 40
 
     def near(*shape):
         u = torch.rand(*shape, dtype=torch.float64, device="cuda", generator=g) - 0.5
-        return (float(0x787878) + 0.8 * u) * 2.0**-23
+        for _ in range(3):
+            u = u / 256 + torch.randint(104, 126, shape, device="cuda", generator=g)
+        return u * 2.0**-7
 
     I, A, x = near(16, 16), near(M, K), near(B, 16, K)
     got, ref = tp([I, A], x), tp([I, A], x, cut=False)
