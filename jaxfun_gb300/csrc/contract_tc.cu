@@ -1710,10 +1710,9 @@ extern "C" int jfg_tc_autotune(int ngroups, const jfg_contract_desc* descs,
     for (int o = 0; o < orders; ++o)
       for (int sg : {0, 3, 2})
         for (int mt : {0, 64}) {
-          jfg_tc_config c;
+          jfg_tc_config c = jfg::tc_default_config();
           c.operand_a_in_tmem = ta;
           c.order = o;
-          c.ctas = 0;
           c.stages = sg;
           c.mtile = mt;
           cands.push_back(c);
