@@ -8,6 +8,7 @@
 // kernel is DFMA-bound long before it is memory-bound.
 #include <stdio.h>
 
+#include <cmath>
 #include <type_traits>
 
 #include "jfg_internal.cuh"
@@ -317,6 +318,14 @@ int sm_count(int* n) {
 int contract_f64_tile(const jfg_contract_desc& d) {
   int sms = 0;
   return 16 * (sm_count(&sms) == JFG_OK ? tile_r(d, false, sms) : 4);
+}
+
+double contract_f64_us(const jfg_contract_desc& d) {
+  int sms = 0;
+  if (sm_count(&sms) != JFG_OK || d.batch < 1 || d.M < 1 || d.P < 1) return 0.0;
+  const int t = 16 * tile_r(d, false, sms);
+  const double tiles = (double)d.batch * d.nseg * ((d.M + t - 1) / t) * ((d.P + t - 1) / t);
+  return 5.0 + std::ceil(tiles / sms) * t * t * ((d.K + TK - 1) / TK * TK) / 3900.0;
 }
 
 int contract_f64(const jfg_contract_desc& d, const double* op, const double* in, double* out,

@@ -61,6 +61,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "jfg_internal.cuh"
 #include "tc_common.cuh"
@@ -1484,8 +1485,21 @@ bool sl_pays(const jfg_contract_desc& d, double min_work) {
     return false;
   const int t = contract_f64_tile(d);
   const double tiles = (double)d.batch * d.nseg * ((d.M + t - 1) / t) * ((d.P + t - 1) / t);
-  return tiles * t * t * ((d.K + 15) / 16 * 16) >= min_work;
+  return tiles * t * t * ((d.K + 15) / 16 * 16) >= min_work && sl_us(d) < contract_f64_us(d);
 }
+
+// Fitted to calls at the least work that took digits, M = 5 to 512 by K = 16 to
+// 510 in one to three dimensions: with the rule made of these and of
+// contract_f64_us the slower way is taken nowhere by more than 7 % (by 9 to 90 %
+// at every second shape before, by the work alone).
+double sl_us(const jfg_contract_desc& d) {
+  int sms = 0;
+  if (sm_count(&sms) != JFG_OK) return 0.0;
+  const int pt = d.K > 256 ? 16 : 32;
+  const double items = (double)d.batch * d.nseg * ((d.P + pt - 1) / pt) * ((d.M + 127) / 128);
+  return 6.0 + 0.02 * d.K + std::floor(items / sms) * (1.0 + 0.03 * d.K);
+}
+double sl_cut_us(int M, int K) { return 14.0 + 0.02 * M + 3e-5 * M * K; }
 
 int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, double* out,
                 cudaStream_t st) {

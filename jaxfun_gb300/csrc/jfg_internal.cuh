@@ -91,6 +91,8 @@ struct DotOut {
 int sm_count(int* n);  // SMs of the current device
 // tile of the FP64 CUDA-core launch (64, 32 or 16)
 int contract_f64_tile(const jfg_contract_desc& d);
+// its time in us: an SM does two FMAs per clock, padding included
+double contract_f64_us(const jfg_contract_desc& d);
 int contract_f64(const jfg_contract_desc& d, const double* op, const double* in, double* out,
                  cudaStream_t st);
 int contract_f32(const jfg_contract_desc& d, const float* op, const float* in, float* out,
@@ -131,10 +133,11 @@ int tc_setup();
 constexpr int SL_KMAX = 512;      // largest contracted extent
 constexpr int SL_MAX_SEGS = 8;    // operator segments cut in one launch
 // CUDA-core multiply-adds of a pass (its tiles' padding included) from which
-// the tensor-core contraction is faster: when the operator is cut in the same
-// call, and when it has been cut before.  Two passes of 32 x 64^2 (8.4e6
-// each): 31.5 us cut in the call against 41.9 us; of 16 x 64^2: 31.7 against
-// 25.4 us, of which the cut is ~9 us.
+// the tensor-core contraction is tried: when the operator is cut in the same
+// call, and when it has been cut before.  Two passes of 31 x 64^2 (8.1e6
+// each): 29 us cut in the call against 41 us; of 16 x 64^2: 31.7 against
+// 25.4 us.  Below them shapes differ little; above, sl_us and sl_cut_us tell the
+// shapes that would lose.
 constexpr double SL_MIN_WORK = 8e6;
 constexpr double SL_MIN_WORK_CUT = 4e6;
 // How an operator must look for its digits to be taken (contract_sl.cu); where
@@ -168,7 +171,11 @@ size_t sl_op_bytes(int nseg, int M, int K);  // 0 when K > SL_KMAX
 SlOp sl_op(const double* src, long long ld, long long seg, int nseg, int M, int K, SlRule rule,
            void* work, const double* lam = nullptr);
 int sl_split_ops(const SlOp* ops, int nops, cudaStream_t st);  // operators without dig are skipped
+// a pass on the tensor cores against the CUDA cores: large enough, and faster
+// (its operator cut before)
 bool sl_pays(const jfg_contract_desc& d, double min_work = SL_MIN_WORK);
+double sl_us(const jfg_contract_desc& d);  // a pass, us
+double sl_cut_us(int M, int K);            // cutting operators of up to M x K, us
 int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, double* out,
                 cudaStream_t st);
 int sl_setup();

@@ -10,6 +10,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "jfg_internal.cuh"
@@ -47,15 +48,28 @@ size_t tp_apply_ws(int ndim, const int* rows, const int* cols, int batch, int eb
   return 2 * tp_inter_bytes(ndim, rows, cols, batch, eb) + align_up(ops * sizeof(float2), 256);
 }
 
-// the axes whose pass is large enough for the tensor-core FP64 contraction
+// The axes whose pass is large enough for the tensor-core FP64 contraction; none
+// where their passes together save less than the cut costs: one axis of 512 x 256
+// on 4 vectors 43 us cut in the call, 23 on the CUDA cores, of 128 x 128 on 31
+// 24 and 21; 31 fields of 64 x 64, two passes, 29 and 41.
 static void tp_sl_axes(int ndim, const int* rows, const int* cols, int batch, bool* on) {
   double rest = 1;  // the field at axis i: later axes are already rows
+  double saved = 0.0, cut = 0.0;
   for (int i = 0; i < ndim; ++i) rest *= cols[i];
   for (int i = ndim - 1; i >= 0; --i) {
     const double P = rest / cols[i];
     rest = P * rows[i];
-    on[i] = P <= 2147483647.0 && sl_pays(make_desc(batch, rows[i], (int)P, cols[i]));
+    on[i] = false;
+    if (P > 2147483647.0) continue;
+    const jfg_contract_desc d = make_desc(batch, rows[i], (int)P, cols[i]);
+    on[i] = sl_pays(d);
+    if (on[i]) {
+      saved += contract_f64_us(d) - sl_us(d);
+      cut = std::max(cut, sl_cut_us(rows[i], cols[i]));
+    }
   }
+  if (saved < cut)
+    for (int i = 0; i < ndim; ++i) on[i] = false;
 }
 
 // with room for the operators of those axes cut into digits behind it (FP64)

@@ -141,3 +141,16 @@ def test_levels_past_their_exact_range(K):
     got, ref = tp([I, A], x), tp([I, A], x, cut=False)
     mag = torch.einsum("ma,nb,iab->imn", I, A, x)
     assert ((got - ref).abs() <= 4 * (K + 16 + 2) * 2.0**-53 * mag).all()
+
+
+@pytest.mark.parametrize("rows,cols,B,digits", [
+    ((512,), (256,), 4, False), ((128,), (128,), 31, False), ((5,), (128,), 245, False),
+    ((512, 512), (16, 16), 2, False), ((64, 64), (64, 64), 31, True),
+    ((128, 128), (128, 128), 4, True), ((512,), (256,), 40, True)])
+def test_calls_that_digits_would_slow_down(rows, cols, B, digits):
+    """Room for digits is asked for where the passes save more than the cut costs."""
+    from jaxfun_gb300 import _lib
+
+    L = _lib.lib()
+    a = len(rows), _lib.int_array(rows), _lib.int_array(cols), B, 8
+    assert (L.jfg_tp_apply_workspace_size(*a) > L.jfg_tp_apply_fma_workspace_size(*a)) == digits
