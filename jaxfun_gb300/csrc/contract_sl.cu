@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(SL_NT, 1)
                                   Ea + Ep[c] - 2082, x);
             rare |= (x || Ea + Ep[c] >= BIG) ? 1u << c : 0u;
             // K > 256 (PT 16): levels 2 and 3 may have lost bits past 2^24
-            if (PT == 16 && fmaxf(fabsf(__uint_as_float(r[8 + c])),
+            if (PT == 16 && L.nkb > 4 && fmaxf(fabsf(__uint_as_float(r[8 + c])),
                                   fabsf(__uint_as_float(r[12 + c]))) >= 16777216.f)
               rare |= 1u << c;
           }
@@ -1560,11 +1560,12 @@ int contract_sl(const jfg_contract_desc& d, const SlOp& op, const double* in, do
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return JFG_ERR_ARG;
-  // a CTA per tile of the FMA sums too, should the operator's digits not be taken
-  // (of eigenvector factors and packed operators they are)
+  // where digits take half of the SMs at most, a CTA per tile of the FMA sums too,
+  // should the operator's digits not be taken (of eigenvector factors and packed
+  // operators they are)
   const long long fma_ctas = (long long)d.batch * d.nseg * ((d.M + 15) / 16) * ((d.P + 31) / 32);
   const long long tiles = rows ? row_tiles : items;
-  const long long most = op.rule == SL_DENSE ? std::max(tiles, fma_ctas) : tiles;
+  const long long most = op.rule == SL_DENSE && 2 * tiles <= sms ? std::max(tiles, fma_ctas) : tiles;
   L.ctas = (int)(tiles < sms ? tiles : sms);
   const dim3 grid((unsigned)(most < sms ? most : sms));
   if (rows) return launch_rows(L, grid, st);
