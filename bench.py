@@ -976,7 +976,7 @@ def run_ours(args):
             tuned = solver.autotune(mws)
             tuned_txt = "; ".join(
                 f"{t['signature'].split(':', 1)[1]} -> {t['schedule']}, {t['stages'] or 'max'} "
-                f"stages, {t['store']} stores, mtile {t['mtile']} ({1e3 * t['ms']:.1f} us)"
+                f"stages, mtile {t['mtile']} ({1e3 * t['ms']:.1f} us)"
                 for t in tuned)
         for _ in range(args.warmup):
             solve()
